@@ -37,10 +37,16 @@ struct Handle {
     int max_batch = 0;
     int cpb = 1, threads = 32, ctas_per_sm = 1, sm_count = 1, max_grid = 1, minb = 1;
     size_t smem = 0;
+    // small batches: one codeword on a cluster of CTAs (split.cu), plans from
+    // the largest cluster to the smallest
+    std::vector<SplitHead> split;
+    std::vector<int> split_room;     // clusters resident at once
+    std::vector<size_t> split_at;    // the plan's place in scratch, bytes
     uint32_t* state = nullptr;
     uint32_t* state2 = nullptr;  // the second lane's check-node state (host-buffer pipeline)
     // [0] work counter, [1] error flag, [kChunkCounter + k] work counter of
-    // chunk k of a host-buffer decode
+    // chunk k of a host-buffer decode; the small-batch plans from byte
+    // kScratchBytes on
     int* scratch = nullptr;
     float* stage_llr = nullptr;
     uint8_t* stage_packed = nullptr;
@@ -166,6 +172,69 @@ void free_handle(Handle* h) {
     delete h;
 }
 
+// Cluster sizes tried for small batches: each holds more codewords at once
+// than the one before (GB300 at one CTA per SM: 7, 13, 23, 28, 36, 46, 76 and
+// 152 clusters; a GPC's SMs do not divide evenly by the other sizes).
+const int kSplitRanks[] = {16, 10, 6, 5, 4, 3, 2, 1};
+constexpr int kSplitMinTasks = 12;  // 32-sub-row tasks per CTA worth a larger cluster
+
+// Plans for the cluster sizes that fit; their bytes go behind the handle's
+// scratch words in device memory.
+int split_prepare(Handle* h, size_t smem_limit, std::vector<unsigned char>* bytes) {
+    if (split_kernel_attributes(smem_limit) != cudaSuccess) return NRLDPC_ERR_CUDA;
+    const int tasks = h->tab.rows * ((h->tab.z + 31) / 32);
+    for (int ranks : kSplitRanks) {
+        if (ranks > 1 && tasks < ranks * kSplitMinTasks) continue;
+        SplitHead p;
+        const size_t at = bytes->size();
+        if (!make_split_plan(h->tab, ranks, smem_limit, &p, bytes)) continue;
+        const int room = split_max_clusters(p);
+        if (room < 1) {
+            bytes->resize(at);
+            continue;
+        }
+        h->split.push_back(p);
+        h->split_room.push_back(room);
+        h->split_at.push_back(at);
+    }
+    return NRLDPC_OK;
+}
+
+// Plan for n codewords, or -1 for decode_kernel: the smaller of two time
+// estimates, in edges of one warp (45 ns per 10 iterations).  A wave of
+// clusters takes kSplitFixed per phase (barriers, the passes' latency) plus
+// the busiest CTA's edges; decode_kernel's walk down the rows costs per row
+// and edge, more with more warps on the SM.  Fitted to GB300 times, 10
+// iterations, us (model): BG1 Z=384 on 16 / 8 / 4 / 3 CTAs 52 / 68 / 103 / 151
+// (47 / 64 / 98 / 150), BG2 Z=384 40 / 48 / 72 / 89, BG1 Z=96 on 4 / 2 / 1
+// CTAs 42 / 59 / 81 (47 / 64 / 98); decode_kernel BG1 Z=384 / 208 / 96 at one
+// CTA per SM 300 / 245 / 204 (300 / 248 / 207), BG2 Z=384 / 128 219 / 157, two
+// CTAs per SM 1.5-1.65 times that.
+constexpr long kSplitFixed = 667;
+
+long fused_cost(const Handle* h, int n) {
+    const long groups = (n + h->cpb - 1) / h->cpb, w = h->threads / 32;
+    const long one = h->tab.rows * (29 + 21 * w / 10) + h->tab.n_edges * (81 + 4 * w) / 10;
+    long cost = groups / h->max_grid * (one * (4 + 2 * h->ctas_per_sm) / 5);
+    const long rest = groups % h->max_grid;
+    if (rest) cost += one * (3 + 2 * ((rest + h->sm_count - 1) / h->sm_count)) / 5;
+    return cost;
+}
+
+int split_choice(const Handle* h, int n) {
+    int best = -1;
+    long least = fused_cost(h, n);
+    for (size_t k = 0; k < h->split.size(); k++) {
+        const long waves = (n + h->split_room[k] - 1) / h->split_room[k];
+        const long cost = waves * (kSplitFixed * h->split[k].phases + h->split[k].load);
+        if (cost < least) {
+            least = cost;
+            best = static_cast<int>(k);
+        }
+    }
+    return best;
+}
+
 int init_impl(const int* base, int rows, int cols, int kb, const nrldpc_config* cfg,
               nrldpc_handle** out) {
     if (!cfg || !out || cfg->max_batch < 1 || !(cfg->alpha > 0.0f) || cfg->cw_per_cta < 0)
@@ -226,10 +295,15 @@ int init_impl(const int* base, int rows, int cols, int kb, const nrldpc_config* 
     const size_t state_elems =
         static_cast<size_t>(h->max_grid) * cpb * h->tab.rows * static_cast<size_t>(z);
     const size_t n_llr = static_cast<size_t>(cfg->max_batch) * h->tab.n_bp;
+    std::vector<unsigned char> scratch(kScratchBytes, 0);  // zero words, then the plans
+    if (const int rc = split_prepare(h, smem_limit, &scratch)) {
+        delete h;
+        return rc;
+    }
     if (cudaMalloc(&h->state, state_elems * kStateBytesPerRow) != cudaSuccess ||
         cudaMalloc(&h->state2, state_elems * kStateBytesPerRow) != cudaSuccess ||
-        cudaMalloc(&h->scratch, kScratchBytes) != cudaSuccess ||
-        cudaMemset(h->scratch, 0, kScratchBytes) != cudaSuccess ||
+        cudaMalloc(&h->scratch, scratch.size()) != cudaSuccess ||
+        cudaMemcpy(h->scratch, scratch.data(), scratch.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMalloc(&h->stage_llr, n_llr * sizeof(float)) != cudaSuccess ||
         cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&h->lane_stream, cudaStreamNonBlocking) != cudaSuccess ||
@@ -262,6 +336,23 @@ int decode_impl(Handle* h, const float* llr, uint8_t* packed, int n_cw, int n_it
     if (n_cw > h->max_batch) return NRLDPC_ERR_TOO_LARGE;
     if (reinterpret_cast<uintptr_t>(llr) % 16 != 0) return NRLDPC_ERR_ALIGNMENT;
     if (weighted && (!h->weights || h->n_w_iters < 1)) return NRLDPC_ERR_INVALID_ARG;
+    const int plan = (h->schedule == NRLDPC_SCHEDULE_FLOODING && extra_tx == 0) ? split_choice(h, n_cw) : -1;
+    if (plan >= 0) {
+        SplitArgs a{};
+        a.plan = reinterpret_cast<const unsigned char*>(h->scratch) + h->split_at[plan];
+        a.llr = llr;
+        a.packed = packed;
+        a.app = app;
+        a.iters = iters;
+        a.n_cw = n_cw;
+        a.n_iter = n_iter;
+        a.n_w_iters = h->n_w_iters;
+        a.early_stop = early;
+        a.llr_from_host = llr_from_host ? 1 : 0;
+        a.alpha = h->alpha;
+        return map_cuda(launch_split(h->split[plan], a, weighted ? h->weights : nullptr,
+                                     std::min(n_cw, h->split_room[plan]), stream));
+    }
     DecodeArgs a{};
     a.llr = llr;
     a.packed = packed;

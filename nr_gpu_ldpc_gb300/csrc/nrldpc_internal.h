@@ -4,6 +4,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <vector>
 
 #include "../../include/nr_gpu_ldpc_gb300.h"
 
@@ -121,6 +122,50 @@ inline size_t group_smem_bytes(const CodeTable& t, int cpb) {
 cudaError_t launch_batch_decode(const BatchDecodeArgs& args, int grid, int threads, size_t smem,
                                 cudaStream_t stream);
 const void* batch_decode_kernel_ptr();
+
+// One codeword on a cluster of CTAs (split.cu).  A plan is a head and one
+// table image per rank, contiguous in device memory: which CTA owns which base
+// row and core column, the check-node and variable-node tasks of each warp
+// (32 sub-rows or positions each), and the shared-memory layout.
+constexpr int kSplitMaxRanks = 16;   // CTAs per cluster
+constexpr int kSplitMaxPhases = 8;   // row ranges of an iteration
+constexpr int kSplitMaxWarps = 24;   // per CTA
+constexpr size_t kSplitHeader = 128;
+constexpr int kSplitKeepTo = 10;     // longest row whose dt addresses stay in registers
+constexpr int kSplitVnAhead = 8;     // dt requested before the first add
+constexpr int kSplitRowCost = 4;     // a row's fixed work, in edges
+constexpr int kSplitColCost = 6;     // a column's fixed work, in edges
+struct alignas(16) SplitHead {
+    int z, n_bp, packed_bytes, n_core, core_floats, ranks, phases, warps, n_edges;
+    int load;  // edges (and fixed work) of the busiest rank's tasks, per warp of sub-rows
+    // image: edges {offset, wrap threshold, owner << 24 | dt place} of the
+    // rank's rows; rows {first edge | edge in the code << 16, state, suffix
+    // column << 9 | shift, degree | suffix << 8}; columns {offset, ranks that
+    // read it}; their dt {first | count << 16} per phase; every column's
+    // owner; task lists per (phase,) warp
+    int o_edge, o_row, o_col, o_beg, o_own, o_cnptr, o_cn, o_vnptr, o_vn, image_bytes;
+    int off_l, off_state, off_dt, off_acc, smem;  // shared memory
+};
+struct SplitJob {            // one codeword of a mixed batch
+    int64_t llr_offset, out_offset;
+    int32_t plan, job;       // byte offset of its code's plan; iteration-count index
+};
+struct SplitArgs {
+    const unsigned char* plan;
+    const SplitJob* jobs;    // null: n_cw codewords of one code, back to back
+    const float* llr;
+    uint8_t* packed;
+    float* app;
+    int32_t* iters;
+    int n_cw, n_iter, n_w_iters, early_stop, llr_from_host;
+    float alpha;
+};
+bool make_split_plan(const CodeTable& tab, int ranks, size_t smem_limit, SplitHead* head,
+                     std::vector<unsigned char>* out);
+cudaError_t split_kernel_attributes(size_t smem);
+int split_max_clusters(const SplitHead& head);  // resident at once
+cudaError_t launch_split(const SplitHead& head, const SplitArgs& args, const WeightTable* weights, int n_clusters,
+                         cudaStream_t stream);
 
 // Host-side launchers (decode.cu / channel.cu).
 // minb: CTAs per SM the kernel's register budget assumes (1 or 2).

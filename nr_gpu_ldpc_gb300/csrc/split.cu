@@ -1,0 +1,691 @@
+// Flooding normalized min-sum for batches that leave SMs idle: one codeword on
+// a cluster of CTAs (sm_103a).
+//
+// decode_kernel walks a codeword's base rows in order on one SM, which is the
+// better use of a full GPU but leaves most of it idle on a small batch.  Here
+// the two halves of a flooding iteration are separate passes, each spread
+// over every warp of the cluster:
+//   * check-node pass: the CTA that owns a base row runs it for all Z
+//     sub-rows from its own copy of the posteriors, keeps the row's 16-byte
+//     state in shared memory and sends dt = R_new - R_old of each core edge to
+//     the CTA that owns the edge's column (distributed shared memory);
+//   * variable-node pass: the owner of a column adds its dt in ascending
+//     base-row order and sends the sums to the CTAs whose rows read them.
+// A suffix column has a single edge: its posterior stays in the row's state.
+// The sums are those of decode_kernel term by term (L + dt_r0 + dt_r1 + ...,
+// explicit round-to-nearest), so results are bit-identical to it.
+//
+// Everything is sent, nothing fetched: distributed shared memory moves about
+// 17 B per clock and SM whichever way it is accessed (24 KB in 1,450 clocks of
+// loads or stores, scalar or 128-bit; bulk copies slower), and a store of the
+// check-node pass costs its warp no wait.  Fetching dt from the rows' owners
+// instead took 5,700 of 12,300 clocks per iteration on 16 CTAs (BG1 Z=384).
+//
+// Early stop costs no pass of its own: the check-node pass of iteration t + 1
+// reads every posterior of iteration t, so it collects the row parities of
+// their hard decisions; when every row of the cluster is satisfied the
+// codeword leaves with iteration t's posteriors, which the passes so far have
+// not touched (the suffix hard decisions are kept in the state word).
+//
+// Shared memory per CTA: all core posteriors, the states of its rows and the
+// dt of its columns.  When the dt do not fit, the rows run in phases
+// (contiguous row ranges, both passes per phase) with the partial sums kept
+// by their owners; the chain of adds is the same.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstring>
+#include <vector>
+
+#include "nrldpc_internal.h"
+
+namespace nrldpc {
+namespace {
+
+constexpr int kSplitThreads = kSplitMaxWarps * 32;
+constexpr uint32_t kHdBit = 0x80000000u;  // state info: hard decision of the suffix posterior read
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) {
+    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+__device__ __forceinline__ float lds(uint32_t a) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void sts(uint32_t a, float v) {
+    asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+// Address of this CTA's shared address `a` in the CTA of rank `rank`.
+__device__ __forceinline__ uint32_t mapa(uint32_t a, uint32_t rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ uint32_t ldc_u32(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void stc(uint32_t a, float v) {
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+__device__ __forceinline__ void stc_u32(uint32_t a, uint32_t v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void stc_v4(uint32_t a, float4 v) {
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+                 : "memory");
+}
+// Barrier over every thread of the cluster; shared-memory writes before it
+// (local and remote) are seen after it.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t cluster_size() {
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
+// One lifted row: the arithmetic of decode.cu's row_update (flooding), with
+// dt of each core edge sent to its column's owner instead of added here.
+//   edge: the row's first {offset, wrap threshold, distance from a posterior
+//   to its edge's dt at the owner}; s4: shared address of the posteriors plus
+//   4*s; par: hard-decision parity of the posteriors read (bit 0).
+template <int D, bool WEIGHTED, bool ONE>
+__device__ __forceinline__ void cn_row(const uint4* edge, bool sfx, uint32_t s, uint32_t s4, uint32_t z4, uint4* state,
+                                       const float* wprev, const float* wcur, float alpha, bool check, uint32_t& par,
+                                       float& sfx_old) {
+    constexpr int LAST = D - 1;
+    constexpr bool kAgain = D > kSplitKeepTo;  // long rows: too many registers to keep the addresses
+    const uint4 st = *state;
+    uint32_t to[D];
+    float lv[D];
+#pragma unroll
+    for (int i = 0; i < D; i++) {
+        if (i == LAST && sfx) {
+            to[i] = 0;
+            lv[i] = __uint_as_float(st.w);
+        } else {
+            const uint4 ea = edge[i];
+            uint32_t a = s4 + ea.x;
+            if (s >= ea.y) a -= z4;
+            lv[i] = lds(a);
+            if (!kAgain) to[i] = a + ea.z;
+        }
+    }
+    if (check) {
+#pragma unroll
+        for (int i = 0; i < D; i++) par ^= lv[i] > 0.0f ? 0u : 1u;
+    }
+    const float om1 = __uint_as_float(st.x), om2 = __uint_as_float(st.y);
+    const uint32_t oinfo = st.z;
+    const int oidx = static_cast<int>(oinfo & 31u);
+    float oa1 = 0.0f, oa2 = 0.0f;
+    if (!WEIGHTED) {
+        oa1 = __fmul_rn(alpha, om1);
+        oa2 = __fmul_rn(alpha, om2);
+    }
+    float keep[D];
+    float m1 = 1000.0f, m2 = 1000.0f;
+    int idx = 0;
+    uint32_t qmask = 0;
+#pragma unroll
+    for (int i = 0; i < D; i++) {
+        float mag;
+        if (WEIGHTED)
+            mag = __fmul_rn(wprev[i], i == oidx ? om2 : om1);
+        else
+            mag = i == oidx ? oa2 : oa1;
+        const float ro = __uint_as_float(__float_as_uint(mag) ^ ((oinfo << (24 - D + i)) & 0x80000000u));
+        const float q = __fsub_rn(lv[i], ro);
+        keep[i] = ro;
+        const float qa = fabsf(q);
+        qmask = __funnelshift_l(__float_as_uint(__fadd_rn(q, 0.0f)), qmask, 1);  // edge i at bit D-1-i, -0 as +0
+        if (qa < m1) idx = i;
+        const float mx = max_nan(m1, qa);  // NaN |Q| leaves min1/min2 untouched
+        m1 = fminf(m1, qa);
+        m2 = fminf(m2, mx);
+    }
+    const uint32_t rsign = qmask ^ (0u - static_cast<uint32_t>(__popc(qmask) & 1));
+    float a1 = 0.0f, a2 = 0.0f;
+    if (!WEIGHTED) {
+        a1 = __fmul_rn(alpha, m1);
+        a2 = __fmul_rn(alpha, m2);
+    }
+    float sfx_new = 0.0f;
+#pragma unroll
+    for (int i = 0; i < D; i++) {
+        float mag;
+        if (WEIGHTED)
+            mag = __fmul_rn(wcur[i], i == idx ? m2 : m1);
+        else
+            mag = i == idx ? a2 : a1;
+        const float rn = __uint_as_float(__float_as_uint(mag) ^ ((rsign << (32 - D + i)) & 0x80000000u));
+        const float d = __fsub_rn(rn, keep[i]);
+        if (i == LAST && sfx) {
+            sfx_new = __fadd_rn(__uint_as_float(st.w), d);
+        } else {
+            uint32_t a = to[i];
+            if (kAgain) {
+                const uint4 ea = edge[i];
+                a = s4 + ea.x + ea.z;
+                if (s >= ea.y) a -= z4;
+            }
+            if (ONE)
+                sts(a, d);
+            else
+                stc(a, d);
+        }
+    }
+    sfx_old = __uint_as_float(st.w);
+    uint32_t info = static_cast<uint32_t>(idx) | ((rsign & ((1u << D) - 1u)) << 8);
+    if (!(sfx_old > 0.0f)) info |= kHdBit;
+    *state = make_uint4(__float_as_uint(m1), __float_as_uint(m2), info, __float_as_uint(sfx_new));
+}
+
+// Position of a suffix row's last column at sub-row s (rw.z: first position
+// of the column << 9 | shift).
+__device__ __forceinline__ int sfx_pos(const uint4& rw, uint32_t s, int z) {
+    int p = static_cast<int>(s + (rw.z & 511u));
+    if (p >= z) p -= z;
+    return static_cast<int>(rw.z >> 9) + p;
+}
+
+template <bool W>
+struct SplitWeights {
+    using type = NoWeights;
+};
+template <>
+struct SplitWeights<true> {
+    using type = WeightTable;
+};
+
+// Bound by SM issue in the check-node pass and, on large clusters, by the
+// distributed-shared-memory stores and the barriers (each waits for the stores
+// before it); 24 warps per CTA hide more of it than 16, and the 80 registers
+// that leaves hold a degree-19 row.  ONE: clusters of one CTA (small codes),
+// plain shared memory and CTA barriers.
+template <bool WEIGHTED, bool ONE>
+__global__ void __launch_bounds__(kSplitThreads, 1)
+    split_decode_kernel(const __grid_constant__ SplitArgs a, const __grid_constant__ typename SplitWeights<WEIGHTED>::type wt) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int rank = ONE ? 0 : static_cast<int>(cluster_rank()), C = ONE ? 1 : static_cast<int>(cluster_size());
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = blockDim.x, W = nt >> 5;
+    auto sync = [] {
+        if (ONE)
+            __syncthreads();
+        else
+            cluster_sync();
+    };
+    uint32_t* s_fail = reinterpret_cast<uint32_t*>(smem);  // [2] an unsatisfied row, by iteration parity
+    // the plan's head and this rank's tables; read where they are used, so
+    // that the row bodies have the registers
+    SplitHead* s_head = reinterpret_cast<SplitHead*>(smem + 16);
+    const volatile SplitHead& h = *s_head;
+    unsigned char* image = smem + kSplitHeader;
+    if (tid < 2) s_fail[tid] = 0;
+    const unsigned char* loaded = nullptr;
+    for (int item = blockIdx.x / C; item < a.n_cw; item += gridDim.x / C) {
+        const unsigned char* plan = a.plan;
+        int cw = item;
+        const float* llr = a.llr;
+        uint8_t* packed = a.packed;
+        if (a.jobs) {
+            const SplitJob j = a.jobs[item];
+            plan += j.plan;
+            cw = j.job;
+            llr += j.llr_offset;
+            packed += j.out_offset;
+        }
+        sync();  // every CTA runs, and is done with the previous codeword
+        if (plan != loaded) {
+            if (tid < static_cast<int>(sizeof(SplitHead) / 4))
+                reinterpret_cast<int*>(s_head)[tid] = reinterpret_cast<const int*>(plan)[tid];
+            const int bytes = reinterpret_cast<const SplitHead*>(plan)->image_bytes;
+            const uint4* src = reinterpret_cast<const uint4*>(plan + sizeof(SplitHead) + static_cast<size_t>(rank) * bytes);
+            for (int k = tid; k < bytes / 16; k += nt) reinterpret_cast<uint4*>(image)[k] = src[k];
+            __syncthreads();
+        }
+        const int z = h.z, P = h.phases;
+        const uint32_t z4 = 4u * static_cast<uint32_t>(z);
+        if (!a.jobs) {
+            llr += static_cast<size_t>(cw) * h.n_bp;
+            packed += static_cast<size_t>(cw) * h.packed_bytes;
+        }
+        const uint32_t l_addr = smem_u32(smem) + h.off_l, dt_addr = smem_u32(smem) + h.off_dt;
+        float* app = a.app ? a.app + static_cast<size_t>(cw) * h.n_bp : nullptr;
+        {   // core LLRs: the whole copy by each CTA, or (host memory) its share, sent to all
+            const int total = h.core_floats / 4;
+            const int per = a.llr_from_host ? (total + C - 1) / C : total;
+            const int lo = a.llr_from_host ? rank * per : 0, hi = min(total, lo + per);
+            for (int m = lo + tid; m < hi; m += nt) {
+                const float4 v = __ldcs(reinterpret_cast<const float4*>(llr) + m);
+                if (!ONE && a.llr_from_host)
+                    for (int q = 0; q < C; q++) stc_v4(mapa(l_addr + 16u * m, q), v);
+                else
+                    reinterpret_cast<float4*>(smem + h.off_l)[m] = v;
+            }
+        }
+        if (plan != loaded) {  // dt place at the owner -> distance from the posterior to it
+            uint4* edge = reinterpret_cast<uint4*>(image + h.o_edge);
+            for (int k = tid; k < h.n_edges; k += nt) {
+                const uint32_t to = edge[k].z, block = edge[k].x - 4u * (static_cast<uint32_t>(z) - edge[k].y);
+                const uint32_t base = ONE ? dt_addr : mapa(dt_addr, to >> 24);
+                edge[k].z = base + (to & 0xffffffu) * z4 - (l_addr + block);
+            }
+            loaded = plan;
+        }
+        {   // zero states with the suffix LLRs: R_old = +0 in the first iteration
+            const uint16_t* cn = reinterpret_cast<const uint16_t*>(image + h.o_cn);
+            const int n_cn = reinterpret_cast<const uint16_t*>(image + h.o_cnptr)[P * W];
+            for (int k = warp; k < n_cn; k += W) {
+                const uint4 rw = reinterpret_cast<const uint4*>(image + h.o_row)[cn[k] >> 4];
+                const uint32_t s = static_cast<uint32_t>((cn[k] & 15) * 32 + lane);
+                if (s >= static_cast<uint32_t>(z)) continue;
+                float w = 0.0f;
+                if (rw.w >> 8) w = __ldcs(llr + sfx_pos(rw, s, z));
+                reinterpret_cast<uint4*>(smem + h.off_state)[rw.y + s] = make_uint4(0u, 0u, 0u, __float_as_uint(w));
+            }
+        }
+        sync();
+        int it = a.n_iter;
+        bool conv = false;
+        for (int t = 0; t < a.n_iter && !conv; t++) {
+            const bool check = a.early_stop && t > 0;
+            const float* wprev = nullptr;
+            const float* wcur = nullptr;
+            if constexpr (WEIGHTED) {
+                wprev = wt.w[t == 0 ? kMaxWIters : min(t - 1, a.n_w_iters - 1)];
+                wcur = wt.w[min(t, a.n_w_iters - 1)];
+            }
+            for (int p = 0; p < P; p++) {
+                const uint16_t* cnptr = reinterpret_cast<const uint16_t*>(image + h.o_cnptr) + p * W + warp;
+                const uint16_t* cn = reinterpret_cast<const uint16_t*>(image + h.o_cn);
+                uint4* states = reinterpret_cast<uint4*>(smem + h.off_state);
+                const int k1 = cnptr[1];
+                for (int k = cnptr[0]; k < k1; k++) {
+                    const int task = cn[k];
+                    const uint32_t s = static_cast<uint32_t>((task & 15) * 32 + lane);
+                    const uint4 rw = reinterpret_cast<const uint4*>(image + h.o_row)[task >> 4];
+                    uint32_t bad = 0;
+                    if (s < static_cast<uint32_t>(z)) {
+                        const bool sfx = (rw.w >> 8) != 0;
+                        float sfx_old = 0.0f;
+                        const uint4* edge = reinterpret_cast<const uint4*>(image + h.o_edge) + (rw.x & 0xffffu);
+                        const uint32_t we = WEIGHTED ? rw.x >> 16 : 0u;
+                        switch (rw.w & 255u) {
+#define NRLDPC_CN_CASE(D)                                                                                             \
+    case D:                                                                                                           \
+        cn_row<D, WEIGHTED, ONE>(edge, sfx, s, l_addr + 4u * s, z4, states + rw.y + s, WEIGHTED ? wprev + we : nullptr, \
+                                 WEIGHTED ? wcur + we : nullptr, a.alpha, check, bad, sfx_old);                       \
+        break;
+                            NRLDPC_CN_CASE(1) NRLDPC_CN_CASE(2) NRLDPC_CN_CASE(3) NRLDPC_CN_CASE(4)
+                            NRLDPC_CN_CASE(5) NRLDPC_CN_CASE(6) NRLDPC_CN_CASE(7) NRLDPC_CN_CASE(8)
+                            NRLDPC_CN_CASE(9) NRLDPC_CN_CASE(10) NRLDPC_CN_CASE(11) NRLDPC_CN_CASE(12)
+                            NRLDPC_CN_CASE(13) NRLDPC_CN_CASE(14) NRLDPC_CN_CASE(15) NRLDPC_CN_CASE(16)
+                            NRLDPC_CN_CASE(17) NRLDPC_CN_CASE(18) NRLDPC_CN_CASE(19)
+#undef NRLDPC_CN_CASE
+                            default:
+                                break;
+                        }
+                        // the posterior the codeword leaves with if it stops here
+                        if (check && app && sfx) app[sfx_pos(rw, s, z)] = sfx_old;
+                    }
+                    if (check && __any_sync(0xffffffffu, bad & 1u) && lane < C) {
+                        const uint32_t f = smem_u32(&s_fail[t & 1]);
+                        if (ONE)
+                            s_fail[t & 1] = 1u;
+                        else
+                            stc_u32(mapa(f, lane), 1u);
+                    }
+                }
+                sync();  // the dt of this phase, and (last phase) the failures, are in place
+                if (check && p == P - 1 && s_fail[t & 1] == 0) {
+                    conv = true;  // iteration t - 1 left a codeword: t iterations ran
+                    it = t;
+                    break;
+                }
+                const uint16_t* vnptr = reinterpret_cast<const uint16_t*>(image + h.o_vnptr) + warp;
+                const uint16_t* vn = reinterpret_cast<const uint16_t*>(image + h.o_vn);
+                const int v1 = vnptr[1];
+                for (int k = vnptr[0]; k < v1; k++) {
+                    const int task = vn[k];
+                    const uint32_t pos = static_cast<uint32_t>((task & 15) * 32 + lane);
+                    const uint4 cm = reinterpret_cast<const uint4*>(image + h.o_col)[task >> 4];  // L offset, readers
+                    const uint32_t be = reinterpret_cast<const uint32_t*>(image + h.o_beg)[(task >> 4) * P + p];
+                    if (pos >= static_cast<uint32_t>(z)) continue;
+                    const uint32_t la = l_addr + cm.x + 4u * pos;
+                    uint32_t d = dt_addr + (be & 0xffffu) * z4 + 4u * pos;
+                    float* acc = reinterpret_cast<float*>(smem + h.off_acc) + k * 32 + lane;
+                    float v = p == 0 ? lds(la) : *acc;
+                    for (int m = static_cast<int>(be >> 16); m > 0; m -= kSplitVnAhead) {
+                        float x[kSplitVnAhead];
+#pragma unroll
+                        for (int i = 0; i < kSplitVnAhead; i++) {
+                            if (i < m) x[i] = lds(d);
+                            d += z4;
+                        }
+#pragma unroll
+                        for (int i = 0; i < kSplitVnAhead; i++)
+                            if (i < m) v = __fadd_rn(v, x[i]);
+                    }
+                    if (p < P - 1) {
+                        *acc = v;
+                    } else if (ONE) {
+                        sts(la, v);
+                    } else {
+                        for (uint32_t m = cm.y; m; m &= m - 1) stc(mapa(la, __ffs(m) - 1), v);
+                    }
+                }
+                sync();  // posteriors (last phase) or dt buffers free for the next pass
+                if (tid == 0 && p == P - 1) s_fail[t & 1] = 0;  // written again two iterations on
+            }
+        }
+        // Packed hard decisions (and posteriors): 32 positions per warp.
+        const int n = h.n_bp, packed_bytes = h.packed_bytes, nc = h.n_core;
+        const uint32_t* owners = reinterpret_cast<const uint32_t*>(image + h.o_own);
+        const bool word_store = (reinterpret_cast<uintptr_t>(packed) & 3u) == 0;
+        for (int w = rank * W + warp; w * 32 < n; w += C * W) {
+            const int pos = w * 32 + lane;
+            uint32_t one = 0;
+            if (pos < n) {
+                const int c = pos / z;
+                const uint32_t own = owners[c];  // rank << 28 | state offset or 0 | shift
+                uint32_t sa = l_addr + 4u * pos, word = 0;
+                if (c >= nc) {
+                    int s = pos - c * z - static_cast<int>(own & 511u);
+                    if (s < 0) s += z;
+                    sa = smem_u32(smem) + h.off_state + 16u * (((own >> 9) & 0x7ffffu) + s) + (conv ? 8u : 12u);
+                }
+                word = ONE ? __float_as_uint(lds(sa)) : ldc_u32(mapa(sa, own >> 28));
+                if (c >= nc && conv) {
+                    one = word >> 31;
+                } else {
+                    one = __uint_as_float(word) > 0.0f ? 0u : 1u;
+                    if (app) app[pos] = __uint_as_float(word);
+                }
+            }
+            const uint32_t word = __ballot_sync(0xffffffffu, one);
+            const int b = 4 * w;
+            if (word_store && b + 4 <= packed_bytes) {
+                if (lane == 0) *reinterpret_cast<uint32_t*>(packed + b) = word;
+            } else if (lane < 4 && b + lane < packed_bytes) {
+                packed[b + lane] = static_cast<uint8_t>(word >> (8 * lane));
+            }
+        }
+        if (a.iters && rank == 0 && tid == 0) a.iters[cw] = it;
+    }
+    sync();  // no CTA leaves while another reads its shared memory
+}
+
+// Lists of task[i] (cost[i], largest first) for n_bins warps, each task to
+// the least loaded: ptr[0..n_bins] and the tasks bin by bin.
+void spread(const std::vector<std::pair<int, int>>& tasks, int n_bins, int from, uint16_t* ptr, uint16_t* out) {
+    int load[kSplitMaxWarps] = {0}, count[kSplitMaxWarps + 1] = {0}, bin[kMaxCols * 12];
+    for (size_t i = 0; i < tasks.size(); i++) {
+        int b = 0;
+        for (int j = 1; j < n_bins; j++)
+            if (load[j] < load[b]) b = j;
+        bin[i] = b;
+        load[b] += tasks[i].first;
+        count[b + 1]++;
+    }
+    for (int b = 0; b < n_bins; b++) {
+        count[b + 1] += count[b];
+        ptr[b] = static_cast<uint16_t>(from + count[b]);
+    }
+    ptr[n_bins] = static_cast<uint16_t>(from + count[n_bins]);
+    for (size_t i = 0; i < tasks.size(); i++) out[from + count[bin[i]]++] = static_cast<uint16_t>(tasks[i].second);
+}
+
+}  // namespace
+
+// Rows and columns to CTAs, tasks to warps and the shared-memory layout for
+// clusters of `ranks` CTAs: appends the head and one table image per rank to
+// `out`.  False when the code does not fit such clusters.
+bool make_split_plan(const CodeTable& t, int ranks, size_t smem_limit, SplitHead* head,
+                     std::vector<unsigned char>* out) {
+    const int chunks = (t.z + 31) / 32, rows = t.rows, nc = t.n_core;
+    int core[kMaxRows], col_deg[kMaxCols] = {0}, col_row[kMaxCols][kMaxRows], col_edge[kMaxCols][kMaxRows], total = 0;
+    for (int r = 0; r < rows; r++) {  // rows and edges of each column, ascending
+        core[r] = t.row_deg[r] - (t.row_sfx[r] ? 1 : 0);
+        total += core[r];
+        for (int e = t.row_ptr[r]; e < t.row_ptr[r + 1]; e++) {
+            const int c = t.edge_col[e];
+            col_row[c][col_deg[c]] = r;
+            col_edge[c][col_deg[c]++] = e;
+        }
+    }
+    // the posteriors and an even share of the states have to fit whatever the phases
+    if (4 * static_cast<size_t>(t.core_floats) + 16 * static_cast<size_t>((rows + ranks - 1) / ranks) * t.z > smem_limit)
+        return false;
+    for (int P = 1; P <= kSplitMaxPhases && P <= rows; P++) {
+        // phases: contiguous rows, about the same edges each
+        int phase_of[kMaxRows], sum = 0;
+        for (int r = 0; r < rows; r++) {
+            phase_of[r] = std::min(P - 1, static_cast<int>(static_cast<long>(sum + core[r] / 2) * P / std::max(1, total)));
+            sum += core[r];
+        }
+        // columns to ranks, largest degree first, to the rank with the least
+        // dt; dt places of a column's edges, ascending rows, per phase
+        int col_rank[kMaxCols], col_beg[kMaxCols][kSplitMaxPhases], col_cnt[kMaxCols][kSplitMaxPhases];
+        int dt_of[kMaxEdges], deg_sum[kSplitMaxRanks] = {0}, dt[kSplitMaxRanks][kSplitMaxPhases] = {{0}}, max_dt = 0;
+        std::vector<int> cols(nc), local_cols[kSplitMaxRanks];
+        for (int c = 0; c < nc; c++) cols[c] = c;
+        std::stable_sort(cols.begin(), cols.end(), [&](int x, int y) { return col_deg[x] > col_deg[y]; });
+        for (int c : cols) {
+            int k = 0;
+            for (int j = 1; j < ranks; j++)
+                if (deg_sum[j] < deg_sum[k]) k = j;
+            col_rank[c] = k;
+            deg_sum[k] += col_deg[c] + kSplitColCost;
+            local_cols[k].push_back(c);
+            for (int p = 0; p < P; p++) col_beg[c][p] = dt[k][p];
+            for (int i = 0; i < col_deg[c]; i++) dt_of[col_edge[c][i]] = dt[k][phase_of[col_row[c][i]]]++;
+            for (int p = 0; p < P; p++) {
+                col_cnt[c][p] = dt[k][p] - col_beg[c][p];
+                max_dt = std::max(max_dt, dt[k][p]);
+            }
+        }
+        // rows of a phase to ranks, largest degree first, to the rank with
+        // the least work in the phase (then the fewest rows so far)
+        int row_rank[kMaxRows], row_at[kMaxRows];
+        std::vector<int> local_rows[kSplitMaxRanks];
+        std::vector<std::pair<int, int>> list[kSplitMaxRanks][kSplitMaxPhases];
+        int busiest = 0;  // summed over the phases
+        for (int p = 0; p < P; p++) {
+            std::vector<int> order;
+            for (int r = 0; r < rows; r++)
+                if (phase_of[r] == p) order.push_back(r);
+            std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return t.row_deg[x] > t.row_deg[y]; });
+            int load[kSplitMaxRanks] = {0};
+            for (int r : order) {
+                int k = 0;
+                for (int j = 1; j < ranks; j++)
+                    if (load[j] < load[k] || (load[j] == load[k] && local_rows[j].size() < local_rows[k].size())) k = j;
+                row_rank[r] = k;
+                row_at[r] = static_cast<int>(local_rows[k].size());
+                local_rows[k].push_back(r);
+                load[k] += t.row_deg[r] + kSplitRowCost;
+                for (int c = 0; c < chunks; c++)
+                    list[k][p].push_back({t.row_deg[r] + kSplitRowCost, (row_at[r] << 4) | c});
+            }
+            busiest += chunks * *std::max_element(load, load + ranks);
+        }
+        size_t n_rows = 0, n_cols = 0, most = 0, n_edges = 0, n_cn = 0;
+        for (int k = 0; k < ranks; k++) {
+            size_t e = 0, cn = 0;
+            for (int r : local_rows[k]) e += t.row_deg[r];
+            for (int p = 0; p < P; p++) {
+                most = std::max(most, list[k][p].size());
+                cn += list[k][p].size();
+            }
+            n_edges = std::max(n_edges, e);
+            n_cn = std::max(n_cn, cn);
+            n_rows = std::max(n_rows, local_rows[k].size());
+            n_cols = std::max(n_cols, local_cols[k].size());
+        }
+        const int W = std::max(4, std::min(kSplitMaxWarps, static_cast<int>(std::max(most, n_cols * chunks))));
+        // image layout (the same for every rank) and shared memory
+        size_t at = 0;
+        auto take = [&](size_t bytes) {
+            const size_t here = at;
+            at += (bytes + 15) / 16 * 16;
+            return static_cast<int>(here);
+        };
+        SplitHead h{};
+        h.z = t.z;
+        h.n_bp = t.n_bp;
+        h.packed_bytes = t.packed_bytes;
+        h.n_core = nc;
+        h.core_floats = t.core_floats;
+        h.ranks = ranks;
+        h.phases = P;
+        h.warps = W;
+        h.n_edges = static_cast<int>(n_edges);
+        h.load = busiest;
+        h.o_edge = take(16 * n_edges);
+        h.o_row = take(16 * n_rows);
+        h.o_col = take(16 * n_cols);
+        h.o_beg = take(4 * n_cols * P);
+        h.o_own = take(4 * static_cast<size_t>(t.cols));
+        h.o_cnptr = take(2 * (static_cast<size_t>(P) * W + 1));
+        h.o_cn = take(2 * n_cn);
+        h.o_vnptr = take(2 * (static_cast<size_t>(W) + 1));
+        h.o_vn = take(2 * n_cols * chunks);
+        h.image_bytes = static_cast<int>(at);
+        auto up = [](size_t x) { return (x + 127) / 128 * 128; };
+        const size_t l = up(kSplitHeader + at), st = up(l + 4 * static_cast<size_t>(t.core_floats)),
+                     d = up(st + 16 * n_rows * t.z), acc = up(d + 4 * static_cast<size_t>(max_dt) * t.z),
+                     end = acc + (P > 1 ? 128 * n_cols * chunks : 0);
+        if (end > smem_limit) continue;
+        h.off_l = static_cast<int>(l);
+        h.off_state = static_cast<int>(st);
+        h.off_dt = static_cast<int>(d);
+        h.off_acc = static_cast<int>(acc);
+        h.smem = static_cast<int>(end);
+        // the images
+        const size_t base = out->size();
+        out->resize(base + sizeof(SplitHead) + static_cast<size_t>(ranks) * at, 0);
+        std::memcpy(out->data() + base, &h, sizeof(h));
+        for (int k = 0; k < ranks; k++) {
+            unsigned char* im = out->data() + base + sizeof(SplitHead) + static_cast<size_t>(k) * at;
+            auto* edge = reinterpret_cast<uint4*>(im + h.o_edge);
+            auto* row = reinterpret_cast<uint4*>(im + h.o_row);
+            auto* col = reinterpret_cast<uint4*>(im + h.o_col);
+            auto* beg = reinterpret_cast<uint32_t*>(im + h.o_beg);
+            auto* own = reinterpret_cast<uint32_t*>(im + h.o_own);
+            auto* cnptr = reinterpret_cast<uint16_t*>(im + h.o_cnptr);
+            auto* cn = reinterpret_cast<uint16_t*>(im + h.o_cn);
+            auto* vnptr = reinterpret_cast<uint16_t*>(im + h.o_vnptr);
+            auto* vn = reinterpret_cast<uint16_t*>(im + h.o_vn);
+            uint32_t m = 0;
+            for (size_t i = 0; i < local_rows[k].size(); i++) {
+                const int r = local_rows[k][i], last = t.row_ptr[r + 1] - 1;
+                row[i] = make_uint4(m | (static_cast<uint32_t>(t.row_ptr[r]) << 16), static_cast<uint32_t>(i) * t.z,
+                                    ((static_cast<uint32_t>(t.edge_col[last]) * t.z) << 9) | t.edge_shift[last],
+                                    t.row_deg[r] | (t.row_sfx[r] ? 256u : 0u));
+                for (int e = t.row_ptr[r]; e <= last; e++, m++) {
+                    const int c = t.edge_col[e];
+                    edge[m] = make_uint4(t.eaddr[e].x, t.eaddr[e].y, 0u, 0u);
+                    if (c < nc) edge[m].z = (static_cast<uint32_t>(col_rank[c]) << 24) | static_cast<uint32_t>(dt_of[e]);
+                }
+            }
+            std::vector<std::pair<int, int>> vl;
+            for (size_t i = 0; i < local_cols[k].size(); i++) {
+                const int c = local_cols[k][i];
+                uint32_t need = 1u << k;  // its owner (for the output) and every rank with a row that reads it
+                for (int j = 0; j < col_deg[c]; j++) need |= 1u << row_rank[col_row[c][j]];
+                col[i] = make_uint4(4u * static_cast<uint32_t>(c) * t.z, need, 0u, 0u);
+                for (int p = 0; p < P; p++)
+                    beg[i * P + p] = static_cast<uint32_t>(col_beg[c][p]) | (static_cast<uint32_t>(col_cnt[c][p]) << 16);
+                for (int j = 0; j < chunks; j++)
+                    vl.push_back({col_deg[c] + kSplitColCost, (static_cast<int>(i) << 4) | j});
+            }
+            for (int c = 0; c < nc; c++) own[c] = static_cast<uint32_t>(col_rank[c]) << 28;
+            for (int c = nc; c < t.cols; c++) {
+                const int r = t.sfx_row[c];
+                own[c] = (static_cast<uint32_t>(row_rank[r]) << 28) | (static_cast<uint32_t>(row_at[r] * t.z) << 9) |
+                         t.edge_shift[t.row_ptr[r + 1] - 1];
+            }
+            int n = 0;
+            for (int p = 0; p < P; p++) {
+                spread(list[k][p], W, n, cnptr + p * W, cn);
+                n += static_cast<int>(list[k][p].size());
+            }
+            spread(vl, W, 0, vnptr, vn);
+        }
+        *head = h;
+        return true;
+    }
+    return false;
+}
+
+namespace {
+const void* split_kernel(bool weighted, bool one) {
+    if (one)
+        return weighted ? reinterpret_cast<const void*>(&split_decode_kernel<true, true>)
+                        : reinterpret_cast<const void*>(&split_decode_kernel<false, true>);
+    return weighted ? reinterpret_cast<const void*>(&split_decode_kernel<true, false>)
+                    : reinterpret_cast<const void*>(&split_decode_kernel<false, false>);
+}
+void split_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, const SplitHead& h, int n_clusters,
+                  cudaStream_t stream) {
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = static_cast<unsigned>(h.ranks);
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    cfg->gridDim = dim3(static_cast<unsigned>(h.ranks * n_clusters));
+    cfg->blockDim = dim3(static_cast<unsigned>(h.warps * 32));
+    cfg->dynamicSmemBytes = static_cast<size_t>(h.smem);
+    cfg->stream = stream;
+    cfg->attrs = attr;
+    cfg->numAttrs = 1;
+}
+}  // namespace
+
+cudaError_t split_kernel_attributes(size_t smem) {
+    for (int w = 0; w < 4; w++) {
+        const void* k = split_kernel((w & 1) != 0, (w & 2) != 0);
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+int split_max_clusters(const SplitHead& h) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+    split_config(&cfg, &attr, h, 1, nullptr);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, split_kernel(false, h.ranks == 1), &cfg) != cudaSuccess) {
+        cudaGetLastError();  // clusters of this size are not available
+        return 0;
+    }
+    return n;
+}
+
+cudaError_t launch_split(const SplitHead& h, const SplitArgs& args, const WeightTable* weights, int n_clusters,
+                         cudaStream_t stream) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+    split_config(&cfg, &attr, h, n_clusters, stream);
+    NoWeights none{};
+    void* params[2] = {const_cast<SplitArgs*>(&args),
+                       weights ? const_cast<WeightTable*>(weights) : static_cast<void*>(&none)};
+    return cudaLaunchKernelExC(&cfg, split_kernel(weights != nullptr, h.ranks == 1), params);
+}
+
+}  // namespace nrldpc
