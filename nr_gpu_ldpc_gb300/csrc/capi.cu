@@ -172,12 +172,6 @@ void free_handle(Handle* h) {
     delete h;
 }
 
-// Cluster sizes tried for small batches: each holds more codewords at once
-// than the one before (GB300 at one CTA per SM: 7, 13, 23, 28, 36, 46, 76 and
-// 152 clusters; a GPC's SMs do not divide evenly by the other sizes).
-const int kSplitRanks[] = {16, 10, 6, 5, 4, 3, 2, 1};
-constexpr int kSplitMinTasks = 12;  // 32-sub-row tasks per CTA worth a larger cluster
-
 // Plans for the cluster sizes that fit; their bytes go behind the handle's
 // scratch words in device memory.
 int split_prepare(Handle* h, size_t smem_limit, std::vector<unsigned char>* bytes) {
@@ -201,20 +195,14 @@ int split_prepare(Handle* h, size_t smem_limit, std::vector<unsigned char>* byte
 }
 
 // Plan for n codewords, or -1 for decode_kernel: the smaller of two time
-// estimates, in edges of one warp (45 ns per 10 iterations).  A wave of
-// clusters takes kSplitFixed per phase (barriers, the passes' latency) plus
-// the busiest CTA's edges; decode_kernel's walk down the rows costs per row
-// and edge, more with more warps on the SM.  Fitted to GB300 times, 10
+// estimates (split_cost, fused_row_walk).  Fitted to GB300 times, 10
 // iterations, us (model): BG1 Z=384 on 16 / 8 / 4 / 3 CTAs 52 / 68 / 103 / 151
 // (47 / 64 / 98 / 150), BG2 Z=384 40 / 48 / 72 / 89, BG1 Z=96 on 4 / 2 / 1
 // CTAs 42 / 59 / 81 (47 / 64 / 98); decode_kernel BG1 Z=384 / 208 / 96 at one
 // CTA per SM 300 / 245 / 204 (300 / 248 / 207), BG2 Z=384 / 128 219 / 157, two
 // CTAs per SM 1.5-1.65 times that.
-constexpr long kSplitFixed = 667;
-
 long fused_cost(const Handle* h, int n) {
-    const long groups = (n + h->cpb - 1) / h->cpb, w = h->threads / 32;
-    const long one = h->tab.rows * (29 + 21 * w / 10) + h->tab.n_edges * (81 + 4 * w) / 10;
+    const long groups = (n + h->cpb - 1) / h->cpb, one = fused_row_walk(h->tab, h->threads / 32);
     long cost = groups / h->max_grid * (one * (4 + 2 * h->ctas_per_sm) / 5);
     const long rest = groups % h->max_grid;
     if (rest) cost += one * (3 + 2 * ((rest + h->sm_count - 1) / h->sm_count)) / 5;
@@ -226,7 +214,7 @@ int split_choice(const Handle* h, int n) {
     long least = fused_cost(h, n);
     for (size_t k = 0; k < h->split.size(); k++) {
         const long waves = (n + h->split_room[k] - 1) / h->split_room[k];
-        const long cost = waves * (kSplitFixed * h->split[k].phases + h->split[k].load);
+        const long cost = waves * split_cost(h->split[k]);
         if (cost < least) {
             least = cost;
             best = static_cast<int>(k);
@@ -857,12 +845,8 @@ int nrldpc_cb_segment(const uint8_t* d_tb, const nrldpc_segment_info* info, uint
         info->k_prime <= info->L || block_stride * 8 < info->k_prime)
         return NRLDPC_ERR_INVALID_ARG;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    const int data_bits = info->k_prime - info->L;
-    if (launch_cb_gather_blocks(d_tb, info->C, data_bits, info->k_prime, d_blocks, block_stride, st) !=
-        cudaSuccess)
-        return NRLDPC_ERR_CUDA;
-    if (info->L == 0) return NRLDPC_OK;
-    return map_cuda(launch_cb_attach_crc(d_blocks, info->C, data_bits, block_stride, 0x800063u, 24, st));
+    return map_cuda(launch_cb_segment(d_tb, info->C, info->k_prime - info->L, info->k_prime, d_blocks, block_stride,
+                                      0x800063u, info->L > 0 ? 24 : 0, st));
 }
 
 int nrldpc_cb_desegment(const uint8_t* d_blocks, int block_stride, const nrldpc_segment_info* info,
@@ -871,10 +855,8 @@ int nrldpc_cb_desegment(const uint8_t* d_blocks, int block_stride, const nrldpc_
         info->k_prime <= info->L || block_stride * 8 < info->k_prime || (info->L > 0 && !d_crc_rem))
         return NRLDPC_ERR_INVALID_ARG;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    if (info->L > 0 &&
-        launch_crc(d_blocks, info->C, block_stride, info->k_prime, 0x800063u, 24, d_crc_rem, st) != cudaSuccess)
-        return NRLDPC_ERR_CUDA;
-    return map_cuda(launch_cb_gather_tb(d_blocks, block_stride, info->C, info->k_prime - info->L, d_tb, st));
+    return map_cuda(launch_cb_desegment(d_blocks, block_stride, info->C, info->k_prime - info->L, info->k_prime, d_tb,
+                                        0x800063u, info->L > 0 ? 24 : 0, d_crc_rem, st));
 }
 
 int nrldpc_device_error(nrldpc_handle* handle) {

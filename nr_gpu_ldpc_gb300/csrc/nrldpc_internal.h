@@ -160,6 +160,20 @@ struct SplitArgs {
     int n_cw, n_iter, n_w_iters, early_stop, llr_from_host;
     float alpha;
 };
+// Cluster sizes tried: each holds more codewords at once than the one before
+// (GB300 at one CTA per SM: 7, 13, 23, 28, 36, 46, 76 and 152 clusters; a
+// GPC's SMs do not divide evenly by the other sizes).
+constexpr int kSplitRanks[] = {16, 10, 6, 5, 4, 3, 2, 1};
+constexpr int kSplitSizes = 8;
+constexpr int kSplitMinTasks = 12;  // 32-sub-row tasks per CTA worth a larger cluster
+// Time estimates of the two decoders, in edges of one warp (45 ns per 10
+// iterations on GB300): one wave of clusters takes 667 per phase (barriers,
+// the passes' latency) plus the busiest CTA's edges; decode_kernel's walk down
+// the rows costs per row and edge, more with more warps in the CTA.
+inline long split_cost(const SplitHead& h) { return 667L * h.phases + h.load; }
+inline long fused_row_walk(const CodeTable& t, long warps) {
+    return t.rows * (29 + 21 * warps / 10) + t.n_edges * (81 + 4 * warps) / 10;
+}
 bool make_split_plan(const CodeTable& tab, int ranks, size_t smem_limit, SplitHead* head,
                      std::vector<unsigned char>* out);
 cudaError_t split_kernel_attributes(size_t smem);
@@ -206,15 +220,13 @@ cudaError_t launch_dequant(const void* in, int qtype, float scale, size_t n, flo
                            cudaStream_t stream);
 cudaError_t launch_crc(const uint8_t* packed, int n_cw, int stride, int n_bits, uint32_t poly, int len,
                        uint32_t* rem, cudaStream_t stream);
-// Code-block segmentation (channel.cu): bit gathers between a transport
-// block and C code blocks of k_prime bits (data_bits = k_prime - L each), and
-// CRC attachment of the last L bits of each block.
-cudaError_t launch_cb_gather_blocks(const uint8_t* tb, int C, int data_bits, int k_prime, uint8_t* blocks,
-                                    int stride, cudaStream_t stream);
-cudaError_t launch_cb_attach_crc(uint8_t* blocks, int C, int data_bits, int stride, uint32_t poly, int len,
-                                 cudaStream_t stream);
-cudaError_t launch_cb_gather_tb(const uint8_t* blocks, int stride, int C, int data_bits, uint8_t* tb,
-                                cudaStream_t stream);
+// Code-block segmentation (channel.cu): between a transport block and C code
+// blocks of k_prime bits (data_bits of it data), with a CRC of len bits
+// attached to or checked over each block (len 0: none).
+cudaError_t launch_cb_segment(const uint8_t* tb, int C, int data_bits, int k_prime, uint8_t* blocks, int stride,
+                              uint32_t poly, int len, cudaStream_t stream);
+cudaError_t launch_cb_desegment(const uint8_t* blocks, int stride, int C, int data_bits, int k_prime, uint8_t* tb,
+                                uint32_t poly, int len, uint32_t* rem, cudaStream_t stream);
 cudaError_t launch_count_errors(const uint8_t* packed, const uint8_t* cw_packed, int n_cw,
                                 int packed_bytes, int n_info, unsigned long long* counts,
                                 cudaStream_t stream);

@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
             for (int k = tid; k < bytes / 16; k += nt) reinterpret_cast<uint4*>(image)[k] = src[k];
             __syncthreads();
         }
-        const int z = h.z, P = h.phases;
+        const int z = h.z, P = h.phases, lists = h.warps;  // warps with task lists (a mixed batch's CTA may have more)
         const uint32_t z4 = 4u * static_cast<uint32_t>(z);
         if (!a.jobs) {
             llr += static_cast<size_t>(cw) * h.n_bp;
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
         }
         {   // zero states with the suffix LLRs: R_old = +0 in the first iteration
             const uint16_t* cn = reinterpret_cast<const uint16_t*>(image + h.o_cn);
-            const int n_cn = reinterpret_cast<const uint16_t*>(image + h.o_cnptr)[P * W];
+            const int n_cn = reinterpret_cast<const uint16_t*>(image + h.o_cnptr)[P * lists];
             for (int k = warp; k < n_cn; k += W) {
                 const uint4 rw = reinterpret_cast<const uint4*>(image + h.o_row)[cn[k] >> 4];
                 const uint32_t s = static_cast<uint32_t>((cn[k] & 15) * 32 + lane);
@@ -311,11 +311,11 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
                 wcur = wt.w[min(t, a.n_w_iters - 1)];
             }
             for (int p = 0; p < P; p++) {
-                const uint16_t* cnptr = reinterpret_cast<const uint16_t*>(image + h.o_cnptr) + p * W + warp;
+                const uint16_t* cnptr = reinterpret_cast<const uint16_t*>(image + h.o_cnptr) + p * lists + warp;
                 const uint16_t* cn = reinterpret_cast<const uint16_t*>(image + h.o_cn);
                 uint4* states = reinterpret_cast<uint4*>(smem + h.off_state);
-                const int k1 = cnptr[1];
-                for (int k = cnptr[0]; k < k1; k++) {
+                const int k1 = warp < lists ? cnptr[1] : 0;
+                for (int k = warp < lists ? cnptr[0] : 0; k < k1; k++) {
                     const int task = cn[k];
                     const uint32_t s = static_cast<uint32_t>((task & 15) * 32 + lane);
                     const uint4 rw = reinterpret_cast<const uint4*>(image + h.o_row)[task >> 4];
@@ -359,8 +359,8 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
                 }
                 const uint16_t* vnptr = reinterpret_cast<const uint16_t*>(image + h.o_vnptr) + warp;
                 const uint16_t* vn = reinterpret_cast<const uint16_t*>(image + h.o_vn);
-                const int v1 = vnptr[1];
-                for (int k = vnptr[0]; k < v1; k++) {
+                const int v1 = warp < lists ? vnptr[1] : 0;
+                for (int k = warp < lists ? vnptr[0] : 0; k < v1; k++) {
                     const int task = vn[k];
                     const uint32_t pos = static_cast<uint32_t>((task & 15) * 32 + lane);
                     const uint4 cm = reinterpret_cast<const uint4*>(image + h.o_col)[task >> 4];  // L offset, readers
