@@ -158,33 +158,60 @@ struct DerateArgs {
     const JobDev* jobs;
     const float* llr_e;
     float* llr;
-    int n_jobs;
+    int n_jobs, parts, part;
 };
 
-// One CTA per job.  Each non-filler position c of the compressed buffer
-// collects bits k = k_first, k_first + Nc, ... (< e) in order, each read from
-// its interleaved position; the first copy is taken as is, later copies added.
+// Each job's output in `parts` parts of `part` positions or interleaver rows,
+// one CTA per (job, part) at a time: as many parts as it takes for a few jobs
+// to fill the GPU, one where the jobs do (nrldpc_batch_set_jobs).  Without repetition (e <= Nc) every bit k lands at one position of the
+// compressed buffer: a thread takes one interleaver row, reads its qm
+// neighbouring LLRs (bits i, i + E/qm, ...) and writes each beside its
+// neighbours' -- reads and writes both in order, no division per bit.  With
+// repetition each position c collects bits k = k_first, k_first + Nc, ... in
+// order, the first copy taken as is, later ones added.  Bound by memory: one
+// CTA per job with a division chain per position took 29 us for 26 blocks of
+// BG1 Z=384 and 286 us for the 8,192-codeword mix (0.85 GB).
+
 __global__ void __launch_bounds__(256) batch_derate_kernel(const __grid_constant__ DerateArgs a) {
-    for (int i = blockIdx.x; i < a.n_jobs; i += gridDim.x) {
-        const JobDev jb = a.jobs[i];
-        const CodeTable& tab = a.tables[jb.code];
-        const int z = tab.z, n = tab.n_bp, K = tab.kb * z, ncb = n - 2 * z;
+    const float inf = __int_as_float(0x7f800000);
+    for (long w = blockIdx.x; w < static_cast<long>(a.n_jobs) * a.parts; w += gridDim.x) {
+        const int job = static_cast<int>(w / a.parts), from = static_cast<int>(w - static_cast<long>(job) * a.parts) * a.part;
+        const JobDev jb = a.jobs[job];
+        const int z = a.tables[jb.code].z, n = a.tables[jb.code].n_bp, K = a.tables[jb.code].kb * z, ncb = n - 2 * z;
         const int f0 = jb.k_prime - 2 * z, nf = K - jb.k_prime, nc = ncb - nf;
         const int c0 = jb.k0 < f0 ? jb.k0 : (jb.k0 < f0 + nf ? f0 : jb.k0 - nf);
         float* out = a.llr + jb.llr_offset;
         const float* in = a.llr_e + jb.e_offset;
-        for (int j = threadIdx.x; j < 2 * z; j += blockDim.x) out[j] = 0.0f;
-        for (int j = jb.k_prime + threadIdx.x; j < K; j += blockDim.x) out[j] = __int_as_float(0x7f800000);
-        for (int c = threadIdx.x; c < nc; c += blockDim.x) {
-            const int kf = (c - c0 + nc) % nc;
-            float v = 0.0f;
-            if (kf < jb.e) {
-                v = in[il_pos(jb.e, jb.qm, kf)];
-                for (int k = kf + nc; k < jb.e; k += nc) v = __fadd_rn(v, in[il_pos(jb.e, jb.qm, k)]);
-            }
-            out[2 * z + (c < f0 ? c : c + nf)] = v;
+        if (from == 0) {
+            for (int j = threadIdx.x; j < 2 * z; j += blockDim.x) out[j] = 0.0f;
+            for (int j = jb.k_prime + threadIdx.x; j < K; j += blockDim.x) out[j] = inf;
         }
-        __syncthreads();
+        // position of bit k: c = (c0 + k) mod Nc, past the filler run
+        auto put = [&](int k, float v) {
+            int c = c0 + k;
+            if (c >= nc) c -= nc;
+            out[2 * z + (c < f0 ? c : c + nf)] = v;
+        };
+        if (jb.e <= nc) {
+            const int rows = jb.qm == 1 ? jb.e : jb.e / jb.qm;
+            if (jb.qm == 1) {
+#pragma unroll 4
+                for (int k = from + threadIdx.x; k < min(rows, from + a.part); k += blockDim.x) put(k, __ldcs(in + k));
+            } else {
+                for (int i = from + threadIdx.x; i < min(rows, from + a.part); i += blockDim.x) {
+                    const float* row = in + static_cast<long>(i) * jb.qm;
+                    for (int j = 0, k = i; j < jb.qm; j++, k += rows) put(k, row[j]);
+                }
+            }
+#pragma unroll 4
+            for (int k = jb.e + from + threadIdx.x; k < min(nc, jb.e + from + a.part); k += blockDim.x) put(k, 0.0f);
+        } else {
+            for (int k = from + threadIdx.x; k < min(nc, from + a.part); k += blockDim.x) {
+                float v = in[il_pos(jb.e, jb.qm, k)];
+                for (int m = k + nc; m < jb.e; m += nc) v = __fadd_rn(v, in[il_pos(jb.e, jb.qm, m)]);
+                put(k, v);
+            }
+        }
     }
 }
 
@@ -237,10 +264,29 @@ struct Batch {
     // job list
     int n_jobs = 0, n_items = 0;
     std::vector<JobDev> h_jobs;
+    // the job list on the device: one allocation, one copy per set_jobs
+    unsigned char* d_lists = nullptr;
+    std::vector<unsigned char> h_lists;
     JobDev* d_jobs_rm = nullptr;
     nrldpc_job* d_jobs = nullptr;
     int32_t* d_order = nullptr;
     WorkItem* d_items = nullptr;
+    int derate_parts = 1, derate_part = 256;
+    // few jobs: one codeword on a cluster of CTAs (split.cu).  Plans are made
+    // when a job list first needs them and kept (102 codes x 8 cluster sizes,
+    // 10 KB each, at most); split: the current list's launch, ranks 0: none
+    struct Plan {
+        int state = 0;  // 1: made, -1: the code does not fit such clusters
+        int32_t at = 0;
+        SplitHead head;
+    };
+    std::vector<Plan> plans;  // [code][cluster size]
+    std::vector<unsigned char> h_plans;
+    unsigned char* d_plans_split = nullptr;
+    size_t plans_room = 0, plans_sent = 0;
+    SplitJob* d_split = nullptr;
+    SplitHead split{};
+    int split_clusters = 0;
     size_t slot_words = 0, smem = 0;
     int grid = 0, threads = kMaxThreads;
     uint32_t* d_state = nullptr;
@@ -252,6 +298,9 @@ struct Batch {
     cudaGraphNode_t knode = nullptr;
     BatchDecodeArgs kargs{};
 };
+
+constexpr size_t kListBytes =
+    sizeof(JobDev) + sizeof(nrldpc_job) + sizeof(int32_t) + sizeof(WorkItem) + sizeof(SplitJob);
 
 int map_cuda(cudaError_t e) { return e == cudaSuccess ? NRLDPC_OK : NRLDPC_ERR_CUDA; }
 
@@ -286,13 +335,87 @@ void free_batch(Batch* b) {
     drop_graph(b);
     cudaFree(b->d_tables);
     cudaFree(b->d_plans);
-    cudaFree(b->d_jobs_rm);
-    cudaFree(b->d_jobs);
-    cudaFree(b->d_order);
-    cudaFree(b->d_items);
+    cudaFree(b->d_lists);
+    cudaFree(b->d_plans_split);
     cudaFree(b->d_state);
     cudaFree(b->d_scratch);
     delete b;
+}
+
+// The clusters for this job list (b->split, b->split_clusters and the jobs'
+// plans), or none where the time estimate favours the persistent kernel.
+// Cluster sizes from the largest that holds at least half the jobs at once
+// down to the first that holds all; the jobs are in order of falling work.
+int choose_split(Batch* b, const std::vector<int32_t>& order, const std::vector<WorkItem>& items,
+                 std::vector<SplitJob>* jobs) {
+    static const int kRoom[kSplitSizes] = {7, 13, 23, 28, 36, 46, 76, 152};  // at one CTA per SM of 152
+    const int n = b->n_jobs;
+    if (n > 2L * kRoom[kSplitSizes - 1] * b->sm_count / 152) return NRLDPC_OK;
+    long fused_sum = 0, least = 0;
+    for (const WorkItem& it : items) {
+        const long c = fused_row_walk(b->h_tables[it.code], b->threads / 32);
+        fused_sum += c;
+        least = std::max(least, c);  // the longest item
+    }
+    least = std::max(least, fused_sum * 33 / 40 / b->sm_count);  // two CTAs per SM: 1.65 times one's time
+    int tasks = 0;
+    for (const int32_t j : order) {
+        const CodeTable& t = b->h_tables[b->h_jobs[j].code];
+        tasks = std::max(tasks, t.rows * ((t.z + 31) / 32));
+    }
+    b->plans.resize(kNumCodes * kSplitSizes);
+    int best = -1;
+    for (int s = 0; s < kSplitSizes; s++) {
+        const int ranks = kSplitRanks[s];
+        if (n > 2L * kRoom[s] * b->sm_count / 152 || (ranks > 1 && tasks < ranks * kSplitMinTasks)) continue;
+        SplitHead launch{};
+        launch.ranks = ranks;
+        bool fits = true;
+        for (size_t i = 0; fits && i < order.size(); i++) {
+            const int code = b->h_jobs[order[i]].code;
+            Batch::Plan& p = b->plans[code * kSplitSizes + s];
+            if (p.state == 0) {
+                p.at = static_cast<int32_t>(b->h_plans.size());
+                p.state = make_split_plan(b->h_tables[code], ranks, b->smem_optin, &p.head, &b->h_plans) ? 1 : -1;
+            }
+            fits = p.state > 0;
+            launch.warps = std::max(launch.warps, p.head.warps);
+            launch.smem = std::max(launch.smem, p.head.smem);
+        }
+        if (!fits) continue;
+        const int room = split_max_clusters(launch);
+        if (room < 1) continue;
+        long cost = 0;
+        for (int i = 0; i < n; i += room) cost += split_cost(b->plans[b->h_jobs[order[i]].code * kSplitSizes + s].head);
+        if (cost < least) {
+            least = cost;
+            best = s;
+            b->split = launch;
+            b->split_clusters = std::min(n, room);
+        }
+        if (room >= n) break;
+    }
+    if (best < 0) return NRLDPC_OK;
+    if (b->h_plans.size() > b->plans_room) {  // grows with the codes seen
+        cudaFree(b->d_plans_split);
+        b->d_plans_split = nullptr;
+        b->plans_room = b->plans_sent = 0;
+        const size_t room = 2 * b->h_plans.size();
+        if (cudaMalloc(&b->d_plans_split, room) != cudaSuccess) return NRLDPC_ERR_NO_MEMORY;
+        b->plans_room = room;
+    }
+    if (b->plans_sent < b->h_plans.size()) {
+        if (cudaMemcpy(b->d_plans_split + b->plans_sent, b->h_plans.data() + b->plans_sent,
+                       b->h_plans.size() - b->plans_sent, cudaMemcpyHostToDevice) != cudaSuccess)
+            return NRLDPC_ERR_CUDA;
+        b->plans_sent = b->h_plans.size();
+    }
+    jobs->resize(n);
+    for (int i = 0; i < n; i++) {
+        const JobDev& d = b->h_jobs[order[i]];
+        (*jobs)[i] = {d.llr_offset, d.out_offset, b->plans[d.code * kSplitSizes + best].at, order[i]};
+    }
+    return NRLDPC_OK;
 }
 
 }  // namespace
@@ -348,10 +471,7 @@ int nrldpc_batch_create(int device, int max_jobs, float alpha, nrldpc_batch** ou
         }
     if (cudaMalloc(&b->d_tables, sizeof(CodeTable) * kNumCodes) != cudaSuccess ||
         cudaMalloc(&b->d_plans, sizeof(PlanDev) * kNumCodes) != cudaSuccess ||
-        cudaMalloc(&b->d_jobs_rm, sizeof(JobDev) * max_jobs) != cudaSuccess ||
-        cudaMalloc(&b->d_jobs, sizeof(nrldpc_job) * max_jobs) != cudaSuccess ||
-        cudaMalloc(&b->d_order, sizeof(int32_t) * max_jobs) != cudaSuccess ||
-        cudaMalloc(&b->d_items, sizeof(WorkItem) * max_jobs) != cudaSuccess ||
+        cudaMalloc(&b->d_lists, kListBytes * max_jobs + 5 * 256) != cudaSuccess ||
         cudaMalloc(&b->d_scratch, 256) != cudaSuccess) {
         free_batch(b);
         return NRLDPC_ERR_NO_MEMORY;
@@ -360,7 +480,8 @@ int nrldpc_batch_create(int device, int max_jobs, float alpha, nrldpc_batch** ou
         cudaMemcpy(b->d_plans, plans.data(), sizeof(PlanDev) * kNumCodes, cudaMemcpyHostToDevice) ||
         cudaMemset(b->d_scratch, 0, 256) ||
         cudaFuncSetAttribute(batch_decode_kernel_ptr(), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(b->smem_optin))) {
+                             static_cast<int>(b->smem_optin)) ||
+        split_kernel_attributes(b->smem_optin)) {
         free_batch(b);
         return NRLDPC_ERR_CUDA;
     }
@@ -418,6 +539,7 @@ int nrldpc_batch_set_jobs(nrldpc_batch* batch, const nrldpc_job* jobs, int n_job
     cudaSetDevice(b->device);
     b->h_jobs.assign(n_jobs, JobDev{});
     std::vector<int32_t> order(n_jobs);
+    int longest = 0;
     for (int i = 0; i < n_jobs; i++) {
         const nrldpc_job& j = jobs[i];
         const int id = code_id(j.bg, j.z);
@@ -442,7 +564,12 @@ int nrldpc_batch_set_jobs(nrldpc_batch* batch, const nrldpc_job* jobs, int n_job
         d.e_offset = j.e_offset;
         d.out_offset = j.out_offset;
         order[i] = i;
+        const int nc = ncb - (K - kp);  // positions a bit can land on
+        longest = std::max(longest, e <= nc ? std::max(e / qm, nc - e) : nc);
     }
+    // eight CTAs per SM, in parts of at least 256 positions
+    b->derate_part = std::max(256, (longest * static_cast<int>(std::min(n_jobs, 8 * b->sm_count)) / (8 * b->sm_count) + 255) / 256 * 256);
+    b->derate_parts = std::max(1, (longest + b->derate_part - 1) / b->derate_part);
     // group by code; largest codes first so the tail of the queue is short work
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
         const CodeTable& a = b->h_tables[b->h_jobs[x].code];
@@ -485,15 +612,25 @@ int nrldpc_batch_set_jobs(nrldpc_batch* batch, const nrldpc_job* jobs, int n_job
         if (cudaMalloc(&b->d_state, need * sizeof(uint32_t)) != cudaSuccess) return NRLDPC_ERR_NO_MEMORY;
         b->state_words = need;
     }
-    if (n_jobs) {
-        if (cudaMemcpy(b->d_jobs_rm, b->h_jobs.data(), sizeof(JobDev) * n_jobs, cudaMemcpyHostToDevice) ||
-            cudaMemcpy(b->d_jobs, jobs, sizeof(nrldpc_job) * n_jobs, cudaMemcpyHostToDevice) ||
-            cudaMemcpy(b->d_order, order.data(), sizeof(int32_t) * n_jobs, cudaMemcpyHostToDevice) ||
-            cudaMemcpy(b->d_items, items.data(), sizeof(WorkItem) * items.size(), cudaMemcpyHostToDevice))
-            return NRLDPC_ERR_CUDA;
-    }
-    drop_graph(b);  // launch geometry changed
-    return NRLDPC_OK;
+    b->split.ranks = 0;
+    if (n_jobs == 0) return NRLDPC_OK;
+    std::vector<SplitJob> split;
+    const int rc = choose_split(b, order, items, &split);
+    if (rc) return rc;
+    // one copy for all lists
+    b->h_lists.clear();
+    auto put = [&](const void* p, size_t bytes) {
+        const size_t at = b->h_lists.size();
+        b->h_lists.resize((at + bytes + 255) / 256 * 256);
+        std::memcpy(b->h_lists.data() + at, p, bytes);
+        return b->d_lists + at;
+    };
+    b->d_jobs_rm = reinterpret_cast<JobDev*>(put(b->h_jobs.data(), sizeof(JobDev) * n_jobs));
+    b->d_jobs = reinterpret_cast<nrldpc_job*>(put(jobs, sizeof(nrldpc_job) * n_jobs));
+    b->d_order = reinterpret_cast<int32_t*>(put(order.data(), sizeof(int32_t) * n_jobs));
+    b->d_items = reinterpret_cast<WorkItem*>(put(items.data(), sizeof(WorkItem) * items.size()));
+    if (!split.empty()) b->d_split = reinterpret_cast<SplitJob*>(put(split.data(), sizeof(SplitJob) * split.size()));
+    return map_cuda(cudaMemcpy(b->d_lists, b->h_lists.data(), b->h_lists.size(), cudaMemcpyHostToDevice));
 }
 
 int nrldpc_batch_gen(nrldpc_batch* batch, uint64_t seed, uint64_t cw_base, float* d_llr_e, uint8_t* d_cw,
@@ -511,8 +648,8 @@ int nrldpc_batch_derate(nrldpc_batch* batch, const float* d_llr_e, float* d_llr,
     Batch* b = reinterpret_cast<Batch*>(batch);
     if (!b || !d_llr_e || !d_llr) return NRLDPC_ERR_INVALID_ARG;
     if (b->n_jobs == 0) return NRLDPC_OK;
-    DerateArgs a{b->d_tables, b->d_jobs_rm, d_llr_e, d_llr, b->n_jobs};
-    const int grid = std::min(b->n_jobs, 8 * b->sm_count);
+    DerateArgs a{b->d_tables, b->d_jobs_rm, d_llr_e, d_llr, b->n_jobs, b->derate_parts, b->derate_part};
+    const int grid = static_cast<int>(std::min<long>(static_cast<long>(b->n_jobs) * b->derate_parts, 8L * b->sm_count));
     batch_derate_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(a);
     return map_cuda(cudaGetLastError());
 }
@@ -535,6 +672,19 @@ int nrldpc_batch_decode(nrldpc_batch* batch, const float* d_llr, uint8_t* d_pack
     if (b->n_jobs == 0) return NRLDPC_OK;
     if (!d_llr || !d_packed) return NRLDPC_ERR_INVALID_ARG;
     if (reinterpret_cast<uintptr_t>(d_llr) % 16 != 0) return NRLDPC_ERR_ALIGNMENT;
+    if (b->split.ranks) {
+        SplitArgs a{};
+        a.plan = b->d_plans_split;
+        a.jobs = b->d_split;
+        a.llr = d_llr;
+        a.packed = d_packed;
+        a.iters = d_iters;
+        a.n_cw = b->n_jobs;
+        a.n_iter = n_iter;
+        a.early_stop = early_stop;
+        a.alpha = b->alpha;
+        return map_cuda(launch_split(b->split, a, nullptr, b->split_clusters, reinterpret_cast<cudaStream_t>(stream)));
+    }
     BatchDecodeArgs& k = b->kargs;
     k.tables = b->d_tables;
     k.items = b->d_items;
