@@ -92,9 +92,8 @@ bool fill_table(const int* base, int rows, int cols, int z, int kb, CodeTable* t
             if (v < 0 || e >= kMaxEdges) return false;
             const int sh = v % z;
             t->edge[e] = static_cast<uint32_t>(c * z + sh) | (static_cast<uint32_t>(z - sh) << 16);
-            t->ebase4[e] = static_cast<uint32_t>(c * z + sh) * 4u;
             t->ethr[e] = static_cast<uint16_t>(z - sh);
-            t->eaddr[e] = make_uint2(t->ebase4[e], t->ethr[e]);
+            t->eaddr[e] = make_uint2(static_cast<uint32_t>(c * z) * 4u, static_cast<uint32_t>(sh) * 4u);
             t->edge_col[e] = static_cast<uint8_t>(c);
             t->edge_shift[e] = static_cast<uint16_t>(sh);
             e++;
@@ -269,16 +268,16 @@ int init_impl(const int* base, int rows, int cols, int kb, const nrldpc_config* 
     h->cpb = cpb;
     h->threads = (cpb * z + 31) / 32 * 32;
     h->smem = decode_smem_bytes(h->tab, cpb);
-    // opt in to the device maximum once, so handles of any size can coexist
-    if (map_cuda(decode_kernel_attributes(smem_limit))) {
-        delete h;
-        return NRLDPC_ERR_CUDA;
-    }
     // two CTAs per SM when shared memory allows (the kernel then caps its
     // registers for two); otherwise one CTA with the full register budget
     h->minb = (2 * (h->smem + 1024) <= prop.sharedMemPerMultiprocessor) ? 2 : 1;
-    h->ctas_per_sm = std::max(1, std::min(decode_max_ctas_per_sm(false, h->minb, h->threads, h->smem),
-                                          decode_max_ctas_per_sm(true, h->minb, h->threads, h->smem)));
+    // opt in to the device maximum, so handles of any size can coexist
+    if (map_cuda(decode_kernel_attributes(has_short_rows(h->tab), h->minb, smem_limit))) {
+        delete h;
+        return NRLDPC_ERR_CUDA;
+    }
+    h->ctas_per_sm = std::max(1, std::min(decode_max_ctas_per_sm(h->tab, false, h->minb, h->threads, h->smem),
+                                          decode_max_ctas_per_sm(h->tab, true, h->minb, h->threads, h->smem)));
     h->max_grid = h->ctas_per_sm * h->sm_count;
     const size_t state_elems =
         static_cast<size_t>(h->max_grid) * cpb * h->tab.rows * static_cast<size_t>(z);

@@ -36,6 +36,7 @@
 namespace nrldpc {
 namespace {
 
+constexpr int kKeepQMax = 10;  // longest row whose Q stay in registers (unweighted flooding)
 constexpr int kMaxCpb = 48;
 constexpr int kHeaderBytes = 1024;  // mbarrier, group id, per-slot flags
 // Weights of the current iteration in shared memory, one padded row of
@@ -57,6 +58,13 @@ constexpr long kWaitLimit = 1L << 20;
 // check is bit-sliced.
 constexpr int kFarOffset = 60;
 constexpr int kFarRow = 12;
+
+// min of three, NaN operands ignored
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
 
 __device__ __forceinline__ float max_nan(float a, float b) {
     float r;
@@ -156,41 +164,45 @@ __device__ __forceinline__ uint32_t lds_u8(uint32_t a) {
 // form measured fastest for its kernels).
 // LAYERED (no reference counterpart): one posterior buffer updated in place,
 // A = Q + R_new (dnew = 0), instead of Lnew += R_new - R_old.
-template <int D, bool WEIGHTED, bool LAYERED, bool PACKED>
+// kKeepQ (layered, and unweighted flooding of codes with longer rows for their
+// rows of up to kKeepQMax edges; the kernels for shorter codes are 4% slower
+// with it): Q stays in registers, so the edge that gets min2 is found in the
+// second half as any edge with |Q| == min1 -- the first argmin when the
+// minimum is unique, and when it is not, min2 == min1 and every such edge
+// gets the same message -- and the two minima are taken two edges at a time
+// (kPair: not in the unweighted layered kernels, 1-2% slower with it).
+// Measured with the wrapped address below, BG1 Z=384 flooding 6.16 -> 6.00 ms
+// per 4,096 codewords, layered with weights 4.05 -> 3.97.
+template <int D, bool WEIGHTED, bool LAYERED, int MAXD>
 __device__ __forceinline__ void row_update(const CodeTable& tab, int e0, bool sfx, uint32_t s,
                                            uint32_t s4old, uint32_t dnew, uint32_t z4,
                                            const float4* wprev, const float4* wcur, uint4 st, uint4* st_out,
                                            bool store, bool write_hd, uint32_t hd, float alpha) {
     constexpr int LAST = D - 1;
     constexpr bool kPlain = !WEIGHTED && !LAYERED;
+    constexpr bool kKeepQ = LAYERED || (kPlain && MAXD > kKeepQMax && D <= kKeepQMax);
+    constexpr bool kPair = kKeepQ && (kPlain || WEIGHTED);
     uint32_t addr[D];
     float lv[D];
     const float sraw = __uint_as_float(st.w);  // the suffix posterior as accumulated
+    const uint32_t lbase = s4old - 4u * s;
 #pragma unroll
     for (int i = 0; i < D; i++) {
         if (i == LAST && sfx) {
             addr[i] = 0;
             lv[i] = kPlain ? __fadd_rn(sraw, 0.0f) : __uint_as_float(st.w);  // kPlain: -0 read as +0, like Lold
         } else {
-            uint32_t a;
-            // one 64-bit table read per edge: faster for the layered kernels and
-            // for a table in shared memory (mixed batch); the single-code
-            // flooding kernels read the two words from their parameter bank
-            if (LAYERED || PACKED) {
-                const uint2 ea = tab.eaddr[e0 + i];
-                a = s4old + ea.x;
-                if (s >= ea.y) a -= z4;  // column (s + V) mod Z of the edge's block
-            } else {
-                a = s4old + tab.ebase4[e0 + i];
-                if (s >= tab.ethr[e0 + i]) a -= z4;
-            }
-            addr[i] = a;
-            lv[i] = lds(a);
+            // 4 ((s + V) mod Z) without a compare: where s + V < Z the
+            // difference wraps around to a large unsigned number
+            const uint2 ea = tab.eaddr[e0 + i];
+            const uint32_t t = 4u * s + ea.y;
+            addr[i] = __viaddmin_u32(t, 0u - z4, t) + ea.x + lbase;
+            lv[i] = lds(addr[i]);
         }
     }
     // old messages R_old from the previous iteration's state; kept per edge:
-    // R_old (flooding, for dt) or Q (layered, for A = Q + R_new)
-    float keep[D];
+    // R_old (flooding, for dt) and Q where it is needed again
+    float keep[D], qk[D];
     const float om1 = __uint_as_float(st.x), om2 = __uint_as_float(st.y);
     const uint32_t oinfo = st.z;
     const int oidx = static_cast<int>(oinfo & 31u);
@@ -199,7 +211,7 @@ __device__ __forceinline__ void row_update(const CodeTable& tab, int e0, bool sf
         oa1 = __fmul_rn(alpha, om1);
         oa2 = __fmul_rn(alpha, om2);
     }
-    float m1 = 1000.0f, m2 = 1000.0f;
+    float m1 = 1000.0f, m2 = 1000.0f, first = 0.0f;
     int idx = 0;
     uint32_t qmask = 0;
 #pragma unroll
@@ -211,7 +223,8 @@ __device__ __forceinline__ void row_update(const CodeTable& tab, int e0, bool sf
             mag = i == oidx ? oa2 : oa1;
         const float ro = __uint_as_float(__float_as_uint(mag) ^ ((oinfo << (24 - D + i)) & 0x80000000u));
         const float q = __fsub_rn(lv[i], ro);
-        keep[i] = LAYERED ? q : ro;
+        keep[i] = ro;
+        if (kKeepQ) qk[i] = q;
         const float qa = fabsf(q);
         // the sign bit of q is (q < 0) when q is never -0 (kPlain: L is
         // never -0, so neither is L - R_old); the others take it from q + 0,
@@ -220,12 +233,20 @@ __device__ __forceinline__ void row_update(const CodeTable& tab, int e0, bool sf
         qmask = __funnelshift_l(__float_as_uint(qs), qmask, 1);  // edge i at bit D-1-i
         if (i == 0) {  // from m1 = m2 = 1000: min2 stays 1000 whatever |Q_0| is
             m1 = fminf(m1, qa);
-            continue;
+        } else if (kPair && (i & 1) && i + 1 < D) {
+            first = qa;  // of a pair
+        } else if (kPair && !(i & 1)) {
+            // the larger of the pair and the larger of its smaller and min1
+            // are the candidates for min2; a NaN |Q| leaves both untouched
+            const float lo = fminf(first, qa), hi = max_nan(first, qa);
+            m2 = min3(m2, hi, max_nan(m1, lo));
+            m1 = fminf(m1, lo);
+        } else {
+            if (!kKeepQ && qa < m1) idx = i;
+            const float mx = max_nan(m1, qa);  // NaN |Q| leaves min1/min2 untouched
+            m1 = fminf(m1, qa);
+            m2 = fminf(m2, mx);
         }
-        if (!LAYERED && qa < m1) idx = i;  // layered: found below from the kept Q
-        const float mx = max_nan(m1, qa);  // NaN |Q| leaves min1/min2 untouched
-        m1 = fminf(m1, qa);
-        m2 = fminf(m2, mx);
     }
     const uint32_t par = static_cast<uint32_t>(__popc(qmask) & 1);
     const uint32_t rsign = qmask ^ (0u - par);  // sign of R_i = product of the other signs
@@ -236,12 +257,9 @@ __device__ __forceinline__ void row_update(const CodeTable& tab, int e0, bool sf
     }
     float sfx_new = 0.0f;
     if (LAYERED) {
-        // The edge that gets min2 is any edge with |Q| == min1: the first
-        // argmin when the minimum is unique, and when it is not, min2 ==
-        // min1 and every such edge gets the same message.
 #pragma unroll
         for (int i = 0; i < D; i++) {
-            const bool at_min = fabsf(keep[i]) == m1;
+            const bool at_min = fabsf(qk[i]) == m1;
             if (at_min) idx = i;
             float mag;
             if (WEIGHTED)
@@ -249,7 +267,7 @@ __device__ __forceinline__ void row_update(const CodeTable& tab, int e0, bool sf
             else
                 mag = at_min ? a2 : a1;
             const float rn = __uint_as_float(__float_as_uint(mag) ^ ((rsign << (32 - D + i)) & 0x80000000u));
-            const float v = __fadd_rn(keep[i], rn);
+            const float v = __fadd_rn(qk[i], rn);
             if (i == LAST && sfx)
                 sfx_new = v;
             else
@@ -269,11 +287,13 @@ __device__ __forceinline__ void row_update(const CodeTable& tab, int e0, bool sf
             if (i + kPipe < D)
                 nv[i + kPipe] =
                     (i + kPipe == LAST && sfx) ? (kPlain ? sraw : lv[i + kPipe]) : lds(addr[i + kPipe] + dnew);
+            const bool at_min = kKeepQ ? fabsf(qk[i]) == m1 : i == idx;
+            if (kKeepQ && at_min) idx = i;
             float mag;
             if (WEIGHTED)
-                mag = __fmul_rn(wsel(wcur, i), i == idx ? m2 : m1);
+                mag = __fmul_rn(wsel(wcur, i), at_min ? m2 : m1);
             else
-                mag = i == idx ? a2 : a1;
+                mag = at_min ? a2 : a1;
             const float rn = __uint_as_float(__float_as_uint(mag) ^ ((rsign << (32 - D + i)) & 0x80000000u));
             const float dt = __fsub_rn(rn, keep[i]);
             const float v = __fadd_rn(nv[i], dt);
@@ -290,16 +310,20 @@ __device__ __forceinline__ void row_update(const CodeTable& tab, int e0, bool sf
     }
 }
 
-template <bool WEIGHTED, bool LAYERED, bool PACKED>
+// Degree switch up to MAXD: 10 for BG2 and codes like it, whose kernels then
+// hold no registers for BG1's rows of 19 (1,001 codewords of BG2 Z=208 with
+// early stop 667 -> 625 us with the wrapped address).
+template <bool WEIGHTED, bool LAYERED, int MAXD>
 __device__ __forceinline__ void row_dispatch(int deg, const CodeTable& tab, int e0, bool sfx, uint32_t s,
                                              uint32_t s4old, uint32_t dnew, uint32_t z4,
                                              const float4* wprev, const float4* wcur, uint4 st, uint4* st_out,
                                              bool store, bool write_hd, uint32_t hd, float alpha) {
     switch (deg) {
-#define NRLDPC_ROW_CASE(D)                                                                         \
-    case D:                                                                                        \
-        row_update<D, WEIGHTED, LAYERED, PACKED>(tab, e0, sfx, s, s4old, dnew, z4, wprev, wcur, st, st_out, store, \
-                                         write_hd, hd, alpha);                                    \
+#define NRLDPC_ROW_CASE(D)                                                                                        \
+    case D:                                                                                                       \
+        if constexpr (D <= MAXD)                                                                                  \
+            row_update<D, WEIGHTED, LAYERED, MAXD>(tab, e0, sfx, s, s4old, dnew, z4, wprev, wcur, st, st_out,     \
+                                                   store, write_hd, hd, alpha);                                   \
         break;
         NRLDPC_ROW_CASE(1) NRLDPC_ROW_CASE(2) NRLDPC_ROW_CASE(3) NRLDPC_ROW_CASE(4)
         NRLDPC_ROW_CASE(5) NRLDPC_ROW_CASE(6) NRLDPC_ROW_CASE(7) NRLDPC_ROW_CASE(8)
@@ -398,7 +422,7 @@ __device__ __forceinline__ void write_outputs(const CodeTable& tab, const float*
 // next row's two sub-rows requested while this row's run.
 //   store: write this iteration's state; write_hd: write the suffix hard
 //   decisions.
-template <bool WEIGHTED, bool LAYERED, int SPT, bool PACKED>
+template <bool WEIGHTED, bool LAYERED, int SPT, int MAXD>
 __device__ __forceinline__ void iterate_rows(const CodeTable& tab, uint32_t s, uint32_t tpc, uint32_t s4old,
                                              uint32_t dnew, const float4* wpad, uint4* st_base,
                                              const float* gllr,
@@ -420,7 +444,7 @@ __device__ __forceinline__ void iterate_rows(const CodeTable& tab, uint32_t s, u
     auto run = [&](int r, uint32_t j, uint4 st) {
         const uint32_t sj = s + j * tpc;
         const bool sfx = tab.row_sfx[r] != 0;
-        row_dispatch<WEIGHTED, LAYERED, PACKED>(
+        row_dispatch<WEIGHTED, LAYERED, MAXD>(
             tab.row_deg[r], tab, tab.row_ptr[r], sfx, sj, s4old + 4u * j * tpc, dnew, z4, wpad + r * (kWPad / 4),
             wpad + (kMaxRows + r) * (kWPad / 4), st, (kPlain || store) ? st_base + r * z + sj : nullptr, store,
             kPlain ? write_hd : (write_hd && sfx),
@@ -455,26 +479,18 @@ __device__ __forceinline__ void iterate_rows(const CodeTable& tab, uint32_t s, u
 // of their hard-decision bytes.  Threads stop at the first failure seen by
 // any thread of the slot, so an iteration far from convergence costs a few
 // rows; *far gets the row of the failure.
-template <bool PACKED>
 __device__ __forceinline__ void check_rows(const CodeTable& tab, uint32_t s, uint32_t s4a, uint32_t hd_base,
                                            volatile int* fail, int* far) {
     const int z = tab.z;
-    const uint32_t z4 = 4u * static_cast<uint32_t>(z);
+    const uint32_t z4 = 4u * static_cast<uint32_t>(z), lbase = s4a - 4u * s;
     for (int r = 0; r < tab.rows; r++) {
         if (*fail) return;
         const int e0 = tab.row_ptr[r], e1 = tab.row_ptr[r + 1] - (tab.row_sfx[r] ? 1 : 0);
         uint32_t par = tab.row_sfx[r] ? (lds_u8(hd_base + static_cast<uint32_t>(r * z)) >> 1) & 1u : 0u;
         for (int e = e0; e < e1; e++) {
-            uint32_t a;
-            if (PACKED) {
-                const uint2 ea = tab.eaddr[e];
-                a = s4a + ea.x;
-                if (s >= ea.y) a -= z4;
-            } else {
-                a = s4a + tab.ebase4[e];
-                if (s >= tab.ethr[e]) a -= z4;
-            }
-            par ^= lds(a) > 0.0f ? 0u : 1u;
+            const uint2 ea = tab.eaddr[e];
+            const uint32_t t = 4u * s + ea.y;
+            par ^= lds(__viaddmin_u32(t, 0u - z4, t) + ea.x + lbase) > 0.0f ? 0u : 1u;
         }
         if (par) {
             *fail = 1;
@@ -592,9 +608,7 @@ struct SlotOut {
 // Lold in place.  Early stop: after iteration t < n_iter - 1, a codeword
 // whose hard decisions satisfy every check stops with iters = t + 1 (the
 // oracle's rule, ldpc_oracle.c decode_one_f32).
-// PACKED: the table is in shared memory (the mixed batch): each edge's
-// address words come as one 64-bit read.
-template <bool WEIGHTED, bool LAYERED, int SPT = 1, bool PACKED = false>
+template <bool WEIGHTED, bool LAYERED, int MAXD, int SPT = 1>
 __device__ __forceinline__ void run_group(const CodeTable& tab, int cpb, int slot, uint32_t s, uint32_t tpc,
                                           bool slot_done, float* buf0, uint8_t* hd0,
                                           int* s_fail, uint4* st_base, const float* gllr, SlotOut out,
@@ -643,7 +657,7 @@ __device__ __forceinline__ void run_group(const CodeTable& tab, int cpb, int slo
         const bool far_check = __syncthreads_or(!slot_done && s_far[slot] >= kFarRow);
         const bool act = !slot_done;
         const bool store = !last || out.app != nullptr;
-        iterate_rows<WEIGHTED, LAYERED, SPT, PACKED>(tab, s, tpc, s4old, dnew, wpad, st_base, gllr, hd_base, act,
+        iterate_rows<WEIGHTED, LAYERED, SPT, MAXD>(tab, s, tpc, s4old, dnew, wpad, st_base, gllr, hd_base, act,
                                                      first, store, early_stop || last, alpha);
         if (early_stop && !last) {  // the rows ended with a barrier
             // bit-sliced scratch: flooding in Lold (read again only after the
@@ -656,7 +670,7 @@ __device__ __forceinline__ void run_group(const CodeTable& tab, int cpb, int slo
                            s_far);
             else if (act)
                 for (int j = 0; j < SPT; j++)
-                    check_rows<PACKED>(tab, s + j * tpc, s4old + 4u * j * tpc + dnew, hd_base + j * tpc,
+                    check_rows(tab, s + j * tpc, s4old + 4u * j * tpc + dnew, hd_base + j * tpc,
                                        &s_fail[slot], &s_far[slot]);
             __syncthreads();
             const bool conv = act && s_fail[slot] == 0;
@@ -696,7 +710,7 @@ struct WeightParam<true> {
 
 // FROM_HOST: a.llr is pinned host memory (a separate instantiation, so the
 // device-resident kernels keep their register allocation).
-template <bool WEIGHTED, int MINB, bool LAYERED, bool FROM_HOST>
+template <bool WEIGHTED, int MINB, bool LAYERED, bool FROM_HOST, int MAXD>
 __global__ void __launch_bounds__(kMaxThreads, MINB)
     decode_kernel(const __grid_constant__ CodeTable tab, const __grid_constant__ DecodeArgs a,
                   const __grid_constant__ typename WeightParam<WEIGHTED>::type wt) {
@@ -775,7 +789,7 @@ __global__ void __launch_bounds__(kMaxThreads, MINB)
         const size_t cw = static_cast<size_t>(cw0 + (slot_done ? 0 : slot));
         SlotOut out{a.packed + cw * tab.packed_bytes, a.app ? a.app + cw * n : nullptr,
                     a.iters ? a.iters + cw : nullptr};
-        run_group<WEIGHTED, LAYERED>(tab, cpb, slot, s, static_cast<uint32_t>(z), slot_done, buf0, hd0, s_fail,
+        run_group<WEIGHTED, LAYERED, MAXD>(tab, cpb, slot, s, static_cast<uint32_t>(z), slot_done, buf0, hd0, s_fail,
                                      st_base, a.llr + cw * n, out, a.n_iter, a.early_stop, a.alpha, wtab, wpad,
                                      a.n_w_iters);
     }
@@ -843,11 +857,11 @@ __global__ void __launch_bounds__(kMaxThreads, 2)
         uint4* st_base = reinterpret_cast<uint4*>(a.state + static_cast<size_t>(blockIdx.x) * a.slot_words) +
                          static_cast<size_t>(valid_thread ? slot : 0) * tab.rows * z;
         if (item.spt == 2)
-            run_group<false, false, 2, true>(tab, cpb, slot, s, static_cast<uint32_t>(tpc), !valid_thread, buf0, hd0,
+            run_group<false, false, kMaxDeg, 2>(tab, cpb, slot, s, static_cast<uint32_t>(tpc), !valid_thread, buf0, hd0,
                                        s_fail, st_base, a.llr + job.llr_offset, out, a.n_iter, a.early_stop, a.alpha,
                                        nullptr, nullptr, 1);
         else
-            run_group<false, false, 1, true>(tab, cpb, slot, s, static_cast<uint32_t>(tpc), !valid_thread, buf0, hd0,
+            run_group<false, false, kMaxDeg>(tab, cpb, slot, s, static_cast<uint32_t>(tpc), !valid_thread, buf0, hd0,
                                        s_fail, st_base, a.llr + job.llr_offset, out, a.n_iter, a.early_stop, a.alpha,
                                        nullptr, nullptr, 1);
     }
@@ -859,23 +873,32 @@ size_t decode_smem_bytes(const CodeTable& tab, int cpb) {
     return kHeaderBytes + kWeightBytes + group_smem_bytes(tab, cpb);
 }
 
-template <bool W, int MINB, bool LAY, bool HOST = false>
-const void* kernel_ptr() {
-    return reinterpret_cast<const void*>(&decode_kernel<W, MINB, LAY, HOST>);
+// The kernel for a code of row degrees up to 10 or up to 19; from_host: the
+// unweighted kernels that read host-resident LLRs.
+template <int MAXD, int MINB>
+const void* kernel_of(bool weighted, bool layered, bool from_host) {
+    if (from_host && !weighted)
+        return layered ? reinterpret_cast<const void*>(&decode_kernel<false, MINB, true, true, MAXD>)
+                       : reinterpret_cast<const void*>(&decode_kernel<false, MINB, false, true, MAXD>);
+    if (layered)
+        return weighted ? reinterpret_cast<const void*>(&decode_kernel<true, MINB, true, false, MAXD>)
+                        : reinterpret_cast<const void*>(&decode_kernel<false, MINB, true, false, MAXD>);
+    return weighted ? reinterpret_cast<const void*>(&decode_kernel<true, MINB, false, false, MAXD>)
+                    : reinterpret_cast<const void*>(&decode_kernel<false, MINB, false, false, MAXD>);
 }
 
-// from_host: the unweighted kernels that read host-resident LLRs.
-const void* select_kernel(bool weighted, int minb, bool layered, bool from_host = false) {
-    if (from_host && !weighted) {
-        if (layered) return minb >= 2 ? kernel_ptr<false, 2, true, true>() : kernel_ptr<false, 1, true, true>();
-        return minb >= 2 ? kernel_ptr<false, 2, false, true>() : kernel_ptr<false, 1, false, true>();
+const void* select_kernel(bool short_rows, bool weighted, int minb, bool layered, bool from_host) {
+    if (short_rows) {
+        return minb >= 2 ? kernel_of<10, 2>(weighted, layered, from_host) : kernel_of<10, 1>(weighted, layered, from_host);
     }
-    if (layered) {
-        if (weighted) return minb >= 2 ? kernel_ptr<true, 2, true>() : kernel_ptr<true, 1, true>();
-        return minb >= 2 ? kernel_ptr<false, 2, true>() : kernel_ptr<false, 1, true>();
-    }
-    if (weighted) return minb >= 2 ? kernel_ptr<true, 2, false>() : kernel_ptr<true, 1, false>();
-    return minb >= 2 ? kernel_ptr<false, 2, false>() : kernel_ptr<false, 1, false>();
+    return minb >= 2 ? kernel_of<kMaxDeg, 2>(weighted, layered, from_host)
+                     : kernel_of<kMaxDeg, 1>(weighted, layered, from_host);
+}
+
+bool has_short_rows(const CodeTable& tab) {
+    for (int r = 0; r < tab.rows; r++)
+        if (tab.row_deg[r] > 10) return false;
+    return true;
 }
 
 cudaError_t launch_batch_decode(const BatchDecodeArgs& args, int grid, int threads, size_t smem,
@@ -886,28 +909,23 @@ cudaError_t launch_batch_decode(const BatchDecodeArgs& args, int grid, int threa
 
 const void* batch_decode_kernel_ptr() { return reinterpret_cast<const void*>(&batch_decode_kernel); }
 
-cudaError_t decode_kernel_attributes(size_t smem) {
-    cudaError_t e = cudaFuncSetAttribute(batch_decode_kernel_ptr(),
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
-    if (e != cudaSuccess) return e;
-    for (int l = 0; l < 2; l++)
-        for (int w = 0; w < 3; w++)  // plain, weighted, plain from host
-            for (int m = 1; m <= 2; m++) {
-                cudaError_t e = cudaFuncSetAttribute(select_kernel(w == 1, m, l != 0, w == 2),
-                                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     static_cast<int>(smem));
-                if (e != cudaSuccess) return e;
-            }
+cudaError_t decode_kernel_attributes(bool short_rows, int minb, size_t smem) {
+    for (int k = 0; k < 6; k++) {  // plain, weighted, plain from host; both schedules
+        const int w = k % 3;
+        const cudaError_t e = cudaFuncSetAttribute(select_kernel(short_rows, w == 1, minb, k >= 3, w == 2),
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if (e != cudaSuccess) return e;
+    }
     return cudaSuccess;
 }
 
-int decode_max_ctas_per_sm(bool weighted, int minb, int threads, size_t smem) {
+// both schedules, device- and host-resident LLRs
+int decode_max_ctas_per_sm(const CodeTable& tab, bool weighted, int minb, int threads, size_t smem) {
     int n = 1 << 30;
-    for (int l = 0; l < 4; l++) {  // both schedules, device- and host-resident LLRs
+    for (int l = 0; l < 4; l++) {
         int k = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, select_kernel(weighted, minb, l & 1, l >= 2),
-                                                          threads, smem) != cudaSuccess)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                &k, select_kernel(has_short_rows(tab), weighted, minb, l & 1, l >= 2), threads, smem) != cudaSuccess)
             return 0;
         n = k < n ? k : n;
     }
@@ -919,7 +937,7 @@ cudaError_t launch_decode(const CodeTable& tab, const DecodeArgs& args, const We
     if (args.cpb < 1 || args.cpb > kMaxCpb) return cudaErrorInvalidValue;
     const bool weighted = weights != nullptr;
     if (weighted && args.llr_from_host) return cudaErrorInvalidValue;
-    const void* k = select_kernel(weighted, minb, layered, args.llr_from_host != 0);
+    const void* k = select_kernel(has_short_rows(tab), weighted, minb, layered, args.llr_from_host != 0);
     NoWeights none{};
     void* params[3] = {const_cast<CodeTable*>(&tab), const_cast<DecodeArgs*>(&args),
                        weighted ? const_cast<WeightTable*>(weights) : static_cast<void*>(&none)};

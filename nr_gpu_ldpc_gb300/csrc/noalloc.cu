@@ -70,7 +70,10 @@ int setup_device(int dev, DeviceSetup** out) {
         if (cudaGetSymbolAddress(&p, g_noalloc_state) != cudaSuccess ||
             cudaGetSymbolAddress(&q, g_noalloc_counters) != cudaSuccess ||
             cudaGetDeviceProperties(&prop, dev) != cudaSuccess ||
-            decode_kernel_attributes(prop.sharedMemPerBlockOptin) != cudaSuccess) {
+            decode_kernel_attributes(false, 1, prop.sharedMemPerBlockOptin) != cudaSuccess ||
+            decode_kernel_attributes(false, 2, prop.sharedMemPerBlockOptin) != cudaSuccess ||
+            decode_kernel_attributes(true, 1, prop.sharedMemPerBlockOptin) != cudaSuccess ||
+            decode_kernel_attributes(true, 2, prop.sharedMemPerBlockOptin) != cudaSuccess) {
             cudaGetLastError();  // leave no sticky launch-side error behind; retried next call
             return NRLDPC_ERR_CUDA;
         }
@@ -108,7 +111,7 @@ int noalloc_decode(int bg, int z, float alpha, const float* d_llr, uint8_t* d_pa
     if (smem > s->smem_optin) return NRLDPC_ERR_BAD_CONFIG;
     const int threads = (cpb * z + 31) / 32 * 32;
     const int minb = (2 * (smem + 1024) <= s->smem_per_sm) ? 2 : 1;
-    const int per_sm = decode_max_ctas_per_sm(false, minb, threads, smem);
+    const int per_sm = decode_max_ctas_per_sm(tab, false, minb, threads, smem);
     const size_t slot_bytes = static_cast<size_t>(cpb) * tab.rows * tab.z * kStateBytesPerRow;
     const size_t slots = kNoAllocScratchBytes / slot_bytes;
     if (slots < 1) return NRLDPC_ERR_SCRATCH_TOO_SMALL;

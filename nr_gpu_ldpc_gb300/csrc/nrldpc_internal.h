@@ -37,16 +37,11 @@ struct alignas(16) CodeTable {
     // per edge, row-major ascending (row, then column) = the reference's
     // h_compact1 order: low 16 bits blk_col*Z + V, high 16 bits Z - V
     uint32_t edge[kMaxEdges];
-    // the same edge as byte offset (blk_col*Z + V)*4 into a posterior buffer
-    // and wrap threshold Z - V: the sub-row s column is at s*4 + ebase4,
-    // minus 4Z when s >= ethr
-    uint32_t ebase4[kMaxEdges];
-    uint16_t ethr[kMaxEdges];
+    uint16_t ethr[kMaxEdges];      // Z - V: sub-rows from here on wrap
     uint8_t edge_col[kMaxEdges];
     uint16_t edge_shift[kMaxEdges];  // V mod Z
-    // {ebase4, ethr} of each edge in one 64-bit word: one read per edge for
-    // the layered decoder and for the mixed-batch kernel, which copies the
-    // whole table into shared memory
+    // byte offset of the edge's column in a posterior buffer and 4V, one 64-bit
+    // read per edge: sub-row s's position is at 4 ((s + V) mod Z) from it
     uint2 eaddr[kMaxEdges];
 };
 
@@ -188,8 +183,9 @@ cudaError_t launch_split(const SplitHead& head, const SplitArgs& args, const Wei
 cudaError_t launch_decode(const CodeTable& tab, const DecodeArgs& args, const WeightTable* weights, int grid,
                           int threads, size_t smem, bool layered, int minb, cudaStream_t stream);
 size_t decode_smem_bytes(const CodeTable& tab, int cpb);
-cudaError_t decode_kernel_attributes(size_t smem);
-int decode_max_ctas_per_sm(bool weighted, int minb, int threads, size_t smem);
+bool has_short_rows(const CodeTable& tab);  // every row of degree up to 10: kernels with fewer registers
+cudaError_t decode_kernel_attributes(bool short_rows, int minb, size_t smem);
+int decode_max_ctas_per_sm(const CodeTable& tab, bool weighted, int minb, int threads, size_t smem);
 
 // Learned weighted min-sum training kernels (wms.cu).
 size_t wms_smem_bytes(const CodeTable& tab, int cpb);

@@ -599,7 +599,7 @@ bool make_split_plan(const CodeTable& t, int ranks, size_t smem_limit, SplitHead
                                     t.row_deg[r] | (t.row_sfx[r] ? 256u : 0u));
                 for (int e = t.row_ptr[r]; e <= last; e++, m++) {
                     const int c = t.edge_col[e];
-                    edge[m] = make_uint4(t.eaddr[e].x, t.eaddr[e].y, 0u, 0u);
+                    edge[m] = make_uint4(t.eaddr[e].x + t.eaddr[e].y, t.ethr[e], 0u, 0u);
                     if (c < nc) edge[m].z = (static_cast<uint32_t>(col_rank[c]) << 24) | static_cast<uint32_t>(dt_of[e]);
                 }
             }
