@@ -678,10 +678,9 @@ struct WmsLayout {
 // Kernel attributes and CTAs per SM of the training kernels, once per handle.
 int wms_prepare(Handle* h) {
     if (h->wms_ready) return NRLDPC_OK;
-    const size_t smem = wms_smem_bytes(h->tab, h->cpb);
-    if (cudaSetDevice(h->device) != cudaSuccess || wms_kernel_attributes(smem) != cudaSuccess)
+    if (cudaSetDevice(h->device) != cudaSuccess || wms_kernel_attributes(h->tab, h->cpb) != cudaSuccess)
         return NRLDPC_ERR_CUDA;
-    h->wms_ctas = std::max(1, wms_ctas_per_sm(h->tab, h->threads, smem));
+    h->wms_ctas = std::max(1, wms_ctas_per_sm(h->tab, h->cpb, h->threads));
     h->wms_ready = true;
     return NRLDPC_OK;
 }
@@ -737,7 +736,7 @@ int nrldpc_wms_forward(nrldpc_handle* handle, const float* d_llr, const uint8_t*
                                lay ? reinterpret_cast<float*>(ws + l.states + l.gseed + l.gq) : nullptr,
                                d_loss, nullptr,
                                d_app, h->scratch, n_cw, n_iter, h->cpb, h->sm_count * h->wms_ctas, h->threads,
-                               wms_smem_bytes(h->tab, h->cpb), loss_scale, st));
+                               loss_scale, st));
 }
 
 int nrldpc_wms_backward(nrldpc_handle* handle, int n_cw, int n_iter, const float* d_weights,
@@ -757,7 +756,7 @@ int nrldpc_wms_backward(nrldpc_handle* handle, int n_cw, int n_iter, const float
                                lay ? reinterpret_cast<float*>(ws + l.states + l.gseed + l.gq) : nullptr,
                                nullptr, d_grad,
                                nullptr, h->scratch, n_cw, n_iter, h->cpb, h->sm_count * h->wms_ctas, h->threads,
-                               wms_smem_bytes(h->tab, h->cpb), 0.0f, st));
+                               0.0f, st));
 }
 
 int nrldpc_adam_step(int n, float* d_w, const double* d_grad, float* d_m, float* d_v, int step,

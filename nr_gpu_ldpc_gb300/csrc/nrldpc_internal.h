@@ -188,13 +188,13 @@ cudaError_t decode_kernel_attributes(bool short_rows, int minb, size_t smem);
 int decode_max_ctas_per_sm(const CodeTable& tab, bool weighted, int minb, int threads, size_t smem);
 
 // Learned weighted min-sum training kernels (wms.cu).
-size_t wms_smem_bytes(const CodeTable& tab, int cpb);
-cudaError_t wms_kernel_attributes(size_t smem);
-int wms_ctas_per_sm(const CodeTable& tab, int threads, size_t smem);
+size_t wms_smem_bytes(const CodeTable& tab, int cpb, bool layered);
+cudaError_t wms_kernel_attributes(const CodeTable& tab, int cpb);
+int wms_ctas_per_sm(const CodeTable& tab, int cpb, int threads);  // the fewest of the code's four kernels
 cudaError_t launch_wms(bool backward, bool layered, const CodeTable& tab, const float* llr, const uint8_t* cw,
                        const float* weights, uint4* states, float* gseed, uint4* gq, float* gh, double* loss,
                        double* grad, float* app, int* counters, int n_cw, int T, int cpb, int grid,
-                       int threads, size_t smem, float scale, cudaStream_t stream);
+                       int threads, float scale, cudaStream_t stream);
 cudaError_t launch_adam(int n, float* w, const double* grad, float* m, float* v, int step, float lr,
                         float b1, float b2, float eps, float w_min, cudaStream_t stream);
 

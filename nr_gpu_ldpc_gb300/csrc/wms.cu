@@ -24,8 +24,12 @@
 // shared memory: dloss/dR^t_e = g[col] + h_e, dloss/dQ^t_e = g[col] + (argmin
 // terms), g[col] = dloss/dQ^t_e, and h_e = -dloss/dQ^t_e is carried to
 // iteration t-1 as the gradient of R^{t-1}_e (per lifted edge, in global
-// memory: it does not compress to two numbers per row).
+// memory: it does not compress to two numbers per row; a row's h and its loss
+// seed are staged in shared memory one row ahead -- read in the row itself they
+// left the kernel issuing in a third of its cycles).
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "nrldpc_internal.h"
 
@@ -43,6 +47,28 @@ __device__ __forceinline__ float max_nan(float a, float b) {
 
 __device__ __forceinline__ int cw_bit(const uint8_t* cw, int c) { return (cw[c >> 3] >> (c & 7)) & 1; }
 
+// 32-bit shared-memory accesses by byte address, in program order.
+__device__ __forceinline__ float lds(uint32_t a) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void sts(uint32_t a, float v) {
+    asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+__device__ __forceinline__ void add_shared(uint32_t a, float v) {
+    asm volatile("red.shared.add.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+
+// Byte offset of sub-row s's position, 4 (c Z + (s + V) mod Z), from an edge's
+// {column, 4V} (s4 = 4 s, z4 = 4 Z): where s + V < Z the difference wraps
+// around to a large unsigned number.
+template <typename EdgeWord>  // uint2 or uint4
+__device__ __forceinline__ uint32_t edge_off(const EdgeWord& ea, uint32_t s4, uint32_t z4) {
+    const uint32_t t = s4 + ea.y;
+    return __viaddmin_u32(t, 0u - z4, t) + ea.x;
+}
+
 // Per-thread asynchronous copies global -> shared (each thread waits only
 // for its own groups; the sources are in-bounds device memory, so every
 // copy completes).
@@ -52,8 +78,8 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -67,6 +93,10 @@ __device__ __forceinline__ void cp_async_wait() {
 // of look-ahead in registers left the kernel waiting on loads).
 constexpr int kRing = 4;
 constexpr size_t kRingBytes = static_cast<size_t>(kRing) * kMaxThreads * (16 + 16 + 4);
+
+// Longest row that the adjoints unroll (and whose dloss/dR the layered one
+// stages in shared memory); longer ones run in a loop.
+constexpr int kUnrolled = 10;
 
 // Stored state of one lifted row after iteration t (16 B): min1, min2,
 // info = i1 | i2 << 5 | Q sign bits << 10 (i2 = 31: no second argmin), and
@@ -110,6 +140,7 @@ __device__ __forceinline__ float loss_term(float L, bool bit1, float scale, floa
 // a row's weights come in as 128-bit loads: [2][kMaxRows][kWPad].
 constexpr int kWPad = 20;
 constexpr int kFwdWeightFloats = 2 * kMaxRows * kWPad;
+static_assert(kFwdWeightFloats >= 5 * kMaxEdges, "the adjoints' edge words and gradient sums take the weights' place");
 
 // Weight i of a padded row held as float4s (i is constant after unrolling).
 __device__ __forceinline__ float wsel(const float4* w, int i) {
@@ -124,19 +155,26 @@ __device__ __forceinline__ float wsel(const float4* w, int i) {
 // is the sign bit of Q_i + 0 ((Q < 0): -0 gives +0, a NaN result is the
 // canonical positive NaN), collected by a funnel shift (edge i at bit
 // D-1-i) and bit-reversed into the stored order (edge i at bit i).
+// l: shared address of the posteriors read; dnew: from there to the ones
+// written.
 template <int D, bool LAYERED>
-__device__ __forceinline__ void fwd_row(const CodeTable& tab, int e0, uint32_t s, const float* lold,
-                                        float* lnew, const float4* w_prev, const float4* w_cur,
-                                        uint4 st, uint4* st_out, bool sfx, bool ybit, float* seed_t,
-                                        float scale, float* loss) {
+__device__ __forceinline__ void fwd_row(const CodeTable& tab, int e0, uint32_t s4, uint32_t z4, uint32_t l,
+                                        uint32_t dnew, const float4* w_prev, const float4* w_cur, uint4 st,
+                                        uint4* st_out, bool sfx, bool ybit, float* seed_t, float scale,
+                                        float* loss) {
     constexpr int LAST = D - 1;
-    const uint32_t z = static_cast<uint32_t>(tab.z);
     uint32_t addr[D];
     float lv[D], rold[D];
 #pragma unroll
     for (int i = 0; i < D; i++) {
-        addr[i] = edge_at(tab.edge[e0 + i], s, z);
-        lv[i] = (i == LAST && sfx) ? __uint_as_float(st.w) : lold[addr[i]];
+        const uint32_t off = edge_off(tab.eaddr[e0 + i], s4, z4);
+        if (i == LAST && sfx) {
+            addr[i] = off;  // of its loss seed
+            lv[i] = __uint_as_float(st.w);
+        } else {
+            addr[i] = l + off;
+            lv[i] = lds(addr[i]);
+        }
     }
     const float om1 = __uint_as_float(st.x), om2 = __uint_as_float(st.y);
     const uint32_t oq = st.z >> 10;
@@ -162,12 +200,17 @@ __device__ __forceinline__ void fwd_row(const CodeTable& tab, int e0, uint32_t s
     }
     const uint32_t qmask = __brev(qrev) >> (32 - D);  // Q_i's sign at bit i
     const uint32_t rsign = qmask ^ (0u - (static_cast<uint32_t>(__popc(qmask)) & 1u));  // R_new_i's
+    // the posteriors written are read kAhead edges before their stores (fewer
+    // live registers than the whole row)
+    constexpr int kAhead = 4;
+    auto posterior = [&](int i) { return (LAYERED || (i == LAST && sfx)) ? lv[i] : lds(addr[i] + dnew); };
     float nv[D];
 #pragma unroll
-    for (int i = 0; i < D; i++) nv[i] = (LAYERED || (i == LAST && sfx)) ? lv[i] : lnew[addr[i]];
+    for (int i = 0; i < kAhead && i < D; i++) nv[i] = posterior(i);
     float sfx_new = 0.0f;
 #pragma unroll
     for (int i = 0; i < D; i++) {
+        if (i + kAhead < D) nv[i + kAhead] = posterior(i + kAhead);
         const float mag = __fmul_rn(wsel(w_cur, i), i == i1 ? m2 : m1);
         const float rn = __uint_as_float(__float_as_uint(mag) ^ ((rsign << (31 - i)) & 0x80000000u));
         // layered: A = Q + R_new; flooding: Lnew += R_new - R_old
@@ -175,11 +218,12 @@ __device__ __forceinline__ void fwd_row(const CodeTable& tab, int e0, uint32_t s
         if (i == LAST && sfx)
             sfx_new = v;
         else
-            lnew[addr[i]] = v;
+            sts(addr[i] + dnew, v);
     }
     *st_out = make_uint4(__float_as_uint(m1), __float_as_uint(m2), pack_info(i1, i2, qmask),
                          __float_as_uint(sfx_new));
-    if (sfx) seed_t[addr[LAST]] = loss_term(sfx_new, ybit, scale, loss);
+    if (sfx)
+        *reinterpret_cast<float*>(reinterpret_cast<char*>(seed_t) + addr[LAST]) = loss_term(sfx_new, ybit, scale, loss);
 }
 
 // Degree switch up to MAXD (the code's largest row degree class: 10 covers
@@ -192,14 +236,14 @@ __device__ __forceinline__ void fwd_row(const CodeTable& tab, int e0, uint32_t s
     }
 
 template <int MAXD, bool LAYERED>
-__device__ __forceinline__ void fwd_dispatch(int deg, const CodeTable& tab, int e0, uint32_t s,
-                                             const float* lold, float* lnew, const float4* wp,
-                                             const float4* wc, uint4 st, uint4* st_out, bool sfx, bool ybit,
-                                             float* seed_t, float scale, float* loss) {
+__device__ __forceinline__ void fwd_dispatch(int deg, const CodeTable& tab, int e0, uint32_t s4, uint32_t z4,
+                                             uint32_t l, uint32_t dnew, const float4* wp, const float4* wc, uint4 st,
+                                             uint4* st_out, bool sfx, bool ybit, float* seed_t, float scale,
+                                             float* loss) {
 #define NRLDPC_FWD_CASE(D)                                                                         \
     case D:                                                                                        \
         if constexpr (D <= MAXD)                                                                   \
-            fwd_row<D, LAYERED>(tab, e0, s, lold, lnew, wp, wc, st, st_out, sfx, ybit, seed_t, scale, loss); \
+            fwd_row<D, LAYERED>(tab, e0, s4, z4, l, dnew, wp, wc, st, st_out, sfx, ybit, seed_t, scale, loss); \
         break;
     NRLDPC_DEG_SWITCH(NRLDPC_FWD_CASE)
 #undef NRLDPC_FWD_CASE
@@ -307,8 +351,8 @@ __global__ void __launch_bounds__(kMaxThreads, kWmsMinBlocks)
             for (int r = 0; r < rows; r++) {
                 const uint4 p2 = fetch(r + 2);
                 if (act)
-                    fwd_dispatch<MAXD, LAYERED>(tab.row_deg[r], tab, tab.row_ptr[r], s, lold, lnew,
-                                                wrow + r * (kWPad / 4), wrow + (kMaxRows + r) * (kWPad / 4), p0,
+                    fwd_dispatch<MAXD, LAYERED>(tab.row_deg[r], tab, tab.row_ptr[r], 4u * s, 4u * z, smem_u32(lold),
+                                                smem_u32(lnew) - smem_u32(lold), wrow + r * (kWPad / 4), wrow + (kMaxRows + r) * (kWPad / 4), p0,
                                                 st_cur + r * z + s, tab.row_sfx[r] != 0,
                                                 (ysfx >> r) & 1u, seed_t, a.scale, &loss_part);
                 p0 = p1;
@@ -357,8 +401,9 @@ __global__ void __launch_bounds__(kMaxThreads, kWmsMinBlocks)
 // half with its partner, P - 1 shuffles for P = D rounded up to a power of
 // two) followed by a plain reduction over the remaining lane bits, instead of
 // a 5-shuffle reduction per value.
-template <int D>
-__device__ __forceinline__ void warp_sum_to(float (&v)[D], float* acc) {
+// OWN: acc belongs to this warp alone, so a plain add does.  count: sums wanted.
+template <int D, bool OWN = false>
+__device__ __forceinline__ void warp_sum_to(float (&v)[D], float* acc, int count = D) {
     constexpr int P = D <= 1 ? 1 : D <= 2 ? 2 : D <= 4 ? 4 : D <= 8 ? 8 : D <= 16 ? 16 : 32;
     constexpr int LOGP = P == 1 ? 0 : P == 2 ? 1 : P == 4 ? 2 : P == 8 ? 3 : P == 16 ? 4 : 5;
     const int lane = static_cast<int>(threadIdx.x & 31u);
@@ -382,7 +427,10 @@ __device__ __forceinline__ void warp_sum_to(float (&v)[D], float* acc) {
     // lane L now holds the sum for value L >> (5 - LOGP)
     if ((lane & ((32 >> LOGP) - 1)) == 0) {
         const int i = lane >> (5 - LOGP);
-        if (i < D) atomicAdd(&acc[i], w[0]);
+        if (i < D && i < count) {
+            if (OWN) acc[i] += w[0];
+            else atomicAdd(&acc[i], w[0]);
+        }
     }
 }
 
@@ -390,64 +438,122 @@ __device__ __forceinline__ void warp_sum_to(float (&v)[D], float* acc) {
 // gl = dloss/dL^{t+1} and gl_next = dloss/dL^t over the core columns.  The
 // suffix edge's dloss/dL^{t+1} is its loss seed plus what the next
 // iteration's row sent back through Q (only this row touches the column).
+// Inactive threads (act false) read some slot's buffer and add zeros to the
+// weight gradients: no branch per edge.
+// The signs enter as bits (dloss/dR times a sign is a flipped sign bit), and
+// the two argmin edges' positions are looked up at the end instead of selected
+// in the edge loop.  edges: the row's first {column, 4V, weight} in shared
+// memory, one 128-bit read per edge (from the parameter bank the compiler's
+// non-uniform constant loads left the kernel waiting on them).
+struct BwdRow {
+    float m1, m2, acc1, acc2;  // acc: dloss/d min1, dloss/d min2
+    int i1, i2;
+    uint32_t q, rsign;         // signs of Q_i and R_i at bit i
+};
+
+__device__ __forceinline__ BwdRow bwd_open(uint4 st) {
+    BwdRow r;
+    r.m1 = __uint_as_float(st.x);
+    r.m2 = __uint_as_float(st.y);
+    r.acc1 = r.acc2 = 0.0f;
+    r.i1 = static_cast<int>(st.z & 31u);
+    r.i2 = static_cast<int>((st.z >> 5) & 31u);
+    r.q = st.z >> 10;
+    r.rsign = r.q ^ (0u - (static_cast<uint32_t>(__popc(r.q)) & 1u));
+    return r;
+}
+
+// Edge i with dloss/dR = gr: its share of the minima's gradients; returns the
+// weight's gradient.
+__device__ __forceinline__ float bwd_edge(BwdRow& r, int i, float gr, float w, bool act) {
+    const float gs = __uint_as_float(__float_as_uint(gr) ^ ((r.rsign << (31 - i)) & 0x80000000u));
+    const float t = gs * w;
+    if (i == r.i1) r.acc2 = t;
+    else r.acc1 += t;
+    return act ? gs * (i == r.i1 ? r.m2 : r.m1) : 0.0f;
+}
+
+// dloss/dR of edge i: dloss/dL^{t+1} minus what the next iteration's row sent
+// back through Q (gin: to its two argmin edges).
+__device__ __forceinline__ float bwd_gr(int i, bool is_sfx, const uint4& ed, uint32_t s4, uint32_t z4, uint32_t gl,
+                                        const uint4& gin, float sfx_seed) {
+    const float back = i == static_cast<int>(gin.z)   ? __uint_as_float(gin.x)
+                       : i == static_cast<int>(gin.w) ? __uint_as_float(gin.y)
+                                                      : 0.0f;
+    const float glv = is_sfx ? __fadd_rn(sfx_seed, back) : lds(gl + edge_off(ed, s4, z4));
+    return glv - back;
+}
+
+// The argmin edges' dloss/dQ: to the posteriors' gradients of the iteration
+// before, and kept for its row.
+__device__ __forceinline__ void bwd_close(const BwdRow& r, int deg, uint32_t s4, uint32_t z4, bool act,
+                                          uint32_t gl_next, const uint4* edges, uint4* gq_io, bool scatter, bool sfx) {
+    if (!act) return;
+    const bool has1 = r.m1 < 1000.0f, has2 = r.i2 < deg && r.m2 < 1000.0f;
+    const float g1 = has1 ? __uint_as_float(__float_as_uint(r.acc1) ^ ((r.q >> r.i1) << 31)) : 0.0f;
+    const float g2 = has2 ? __uint_as_float(__float_as_uint(r.acc2) ^ ((r.q >> r.i2) << 31)) : 0.0f;
+    if (scatter) {  // the suffix column's share comes back through gq instead
+        if (has1 && !(sfx && r.i1 == deg - 1)) add_shared(gl_next + edge_off(edges[r.i1], s4, z4), g1);
+        if (has2 && !(sfx && r.i2 == deg - 1)) add_shared(gl_next + edge_off(edges[r.i2], s4, z4), g2);
+    }
+    *gq_io = make_uint4(__float_as_uint(g1), __float_as_uint(g2), static_cast<uint32_t>(r.i1),
+                        static_cast<uint32_t>(r.i2 < deg ? r.i2 : 31));
+}
+
 template <int D>
-__device__ __forceinline__ void bwd_row(const CodeTable& tab, int e0, uint32_t s, bool act,
-                                        const float* gl, float* gl_next, const float* w_cur,
-                                        float* gw_acc, uint4 st, uint4 gin, uint4* gq_io, bool scatter,
-                                        bool sfx, float sfx_seed) {
-    constexpr int LAST = D - 1;
-    const uint32_t z = static_cast<uint32_t>(tab.z);
-    const float m1 = __uint_as_float(st.x), m2 = __uint_as_float(st.y);
-    const int i1 = static_cast<int>(st.z & 31u), i2 = static_cast<int>((st.z >> 5) & 31u);
-    const uint32_t q = st.z >> 10;
-    const uint32_t par = static_cast<uint32_t>(__popc(q) & 1);
-    const float g1n = __uint_as_float(gin.x), g2n = __uint_as_float(gin.y);
-    const int j1 = static_cast<int>(gin.z), j2 = static_cast<int>(gin.w);
-    uint32_t ad1 = 0, ad2 = 0;  // columns of the two argmin edges
-    float acc1 = 0.0f, acc2 = 0.0f;
+__device__ __forceinline__ void bwd_row(uint32_t s4, uint32_t z4, bool act, uint32_t gl, uint32_t gl_next,
+                                        const uint4* edges, float* gw_acc, uint4 st, uint4 gin,
+                                        uint4* gq_io, bool scatter, bool sfx, float sfx_seed) {
+    BwdRow r = bwd_open(st);
     float gwv[D];
 #pragma unroll
     for (int i = 0; i < D; i++) {
-        const uint32_t a = edge_at(tab.edge[e0 + i], s, z);
-        ad1 = i == i1 ? a : ad1;
-        ad2 = i == i2 ? a : ad2;
-        float gr = 0.0f;
-        if (act) {
-            const float back = i == j1 ? g1n : (i == j2 ? g2n : 0.0f);
-            const float glv = (i == LAST && sfx) ? __fadd_rn(sfx_seed, back) : gl[a];
-            gr = glv - back;
-        }
-        const float sg = ((par ^ (q >> i)) & 1u) ? -1.0f : 1.0f;
-        const float mag = i == i1 ? m2 : m1;
-        gwv[i] = act ? gr * sg * mag : 0.0f;
-        const float t = gr * w_cur[e0 + i] * sg;
-        if (i == i1) acc2 = t;
-        else acc1 += t;
+        const uint4 ed = edges[i];
+        gwv[i] = bwd_edge(r, i, bwd_gr(i, i == D - 1 && sfx, ed, s4, z4, gl, gin, sfx_seed), __uint_as_float(ed.z), act);
     }
-    warp_sum_to<D>(gwv, gw_acc + e0);
-    float g1 = 0.0f, g2 = 0.0f;
-    if (act) {
-        if (m1 < 1000.0f) g1 = acc1 * (((q >> i1) & 1u) ? -1.0f : 1.0f);
-        if (i2 < D && m2 < 1000.0f) g2 = acc2 * (((q >> i2) & 1u) ? -1.0f : 1.0f);
-        if (scatter) {  // the suffix column's share comes back through gq instead
-            if (m1 < 1000.0f && !(sfx && i1 == LAST)) atomicAdd(&gl_next[ad1], g1);
-            if (i2 < D && m2 < 1000.0f && !(sfx && i2 == LAST)) atomicAdd(&gl_next[ad2], g2);
+    warp_sum_to<D>(gwv, gw_acc);
+    bwd_close(r, D, s4, z4, act, gl_next, edges, gq_io, scatter, sfx);
+}
+
+// Rows of more than kUnrolled edges, eight edges at a time in a loop: unrolled,
+// a row of 19 pushed the rows requested ahead out of the registers (BG1 Z=384
+// 1,000 codewords x 6 it: forward and adjoint 3.55 -> 2.97 ms with rows in
+// pieces).
+__device__ __forceinline__ void bwd_long_row(int deg, uint32_t s4, uint32_t z4, bool act, uint32_t gl,
+                                             uint32_t gl_next, const uint4* edges, float* gw_acc, uint4 st, uint4 gin,
+                                             uint4* gq_io, bool scatter, bool sfx, float sfx_seed) {
+    constexpr int N = 8;
+    BwdRow r = bwd_open(st);
+#pragma unroll 1
+    for (int from = 0; from < deg; from += N) {
+        float gwv[N];
+#pragma unroll
+        for (int k = 0; k < N; k++) {
+            const int i = from + k;
+            gwv[k] = 0.0f;
+            if (i >= deg) continue;
+            const uint4 ed = edges[i];
+            gwv[k] = bwd_edge(r, i, bwd_gr(i, i == deg - 1 && sfx, ed, s4, z4, gl, gin, sfx_seed),
+                              __uint_as_float(ed.z), act);
         }
-        *gq_io = make_uint4(__float_as_uint(g1), __float_as_uint(g2), static_cast<uint32_t>(i1),
-                            static_cast<uint32_t>(i2 < D ? i2 : 31));
+        warp_sum_to<N>(gwv, gw_acc + from, deg - from);
     }
+    bwd_close(r, deg, s4, z4, act, gl_next, edges, gq_io, scatter, sfx);
 }
 
 template <int MAXD>
-__device__ __forceinline__ void bwd_dispatch(int deg, const CodeTable& tab, int e0, uint32_t s,
-                                             bool act, const float* gl, float* gln, const float* wc,
-                                             float* gw_acc, uint4 st, uint4 gin, uint4* gq, bool scatter,
+__device__ __forceinline__ void bwd_dispatch(int deg, uint32_t s4, uint32_t z4, bool act, uint32_t gl, uint32_t gln,
+                                             const uint4* edges, float* gw_acc, uint4 st, uint4 gin, uint4* gq, bool scatter,
                                              bool sfx, float sfx_seed) {
 #define NRLDPC_BWD_CASE(D)                                                                           \
     case D:                                                                                          \
-        if constexpr (D <= MAXD) bwd_row<D>(tab, e0, s, act, gl, gln, wc, gw_acc, st, gin, gq, scatter, sfx, sfx_seed); \
+        if constexpr (D <= kUnrolled)                                                                \
+            bwd_row<D>(s4, z4, act, gl, gln, edges, gw_acc, st, gin, gq, scatter, sfx, sfx_seed);    \
         break;
-    NRLDPC_DEG_SWITCH(NRLDPC_BWD_CASE)
+    if (MAXD > kUnrolled && deg > kUnrolled)
+        bwd_long_row(deg, s4, z4, act, gl, gln, edges, gw_acc, st, gin, gq, scatter, sfx, sfx_seed);
+    else
+        NRLDPC_DEG_SWITCH(NRLDPC_BWD_CASE)
 #undef NRLDPC_BWD_CASE
 }
 
@@ -456,14 +562,15 @@ __global__ void __launch_bounds__(kMaxThreads, kWmsMinBlocks)
     wms_backward_kernel(const __grid_constant__ CodeTable tab, const __grid_constant__ WmsArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     int* s_group = reinterpret_cast<int*>(smem);
-    float* wcur = reinterpret_cast<float*>(smem + kHdr);  // [E]
-    float* gw_acc = wcur + kMaxEdges;                     // [E]
-    float* bufs = gw_acc + kMaxEdges;
+    uint4* edges = reinterpret_cast<uint4*>(smem + kHdr);            // [E] {column, 4V, weight of the iteration}
+    float* gw_acc = reinterpret_cast<float*>(edges + kMaxEdges);     // [E]
+    float* bufs = reinterpret_cast<float*>(smem + kHdr + kFwdWeightFloats * sizeof(float));
     const int z = tab.z, n = tab.n_bp, cpb = a.cpb, rows = tab.rows, E = tab.n_edges;
     const int cf = tab.core_floats, ncz = tab.n_core * z;
     const int tid = threadIdx.x, slot = tid / z;
     const uint32_t s = static_cast<uint32_t>(tid - slot * z);
     const bool valid = slot < cpb;
+    for (int e = tid; e < E; e += blockDim.x) edges[e] = make_uint4(tab.eaddr[e].x, tab.eaddr[e].y, 0u, 0u);
     // row ring (BG2 kernels): [kRing][blockDim] states, dloss/dQ, seeds
     uint4* ring_st = reinterpret_cast<uint4*>(bufs + 2 * static_cast<size_t>(cpb) * cf);
     uint4* ring_gq = ring_st + kRing * blockDim.x;
@@ -486,7 +593,7 @@ __global__ void __launch_bounds__(kMaxThreads, kWmsMinBlocks)
         }
         for (int t = a.T - 1; t >= 0; t--) {
             for (int e = tid; e < E; e += blockDim.x) {
-                wcur[e] = a.weights[t * E + e];
+                edges[e].z = __float_as_uint(a.weights[t * E + e]);
                 gw_acc[e] = 0.0f;
             }
             if (act && t > 0) {
@@ -506,7 +613,7 @@ __global__ void __launch_bounds__(kMaxThreads, kWmsMinBlocks)
                         cp_async16(&ring_st[k], st + r * z + s);
                         cp_async16(&ring_gq[k], gq + r * z + s);
                         if (tab.row_sfx[r])
-                            cp_async4(&ring_sd[k], seed_t + edge_at(tab.edge[tab.row_ptr[r + 1] - 1], s, z));
+                            cp_async4(smem_u32(&ring_sd[k]), seed_t + edge_at(tab.edge[tab.row_ptr[r + 1] - 1], s, z));
                     }
                     cp_async_commit();
                 };
@@ -518,7 +625,8 @@ __global__ void __launch_bounds__(kMaxThreads, kWmsMinBlocks)
                     const uint4 sv = act ? ring_st[k] : make_uint4(0u, 0u, 31u << 5, 0u);
                     const uint4 gv = act ? ring_gq[k] : make_uint4(0u, 0u, 31u, 31u);
                     const float sd = (act && tab.row_sfx[r]) ? ring_sd[k] : 0.0f;
-                    bwd_dispatch<MAXD>(tab.row_deg[r], tab, tab.row_ptr[r], s, act, gl, gln, wcur, gw_acc, sv, gv,
+                    bwd_dispatch<MAXD>(tab.row_deg[r], 4u * s, 4u * z, act, smem_u32(gl), smem_u32(gln),
+                                       edges + tab.row_ptr[r], gw_acc + tab.row_ptr[r], sv, gv,
                                        gq + r * z + s, t > 0, tab.row_sfx[r] != 0, sd);
                 }
                 cp_async_wait<0>();
@@ -543,7 +651,8 @@ __global__ void __launch_bounds__(kMaxThreads, kWmsMinBlocks)
                     uint4 s2, g2;
                     float d2;
                     fetch(r + 2, s2, g2, d2);
-                    bwd_dispatch<MAXD>(tab.row_deg[r], tab, tab.row_ptr[r], s, act, gl, gln, wcur, gw_acc, s0, g0,
+                    bwd_dispatch<MAXD>(tab.row_deg[r], 4u * s, 4u * z, act, smem_u32(gl), smem_u32(gln),
+                                       edges + tab.row_ptr[r], gw_acc + tab.row_ptr[r], s0, g0,
                                        gq + r * z + s, t > 0, tab.row_sfx[r] != 0, d0);
                     s0 = s1;
                     g0 = g1;
@@ -567,65 +676,95 @@ __global__ void __launch_bounds__(kMaxThreads, kWmsMinBlocks)
 // g = dloss/dA over the core columns.  The suffix column's dloss/dA before
 // its row is its loss seed minus the dloss/dR carried from the next
 // iteration (h = -dloss/dQ there), the value the in-place A had.
-template <int D, bool SEED_IN_ROW>
-__device__ __forceinline__ void bwd_layered_row(const CodeTable& tab, int e0, uint32_t s, bool act, float* g,
-                                                const float* w_cur, float* gw_acc, uint4 st, float* gh_row,
-                                                bool has_h, bool write_h, bool sfx, float sfx_seed,
-                                                const float* seed_t) {
-    constexpr int LAST = D - 1;
-    const uint32_t z = static_cast<uint32_t>(tab.z);
-    const float m1 = __uint_as_float(st.x), m2 = __uint_as_float(st.y);
-    const int i1 = static_cast<int>(st.z & 31u), i2 = static_cast<int>((st.z >> 5) & 31u);
-    const uint32_t q = st.z >> 10;
-    const uint32_t par = static_cast<uint32_t>(__popc(q) & 1);
-    uint32_t ad[D];
-    float ga[D];
-    float gwv[D];
-    float to1 = 0.0f, to2 = 0.0f;  // dloss/dQ at the argmin edges through R
-#pragma unroll
-    for (int i = 0; i < D; i++) {
-        const uint32_t a = edge_at(tab.edge[e0 + i], s, z);
-        ad[i] = a;
-        float dr = 0.0f;
-        ga[i] = 0.0f;
-        if (act) {
-            const float h = has_h ? gh_row[i * z] : 0.0f;
-            ga[i] = (i == LAST && sfx) ? __fsub_rn(SEED_IN_ROW ? __ldcs(seed_t + a) : sfx_seed, h) : g[a];
-            dr = ga[i] + h;
-        }
-        const float sg = ((par ^ (q >> i)) & 1u) ? -1.0f : 1.0f;
-        const float mag = i == i1 ? m2 : m1;
-        gwv[i] = act ? dr * sg * mag : 0.0f;
-        const float t = dr * w_cur[e0 + i] * sg;
-        if (i == i1) to2 = t;
-        else to1 += t;
-    }
-    warp_sum_to<D>(gwv, gw_acc + e0);
+// The two argmin edges' dloss/dQ, which is dloss/dA before this row.
+__device__ __forceinline__ void bwd_layered_close(const BwdRow& r, int deg, uint32_t s4, uint32_t z4, bool act,
+                                                  uint32_t g, const uint4* edges, float* gh_row, bool write_h,
+                                                  bool sfx, float ga_last) {
     if (!act) return;
-    const float g1 = m1 < 1000.0f ? to1 * (((q >> i1) & 1u) ? -1.0f : 1.0f) : 0.0f;
-    const float g2 = (i2 < D && m2 < 1000.0f) ? to2 * (((q >> i2) & 1u) ? -1.0f : 1.0f) : 0.0f;
+    const int z = static_cast<int>(z4 / 4);
+    auto argmin_edge = [&](int i, float gm) {
+        const bool out = sfx && i == deg - 1;
+        const uint32_t at = g + edge_off(edges[i], s4, z4);
+        const float dq = (out ? ga_last : lds(at)) + gm;
+        if (!out) sts(at, dq);
+        if (write_h) gh_row[i * z] = -dq;
+    };
+    const float g1 = r.m1 < 1000.0f ? __uint_as_float(__float_as_uint(r.acc1) ^ ((r.q >> r.i1) << 31)) : 0.0f;
+    const float g2 = r.m2 < 1000.0f ? __uint_as_float(__float_as_uint(r.acc2) ^ ((r.q >> r.i2) << 31)) : 0.0f;
+    argmin_edge(r.i1, g1);
+    if (r.i2 < deg) argmin_edge(r.i2, g2);
+}
+
+// h_row: shared address of the row's staged dloss/dR (edge i h_step bytes on).
+// dloss/dR^{t-1} = -dloss/dQ goes out edge by edge as if no edge were an
+// argmin; the two that are follow.
+template <int D>
+__device__ __forceinline__ void bwd_layered_row(uint32_t s4, uint32_t z4, bool act, uint32_t g, const uint4* edges,
+                                                float* gw_acc, uint4 st, uint32_t h_row, uint32_t h_step,
+                                                float* gh_row, bool write_h, bool sfx, float sfx_seed) {
+    const int z = static_cast<int>(z4 / 4);
+    BwdRow r = bwd_open(st);
+    float gwv[D], ga_last = 0.0f;
 #pragma unroll
     for (int i = 0; i < D; i++) {
-        float dq = ga[i];
-        if (i == i1) dq += g1;
-        if (i == i2) dq += g2;
-        if ((i == i1 || i == i2) && !(i == LAST && sfx)) g[ad[i]] = dq;  // dloss/dA before this row
-        if (write_h) gh_row[i * z] = -dq;                                // dloss/dR^{t-1}
+        const uint4 ed = edges[i];
+        const float h = lds(h_row + i * h_step);
+        const float ga = (i == D - 1 && sfx) ? __fsub_rn(sfx_seed, h) : lds(g + edge_off(ed, s4, z4));
+        if (i == D - 1) ga_last = ga;
+        gwv[i] = bwd_edge(r, i, ga + h, __uint_as_float(ed.z), act);
+        if (write_h && act) gh_row[i * z] = -ga;
     }
+    warp_sum_to<D, true>(gwv, gw_acc, D);
+    bwd_layered_close(r, D, s4, z4, act, g, edges, gh_row, write_h, sfx, ga_last);
+}
+
+// Rows of more than kUnrolled edges, of any degree: eight edges at a time in a
+// loop, their dloss/dR from global memory (has_h: not at the last iteration).
+// Unrolled like the shorter rows their registers made the compiler spill in
+// every row (BG1 has 4 rows of 19 among 46), and the spills miss the little L1
+// that two CTAs' shared memory leaves.
+__device__ __forceinline__ void bwd_layered_long_row(int deg, uint32_t s4, uint32_t z4, bool act, uint32_t g,
+                                                     const uint4* edges, float* gw_acc, uint4 st, float* gh_row,
+                                                     bool has_h, bool write_h, bool sfx, float sfx_seed) {
+    constexpr int N = 8;
+    const int z = static_cast<int>(z4 / 4);
+    BwdRow r = bwd_open(st);
+    float ga_last = 0.0f;
+#pragma unroll 1
+    for (int from = 0; from < deg; from += N) {
+        float gwv[N], h[N];
+#pragma unroll
+        for (int k = 0; k < N; k++) h[k] = has_h && from + k < deg ? __ldcg(gh_row + (from + k) * z) : 0.0f;
+#pragma unroll
+        for (int k = 0; k < N; k++) {
+            const int i = from + k;
+            gwv[k] = 0.0f;
+            if (i >= deg) continue;
+            const uint4 ed = edges[i];
+            const float ga = (i == deg - 1 && sfx) ? __fsub_rn(sfx_seed, h[k]) : lds(g + edge_off(ed, s4, z4));
+            if (i == deg - 1) ga_last = ga;
+            gwv[k] = bwd_edge(r, i, ga + h[k], __uint_as_float(ed.z), act);
+            if (write_h && act) gh_row[i * z] = -ga;
+        }
+        warp_sum_to<N, true>(gwv, gw_acc + from, deg - from);
+    }
+    bwd_layered_close(r, deg, s4, z4, act, g, edges, gh_row, write_h, sfx, ga_last);
 }
 
 template <int MAXD>
-__device__ __forceinline__ void bwd_layered_dispatch(int deg, const CodeTable& tab, int e0, uint32_t s, bool act,
-                                                     float* g, const float* wc, float* gw_acc, uint4 st,
-                                                     float* gh_row, bool has_h, bool write_h, bool sfx,
-                                                     float sfx_seed, const float* seed_t) {
+__device__ __forceinline__ void bwd_layered_dispatch(int deg, uint32_t s4, uint32_t z4, bool act, uint32_t g,
+                                                     const uint4* edges, float* gw_acc, uint4 st, uint32_t h_row,
+                                                     uint32_t h_step, float* gh_row, bool has_h, bool write_h,
+                                                     bool sfx, float sfx_seed) {
 #define NRLDPC_BWDL_CASE(D)                                                                                 \
     case D:                                                                                                 \
-        if constexpr (D <= MAXD)                                                                            \
-            bwd_layered_row<D, (MAXD > 10)>(tab, e0, s, act, g, wc, gw_acc, st, gh_row, has_h, write_h, sfx,      \
-                                            sfx_seed, seed_t);                                                    \
+        if constexpr (D <= kUnrolled)                                                                         \
+            bwd_layered_row<D>(s4, z4, act, g, edges, gw_acc, st, h_row, h_step, gh_row, write_h, sfx, sfx_seed); \
         break;
-    NRLDPC_DEG_SWITCH(NRLDPC_BWDL_CASE)
+    if (MAXD > kUnrolled && deg > kUnrolled)
+        bwd_layered_long_row(deg, s4, z4, act, g, edges, gw_acc, st, gh_row, has_h, write_h, sfx, sfx_seed);
+    else
+        NRLDPC_DEG_SWITCH(NRLDPC_BWDL_CASE)
 #undef NRLDPC_BWDL_CASE
 }
 
@@ -634,15 +773,24 @@ __global__ void __launch_bounds__(kMaxThreads, kWmsMinBlocks)
     wms_backward_layered_kernel(const __grid_constant__ CodeTable tab, const __grid_constant__ WmsArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     int* s_group = reinterpret_cast<int*>(smem);
-    float* wcur = reinterpret_cast<float*>(smem + kHdr);  // [E]
-    float* gw_acc = wcur + kMaxEdges;                     // [E]
-    float* bufs = gw_acc + kMaxEdges;
+    uint4* edges = reinterpret_cast<uint4*>(smem + kHdr);            // [E] {column, 4V, weight of the iteration}
+    float* bufs = reinterpret_cast<float*>(smem + kHdr + kFwdWeightFloats * sizeof(float));
     const int z = tab.z, n = tab.n_bp, cpb = a.cpb, rows = tab.rows, E = tab.n_edges;
     const int cf = tab.core_floats, ncz = tab.n_core * z;
     const int tid = threadIdx.x, slot = tid / z;
     const uint32_t s = static_cast<uint32_t>(tid - slot * z);
     const bool valid = slot < cpb;
+    for (int e = tid; e < E; e += blockDim.x) edges[e] = make_uint4(tab.eaddr[e].x, tab.eaddr[e].y, 0u, 0u);
     float* gh = a.gh + (static_cast<size_t>(blockIdx.x) * cpb + (valid ? slot : 0)) * E * z;
+    // this thread's column of the staging buffers [2 rows][kUnrolled edges, seed][threads]
+    uint4* staged_st = reinterpret_cast<uint4*>(bufs + static_cast<size_t>(cpb) * cf) + tid;  // [2 rows][threads]
+    float* staged = reinterpret_cast<float*>(staged_st - tid + 2 * blockDim.x);
+    const uint32_t h_step = 4u * blockDim.x, ring = smem_u32(staged) + 4u * tid;
+    // weight gradients of the iteration, one array per warp (adding to a common
+    // one with atomics, every warp at the same few words, took 4% longer)
+    const int warps = blockDim.x / 32;
+    float* gw_all = staged + 2 * (kUnrolled + 1) * blockDim.x;  // [warps][E]
+    float* gw_acc = gw_all + (tid >> 5) * E;
     for (;;) {
         if (tid == 0) *s_group = atomicAdd(a.work_counter, 1);
         __syncthreads();
@@ -653,10 +801,12 @@ __global__ void __launch_bounds__(kMaxThreads, kWmsMinBlocks)
         float* g = bufs + static_cast<size_t>(valid ? slot : 0) * cf;  // dloss/dA
         if (act)
             for (int c = static_cast<int>(s); c < ncz; c += z) g[c] = 0.0f;
+        for (int i = 0; i < 2 * (kUnrolled + 1); i++) sts(ring + i * h_step, 0.0f);  // no dloss/dR at the last iteration
+        for (int i = 0; i < 2; i++) staged_st[i * blockDim.x] = make_uint4(0u, 0u, 31u << 5, 0u);  // inactive threads'
         for (int t = a.T - 1; t >= 0; t--) {
             for (int e = tid; e < E; e += blockDim.x) {
-                wcur[e] = a.weights[t * E + e];
-                gw_acc[e] = 0.0f;
+                edges[e].z = __float_as_uint(a.weights[t * E + e]);
+                for (int w = 0; w < warps; w++) gw_all[w * E + e] = 0.0f;
             }
             const float* seed_t = a.gseed + (static_cast<size_t>(t) * a.n_cw + (act ? cw : 0)) * n;
             if (act) {
@@ -665,33 +815,40 @@ __global__ void __launch_bounds__(kMaxThreads, kWmsMinBlocks)
             }
             __syncthreads();
             const uint4* st = a.states + (static_cast<size_t>(t) * a.n_cw + (act ? cw : 0)) * rows * z;
-            // state of row r-2 requested while row r runs, with its suffix
-            // loss seed in the degree-10 kernels (at degree 19 the extra
-            // registers of the seed ring cost more in spills than it saves)
-            auto fetch = [&](int r, float& sd) -> uint4 {
-                sd = 0.0f;
-                if (!act || r < 0) return make_uint4(0u, 0u, 31u << 5, 0u);
-                if (MAXD <= 10 && tab.row_sfx[r])
-                    sd = __ldcs(seed_t + edge_at(tab.edge[tab.row_ptr[r + 1] - 1], s, z));
-                return __ldcg(st + r * z + s);
+            // a row's state, its dloss/dR of every edge and the suffix edge's
+            // loss seed staged one row ahead (the state two rows ahead in
+            // registers instead: the compiler spills what it has just requested)
+            auto stage = [&](int r) {
+                if (act && r >= 0) {
+                    cp_async16(&staged_st[(r & 1) * blockDim.x], st + r * z + s);
+                    const uint32_t dst = ring + (r & 1) * (kUnrolled + 1) * h_step;
+                    const float* src = gh + static_cast<size_t>(tab.row_ptr[r]) * z + s;
+                    if (t < a.T - 1 && tab.row_deg[r] <= kUnrolled)
+                        for (int i = 0; i < tab.row_deg[r]; i++) cp_async4(dst + i * h_step, src + i * z);
+                    if (tab.row_sfx[r])
+                        cp_async4(dst + kUnrolled * h_step, seed_t + edge_at(tab.edge[tab.row_ptr[r + 1] - 1], s, z));
+                }
+                cp_async_commit();
             };
-            float d0, d1;
-            uint4 s0 = fetch(rows - 1, d0), s1 = fetch(rows - 2, d1);
+            stage(rows - 1);
             for (int r = rows - 1; r >= 0; r--) {
-                float d2;
-                const uint4 s2 = fetch(r - 2, d2);
-                bwd_layered_dispatch<MAXD>(tab.row_deg[r], tab, tab.row_ptr[r], s, act, g, wcur, gw_acc, s0,
-                                           gh + static_cast<size_t>(tab.row_ptr[r]) * z + s, t < a.T - 1, t > 0,
-                                           tab.row_sfx[r] != 0, d0, seed_t);
-                s0 = s1;
-                s1 = s2;
-                d0 = d1;
-                d1 = d2;
+                stage(r - 1);
+                cp_async_wait<1>();  // this thread's copies of row r have landed
+                const uint32_t h_row = ring + (r & 1) * (kUnrolled + 1) * h_step;
+                const float sd = tab.row_sfx[r] ? lds(h_row + kUnrolled * h_step) : 0.0f;
+                bwd_layered_dispatch<MAXD>(tab.row_deg[r], 4u * s, 4u * z, act, smem_u32(g), edges + tab.row_ptr[r],
+                                           gw_acc + tab.row_ptr[r], staged_st[(r & 1) * blockDim.x], h_row, h_step,
+                                           gh + static_cast<size_t>(tab.row_ptr[r]) * z + s, act && t < a.T - 1, t > 0,
+                                           tab.row_sfx[r] != 0, sd);
                 if (r > 0 && tab.sync_after[r - 1]) __syncthreads();
             }
+            cp_async_wait<0>();
             __syncthreads();
-            for (int e = tid; e < E; e += blockDim.x)
-                if (gw_acc[e] != 0.0f) atomicAdd(&a.grad[t * E + e], static_cast<double>(gw_acc[e]));
+            for (int e = tid; e < E; e += blockDim.x) {
+                float sum = 0.0f;
+                for (int w = 0; w < warps; w++) sum += gw_all[w * E + e];
+                if (sum != 0.0f) atomicAdd(&a.grad[t * E + e], static_cast<double>(sum));
+            }
             __syncthreads();
         }
     }
@@ -721,11 +878,15 @@ int max_row_degree(const CodeTable& tab) {
 }  // namespace
 
 // Shared memory: header, weight rows (the forward's padded layout, larger than
-// the adjoints' two [E] arrays), two core-column buffers per codeword, and
-// for codes of row degree <= 10 the flooding adjoint's row ring.
-size_t wms_smem_bytes(const CodeTable& tab, int cpb) {
-    return kHdr + kFwdWeightFloats * sizeof(float) + 2 * static_cast<size_t>(cpb) * tab.core_floats * sizeof(float) +
-           (max_row_degree(tab) <= 10 ? kRingBytes : 0);
+// the adjoints' edge words and gradient sums), then two core-column buffers per
+// codeword (and for codes of row degree <= 10 the flooding adjoint's row ring),
+// or one, the layered adjoint's two staged rows and its warps' gradient sums.
+size_t wms_smem_bytes(const CodeTable& tab, int cpb, bool layered) {
+    const size_t buf = static_cast<size_t>(cpb) * tab.core_floats * sizeof(float);
+    const size_t head = kHdr + kFwdWeightFloats * sizeof(float);
+    if (!layered) return head + 2 * buf + (max_row_degree(tab) <= 10 ? kRingBytes : 0);
+    return head + buf + 2 * (sizeof(uint4) + (kUnrolled + 1) * sizeof(float)) * kMaxThreads +
+           kMaxThreads / 32 * sizeof(float) * tab.n_edges;
 }
 
 namespace {
@@ -745,22 +906,26 @@ const void* wms_kernel_for(const CodeTable& tab, int k) {
 }
 }  // namespace
 
-cudaError_t wms_kernel_attributes(size_t smem) {
-    for (int k = 0; k < 4; k++)
-        for (const void* f : {wms_kernel<10>(k), wms_kernel<19>(k)}) {
-            cudaError_t e =
-                cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-            if (e != cudaSuccess) return e;
-        }
+cudaError_t wms_kernel_attributes(const CodeTable& tab, int cpb) {
+    for (int k = 0; k < 4; k++) {
+        const int smem = static_cast<int>(wms_smem_bytes(tab, cpb, (k & 1) != 0));
+        const void* f = wms_kernel_for(tab, k);
+        // handles of other sizes share the kernel: never below what they need
+        cudaFuncAttributes now;
+        cudaError_t e = cudaFuncGetAttributes(&now, f);
+        if (e == cudaSuccess && now.maxDynamicSharedSizeBytes < smem)
+            e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+    }
     return cudaSuccess;
 }
 
-int wms_ctas_per_sm(const CodeTable& tab, int threads, size_t smem) {
+int wms_ctas_per_sm(const CodeTable& tab, int cpb, int threads) {
     int n = 1 << 30;
     for (int k = 0; k < 4; k++) {
         int c = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, wms_kernel_for(tab, k), threads, smem) !=
-            cudaSuccess)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, wms_kernel_for(tab, k), threads,
+                                                          wms_smem_bytes(tab, cpb, (k & 1) != 0)) != cudaSuccess)
             return 0;
         n = c < n ? c : n;
     }
@@ -770,7 +935,7 @@ int wms_ctas_per_sm(const CodeTable& tab, int threads, size_t smem) {
 cudaError_t launch_wms(bool backward, bool layered, const CodeTable& tab, const float* llr, const uint8_t* cw,
                        const float* weights, uint4* states, float* gseed, uint4* gq, float* gh, double* loss,
                        double* grad, float* app, int* counters, int n_cw, int T, int cpb, int grid,
-                       int threads, size_t smem, float scale, cudaStream_t stream) {
+                       int threads, float scale, cudaStream_t stream) {
     WmsArgs a{};
     a.llr = llr;
     a.cw = cw;
@@ -792,7 +957,7 @@ cudaError_t launch_wms(bool backward, bool layered, const CodeTable& tab, const 
     grid = grid < a.n_groups ? grid : a.n_groups;
     const void* k = wms_kernel_for(tab, (backward ? 2 : 0) + (layered ? 1 : 0));
     void* params[2] = {const_cast<CodeTable*>(&tab), &a};
-    return cudaLaunchKernel(k, dim3(grid), dim3(threads), params, smem, stream);
+    return cudaLaunchKernel(k, dim3(grid), dim3(threads), params, wms_smem_bytes(tab, cpb, layered), stream);
 }
 
 cudaError_t launch_adam(int n, float* w, const double* grad, float* m, float* v, int step, float lr,

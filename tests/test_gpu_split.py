@@ -49,14 +49,17 @@ def test_batch_sizes_at_the_cluster_edges(bg, z, es):
     dec.close()
 
 
+@pytest.mark.parametrize("weighted", [False, True])
 @pytest.mark.parametrize("bg,z,n", [(1, 384, 620), (2, 40, 3000), (1, 96, 1300)])
-def test_same_bits_as_in_a_full_batch(bg, z, n):
+def test_same_bits_as_in_a_full_batch(bg, z, n, weighted):
     dec = Decoder(bg=bg, z=z, max_batch=n)
+    if weighted:
+        dec.set_weights(np.random.default_rng(z).uniform(0.6, 0.95, (5, dec.n_edges)))
     sig = torch.full((n,), codes.noise_sigma(1.9, 1 / 3 if bg == 1 else 1 / 5), device="cuda")
     llr, _ = dec.gen_llr(seed=9, cw_base=0, sigma=sig)
-    big = dec.decode(llr, 8, early_stop=True, want_app=True, want_iters=True)
+    big = dec.decode(llr, 8, early_stop=True, want_app=True, want_iters=True, weighted=weighted)
     for lo, k in ((0, 1), (3, 5), (40, 12), (100, 30), (200, 44), (300, 150)):
-        small = dec.decode(llr[lo:lo + k], 8, early_stop=True, want_app=True, want_iters=True)
+        small = dec.decode(llr[lo:lo + k], 8, early_stop=True, want_app=True, want_iters=True, weighted=weighted)
         for a, b in zip(small, big):
             assert torch.equal(a, b[lo:lo + k])
     dec.close()
