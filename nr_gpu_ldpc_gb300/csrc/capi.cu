@@ -326,6 +326,7 @@ int decode_impl(Handle* h, const float* llr, uint8_t* packed, int n_cw, int n_it
     const int plan = (h->schedule == NRLDPC_SCHEDULE_FLOODING && extra_tx == 0) ? split_choice(h, n_cw) : -1;
     if (plan >= 0) {
         SplitArgs a{};
+        a.head = h->split[plan];
         a.plan = reinterpret_cast<const unsigned char*>(h->scratch) + h->split_at[plan];
         a.llr = llr;
         a.packed = packed;

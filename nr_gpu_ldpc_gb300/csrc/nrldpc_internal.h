@@ -126,14 +126,14 @@ constexpr int kSplitMaxRanks = 16;   // CTAs per cluster
 constexpr int kSplitMaxPhases = 8;   // row ranges of an iteration
 constexpr int kSplitMaxWarps = 24;   // per CTA
 constexpr size_t kSplitHeader = 128;
-constexpr int kSplitKeepTo = 10;     // longest row whose dt addresses stay in registers
+constexpr int kSplitKeep = 10;       // longest row whose Q and dt addresses stay in registers
 constexpr int kSplitVnAhead = 8;     // dt requested before the first add
 constexpr int kSplitRowCost = 4;     // a row's fixed work, in edges
 constexpr int kSplitColCost = 6;     // a column's fixed work, in edges
 struct alignas(16) SplitHead {
     int z, n_bp, packed_bytes, n_core, core_floats, ranks, phases, warps, n_edges;
     int load;  // edges (and fixed work) of the busiest rank's tasks, per warp of sub-rows
-    // image: edges {offset, wrap threshold, owner << 24 | dt place} of the
+    // image: edges {column, 4V, owner << 24 | dt place} of the
     // rank's rows; rows {first edge | edge in the code << 16, state, suffix
     // column << 9 | shift, degree | suffix << 8}; columns {offset, ranks that
     // read it}; their dt {first | count << 16} per phase; every column's
@@ -146,6 +146,7 @@ struct SplitJob {            // one codeword of a mixed batch
     int32_t plan, job;       // byte offset of its code's plan; iteration-count index
 };
 struct SplitArgs {
+    SplitHead head;          // of the plan (without jobs)
     const unsigned char* plan;
     const SplitJob* jobs;    // null: n_cw codewords of one code, back to back
     const float* llr;

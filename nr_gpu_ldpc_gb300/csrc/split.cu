@@ -73,6 +73,13 @@ __device__ __forceinline__ void stc(uint32_t a, float v) {
 __device__ __forceinline__ void stc_u32(uint32_t a, uint32_t v) {
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
+// This thread's asynchronous copy of 16 bytes from global to shared memory.
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() {  // this thread's copies have landed
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
 __device__ __forceinline__ void stc_v4(uint32_t a, float4 v) {
     asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
                  : "memory");
@@ -98,18 +105,27 @@ __device__ __forceinline__ float max_nan(float a, float b) {
     return r;
 }
 
+__device__ __forceinline__ float min3(float a, float b, float c) {  // NaN operands ignored
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
 // One lifted row: the arithmetic of decode.cu's row_update (flooding), with
 // dt of each core edge sent to its column's owner instead of added here.
-//   edge: the row's first {offset, wrap threshold, distance from a posterior
-//   to its edge's dt at the owner}; s4: shared address of the posteriors plus
-//   4*s; par: hard-decision parity of the posteriors read (bit 0).
+//   edge: the row's first {column, 4V, distance from a posterior to its edge's
+//   dt at the owner}; l: shared address of the posteriors; s4: 4*s; st: the
+//   row's state, st_out: where it goes; par: hard-decision parity of the
+//   posteriors read (bit 0).
+// Rows of up to kSplitKeep edges keep Q and the dt addresses in registers (the
+// argmin is then found in the second half and the minima are taken in pairs,
+// as in row_update); longer rows track the argmin and form the address again.
 template <int D, bool WEIGHTED, bool ONE>
-__device__ __forceinline__ void cn_row(const uint4* edge, bool sfx, uint32_t s, uint32_t s4, uint32_t z4, uint4* state,
-                                       const float* wprev, const float* wcur, float alpha, bool check, uint32_t& par,
-                                       float& sfx_old) {
+__device__ __forceinline__ void cn_row(const uint4* edge, bool sfx, uint32_t s4, uint32_t l, uint32_t z4, uint4 st,
+                                       uint4* st_out, const float* wprev, const float* wcur, float alpha, bool check,
+                                       uint32_t& par) {
     constexpr int LAST = D - 1;
-    constexpr bool kAgain = D > kSplitKeepTo;  // long rows: too many registers to keep the addresses
-    const uint4 st = *state;
+    constexpr bool kKeep = D <= kSplitKeep;
     uint32_t to[D];
     float lv[D];
 #pragma unroll
@@ -119,10 +135,9 @@ __device__ __forceinline__ void cn_row(const uint4* edge, bool sfx, uint32_t s, 
             lv[i] = __uint_as_float(st.w);
         } else {
             const uint4 ea = edge[i];
-            uint32_t a = s4 + ea.x;
-            if (s >= ea.y) a -= z4;
+            const uint32_t t = s4 + ea.y, a = __viaddmin_u32(t, 0u - z4, t) + ea.x + l;
             lv[i] = lds(a);
-            if (!kAgain) to[i] = a + ea.z;
+            if (kKeep) to[i] = a + ea.z;
         }
     }
     if (check) {
@@ -137,8 +152,8 @@ __device__ __forceinline__ void cn_row(const uint4* edge, bool sfx, uint32_t s, 
         oa1 = __fmul_rn(alpha, om1);
         oa2 = __fmul_rn(alpha, om2);
     }
-    float keep[D];
-    float m1 = 1000.0f, m2 = 1000.0f;
+    float keep[D], qk[D];
+    float m1 = 1000.0f, m2 = 1000.0f, first = 0.0f;
     int idx = 0;
     uint32_t qmask = 0;
 #pragma unroll
@@ -151,12 +166,23 @@ __device__ __forceinline__ void cn_row(const uint4* edge, bool sfx, uint32_t s, 
         const float ro = __uint_as_float(__float_as_uint(mag) ^ ((oinfo << (24 - D + i)) & 0x80000000u));
         const float q = __fsub_rn(lv[i], ro);
         keep[i] = ro;
+        if (kKeep) qk[i] = q;
         const float qa = fabsf(q);
         qmask = __funnelshift_l(__float_as_uint(__fadd_rn(q, 0.0f)), qmask, 1);  // edge i at bit D-1-i, -0 as +0
-        if (qa < m1) idx = i;
-        const float mx = max_nan(m1, qa);  // NaN |Q| leaves min1/min2 untouched
-        m1 = fminf(m1, qa);
-        m2 = fminf(m2, mx);
+        if (i == 0) {
+            m1 = fminf(m1, qa);
+        } else if (kKeep && (i & 1) && i + 1 < D) {
+            first = qa;  // of a pair
+        } else if (kKeep && !(i & 1)) {
+            const float lo = fminf(first, qa), hi = max_nan(first, qa);
+            m2 = min3(m2, hi, max_nan(m1, lo));
+            m1 = fminf(m1, lo);
+        } else {
+            if (!kKeep && qa < m1) idx = i;
+            const float mx = max_nan(m1, qa);  // NaN |Q| leaves min1/min2 untouched
+            m1 = fminf(m1, qa);
+            m2 = fminf(m2, mx);
+        }
     }
     const uint32_t rsign = qmask ^ (0u - static_cast<uint32_t>(__popc(qmask) & 1));
     float a1 = 0.0f, a2 = 0.0f;
@@ -167,21 +193,23 @@ __device__ __forceinline__ void cn_row(const uint4* edge, bool sfx, uint32_t s, 
     float sfx_new = 0.0f;
 #pragma unroll
     for (int i = 0; i < D; i++) {
+        const bool at_min = kKeep ? fabsf(qk[i]) == m1 : i == idx;
+        if (kKeep && at_min) idx = i;
         float mag;
         if (WEIGHTED)
-            mag = __fmul_rn(wcur[i], i == idx ? m2 : m1);
+            mag = __fmul_rn(wcur[i], at_min ? m2 : m1);
         else
-            mag = i == idx ? a2 : a1;
+            mag = at_min ? a2 : a1;
         const float rn = __uint_as_float(__float_as_uint(mag) ^ ((rsign << (32 - D + i)) & 0x80000000u));
         const float d = __fsub_rn(rn, keep[i]);
         if (i == LAST && sfx) {
             sfx_new = __fadd_rn(__uint_as_float(st.w), d);
         } else {
             uint32_t a = to[i];
-            if (kAgain) {
+            if (!kKeep) {
                 const uint4 ea = edge[i];
-                a = s4 + ea.x + ea.z;
-                if (s >= ea.y) a -= z4;
+                const uint32_t t = s4 + ea.y;
+                a = __viaddmin_u32(t, 0u - z4, t) + ea.x + l + ea.z;
             }
             if (ONE)
                 sts(a, d);
@@ -189,10 +217,9 @@ __device__ __forceinline__ void cn_row(const uint4* edge, bool sfx, uint32_t s, 
                 stc(a, d);
         }
     }
-    sfx_old = __uint_as_float(st.w);
     uint32_t info = static_cast<uint32_t>(idx) | ((rsign & ((1u << D) - 1u)) << 8);
-    if (!(sfx_old > 0.0f)) info |= kHdBit;
-    *state = make_uint4(__float_as_uint(m1), __float_as_uint(m2), info, __float_as_uint(sfx_new));
+    if (!(__uint_as_float(st.w) > 0.0f)) info |= kHdBit;
+    *st_out = make_uint4(__float_as_uint(m1), __float_as_uint(m2), info, __float_as_uint(sfx_new));
 }
 
 // Position of a suffix row's last column at sub-row s (rw.z: first position
@@ -249,14 +276,16 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
             llr += j.llr_offset;
             packed += j.out_offset;
         }
-        sync();  // every CTA runs, and is done with the previous codeword
-        if (plan != loaded) {
-            if (tid < static_cast<int>(sizeof(SplitHead) / 4))
-                reinterpret_cast<int*>(s_head)[tid] = reinterpret_cast<const int*>(plan)[tid];
-            const int bytes = reinterpret_cast<const SplitHead*>(plan)->image_bytes;
-            const uint4* src = reinterpret_cast<const uint4*>(plan + sizeof(SplitHead) + static_cast<size_t>(rank) * bytes);
-            for (int k = tid; k < bytes / 16; k += nt) reinterpret_cast<uint4*>(image)[k] = src[k];
+        if (plan != loaded) {  // head and this rank's tables
+            if (a.jobs) {
+                if (tid < static_cast<int>(sizeof(SplitHead) / 4))
+                    reinterpret_cast<int*>(s_head)[tid] = reinterpret_cast<const int*>(plan)[tid];
+            } else if (tid == 0) {
+                *s_head = a.head;
+            }
             __syncthreads();
+            const unsigned char* src = plan + sizeof(SplitHead) + static_cast<size_t>(rank) * h.image_bytes;
+            for (int k = tid; k < h.image_bytes / 16; k += nt) cp_async16(smem_u32(image) + 16u * k, src + 16 * k);
         }
         const int z = h.z, P = h.phases, lists = h.warps;  // warps with task lists (a mixed batch's CTA may have more)
         const uint32_t z4 = 4u * static_cast<uint32_t>(z);
@@ -266,38 +295,26 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
         }
         const uint32_t l_addr = smem_u32(smem) + h.off_l, dt_addr = smem_u32(smem) + h.off_dt;
         float* app = a.app ? a.app + static_cast<size_t>(cw) * h.n_bp : nullptr;
-        {   // core LLRs: the whole copy by each CTA, or (host memory) its share, sent to all
-            const int total = h.core_floats / 4;
-            const int per = a.llr_from_host ? (total + C - 1) / C : total;
-            const int lo = a.llr_from_host ? rank * per : 0, hi = min(total, lo + per);
-            for (int m = lo + tid; m < hi; m += nt) {
+        // core LLRs: the whole copy by each CTA, or (host memory) its share, sent to all
+        if (ONE || !a.llr_from_host) {
+            for (int m = tid; m < h.core_floats / 4; m += nt) cp_async16(l_addr + 16u * m, llr + 4 * m);
+        } else {
+            const int total = h.core_floats / 4, per = (total + C - 1) / C;
+            sync();  // every CTA runs
+            for (int m = rank * per + tid; m < min(total, (rank + 1) * per); m += nt) {
                 const float4 v = __ldcs(reinterpret_cast<const float4*>(llr) + m);
-                if (!ONE && a.llr_from_host)
-                    for (int q = 0; q < C; q++) stc_v4(mapa(l_addr + 16u * m, q), v);
-                else
-                    reinterpret_cast<float4*>(smem + h.off_l)[m] = v;
+                for (int q = 0; q < C; q++) stc_v4(mapa(l_addr + 16u * m, q), v);
             }
         }
+        cp_async_wait_all();
         if (plan != loaded) {  // dt place at the owner -> distance from the posterior to it
+            __syncthreads();
             uint4* edge = reinterpret_cast<uint4*>(image + h.o_edge);
             for (int k = tid; k < h.n_edges; k += nt) {
-                const uint32_t to = edge[k].z, block = edge[k].x - 4u * (static_cast<uint32_t>(z) - edge[k].y);
-                const uint32_t base = ONE ? dt_addr : mapa(dt_addr, to >> 24);
-                edge[k].z = base + (to & 0xffffffu) * z4 - (l_addr + block);
+                const uint32_t to = edge[k].z, base = ONE ? dt_addr : mapa(dt_addr, to >> 24);
+                edge[k].z = base + (to & 0xffffffu) * z4 - (l_addr + edge[k].x);
             }
             loaded = plan;
-        }
-        {   // zero states with the suffix LLRs: R_old = +0 in the first iteration
-            const uint16_t* cn = reinterpret_cast<const uint16_t*>(image + h.o_cn);
-            const int n_cn = reinterpret_cast<const uint16_t*>(image + h.o_cnptr)[P * lists];
-            for (int k = warp; k < n_cn; k += W) {
-                const uint4 rw = reinterpret_cast<const uint4*>(image + h.o_row)[cn[k] >> 4];
-                const uint32_t s = static_cast<uint32_t>((cn[k] & 15) * 32 + lane);
-                if (s >= static_cast<uint32_t>(z)) continue;
-                float w = 0.0f;
-                if (rw.w >> 8) w = __ldcs(llr + sfx_pos(rw, s, z));
-                reinterpret_cast<uint4*>(smem + h.off_state)[rw.y + s] = make_uint4(0u, 0u, 0u, __float_as_uint(w));
-            }
         }
         sync();
         int it = a.n_iter;
@@ -322,14 +339,20 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
                     uint32_t bad = 0;
                     if (s < static_cast<uint32_t>(z)) {
                         const bool sfx = (rw.w >> 8) != 0;
-                        float sfx_old = 0.0f;
+                        uint4* state = states + rw.y + s;
+                        // first iteration: zero state (R_old = +0), the suffix LLR
+                        uint4 st = make_uint4(0u, 0u, 0u, 0u);
+                        if (t > 0)
+                            st = *state;
+                        else if (sfx)
+                            st.w = __float_as_uint(__ldcs(llr + sfx_pos(rw, s, z)));
                         const uint4* edge = reinterpret_cast<const uint4*>(image + h.o_edge) + (rw.x & 0xffffu);
                         const uint32_t we = WEIGHTED ? rw.x >> 16 : 0u;
                         switch (rw.w & 255u) {
 #define NRLDPC_CN_CASE(D)                                                                                             \
     case D:                                                                                                           \
-        cn_row<D, WEIGHTED, ONE>(edge, sfx, s, l_addr + 4u * s, z4, states + rw.y + s, WEIGHTED ? wprev + we : nullptr, \
-                                 WEIGHTED ? wcur + we : nullptr, a.alpha, check, bad, sfx_old);                       \
+        cn_row<D, WEIGHTED, ONE>(edge, sfx, 4u * s, l_addr, z4, st, state, WEIGHTED ? wprev + we : nullptr,           \
+                                 WEIGHTED ? wcur + we : nullptr, a.alpha, check, bad);                                \
         break;
                             NRLDPC_CN_CASE(1) NRLDPC_CN_CASE(2) NRLDPC_CN_CASE(3) NRLDPC_CN_CASE(4)
                             NRLDPC_CN_CASE(5) NRLDPC_CN_CASE(6) NRLDPC_CN_CASE(7) NRLDPC_CN_CASE(8)
@@ -341,7 +364,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
                                 break;
                         }
                         // the posterior the codeword leaves with if it stops here
-                        if (check && app && sfx) app[sfx_pos(rw, s, z)] = sfx_old;
+                        if (check && app && sfx) app[sfx_pos(rw, s, z)] = __uint_as_float(st.w);
                     }
                     if (check && __any_sync(0xffffffffu, bad & 1u) && lane < C) {
                         const uint32_t f = smem_u32(&s_fail[t & 1]);
@@ -426,8 +449,8 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
             }
         }
         if (a.iters && rank == 0 && tid == 0) a.iters[cw] = it;
+        sync();  // no CTA reuses its shared memory, or leaves, while another reads it
     }
-    sync();  // no CTA leaves while another reads its shared memory
 }
 
 // Lists of task[i] (cost[i], largest first) for n_bins warps, each task to
@@ -599,7 +622,7 @@ bool make_split_plan(const CodeTable& t, int ranks, size_t smem_limit, SplitHead
                                     t.row_deg[r] | (t.row_sfx[r] ? 256u : 0u));
                 for (int e = t.row_ptr[r]; e <= last; e++, m++) {
                     const int c = t.edge_col[e];
-                    edge[m] = make_uint4(t.eaddr[e].x + t.eaddr[e].y, t.ethr[e], 0u, 0u);
+                    edge[m] = make_uint4(t.eaddr[e].x, t.eaddr[e].y, 0u, 0u);
                     if (c < nc) edge[m].z = (static_cast<uint32_t>(col_rank[c]) << 24) | static_cast<uint32_t>(dt_of[e]);
                 }
             }
