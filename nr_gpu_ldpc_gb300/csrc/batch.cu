@@ -380,6 +380,7 @@ int choose_split(Batch* b, const std::vector<int32_t>& order, const std::vector<
             }
             fits = p.state > 0;
             launch.warps = std::max(launch.warps, p.head.warps);
+            launch.phases = std::max(launch.phases, p.head.phases);
             launch.smem = std::max(launch.smem, p.head.smem);
         }
         if (!fits) continue;
@@ -679,6 +680,7 @@ int nrldpc_batch_decode(nrldpc_batch* batch, const float* d_llr, uint8_t* d_pack
         a.llr = d_llr;
         a.packed = d_packed;
         a.iters = d_iters;
+        a.error_flag = b->d_scratch + 1;
         a.n_cw = b->n_jobs;
         a.n_iter = n_iter;
         a.early_stop = early_stop;

@@ -194,12 +194,12 @@ int split_prepare(Handle* h, size_t smem_limit, std::vector<unsigned char>* byte
 }
 
 // Plan for n codewords, or -1 for decode_kernel: the smaller of two time
-// estimates (split_cost, fused_row_walk).  Fitted to GB300 times, 10
-// iterations, us (model): BG1 Z=384 on 16 / 8 / 4 / 3 CTAs 52 / 68 / 103 / 151
-// (47 / 64 / 98 / 150), BG2 Z=384 40 / 48 / 72 / 89, BG1 Z=96 on 4 / 2 / 1
-// CTAs 42 / 59 / 81 (47 / 64 / 98); decode_kernel BG1 Z=384 / 208 / 96 at one
-// CTA per SM 300 / 245 / 204 (300 / 248 / 207), BG2 Z=384 / 128 219 / 157, two
-// CTAs per SM 1.5-1.65 times that.
+// estimates (split_cost, fused_row_walk).  GB300 times, 10 iterations without
+// early stop, us (model): BG1 Z=384 on 16 / 10 / 4 / 3 CTAs 43 / 52 / 95 / 148
+// (47 / 57 / 98 / 150), BG2 Z=384 on 16 / 4 / 3 40 / 72 / 89 (42 / 80 / 96),
+// BG1 Z=96 on 4 / 2 / 1 CTAs 42 / 59 / 80 (47 / 64 / 98); decode_kernel at one
+// CTA per SM BG1 Z=384 / 208 / 96 299 / 245 / 204 (300 / 248 / 207), BG2 Z=384 /
+// 128 219 / 157, two CTAs per SM 1.5-1.65 times that.
 long fused_cost(const Handle* h, int n) {
     const long groups = (n + h->cpb - 1) / h->cpb, one = fused_row_walk(h->tab, h->threads / 32);
     long cost = groups / h->max_grid * (one * (4 + 2 * h->ctas_per_sm) / 5);
@@ -332,6 +332,7 @@ int decode_impl(Handle* h, const float* llr, uint8_t* packed, int n_cw, int n_it
         a.packed = packed;
         a.app = app;
         a.iters = iters;
+        a.error_flag = h->scratch + 1;
         a.n_cw = n_cw;
         a.n_iter = n_iter;
         a.n_w_iters = h->n_w_iters;

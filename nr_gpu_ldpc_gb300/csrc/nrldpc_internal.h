@@ -79,7 +79,7 @@ struct DecodeArgs {
     uint32_t extra_tx;
 };
 
-enum DeviceError : int { kErrNone = 0, kErrLlrLoadTimeout = 1 };
+enum DeviceError : int { kErrNone = 0, kErrLlrLoadTimeout = 1, kErrSplitTimeout = 2 };
 
 // Mixed-code batches (batch.cu): a work item is up to `count` codewords of
 // one code, listed at order[start .. start+count).
@@ -125,7 +125,7 @@ const void* batch_decode_kernel_ptr();
 constexpr int kSplitMaxRanks = 16;   // CTAs per cluster
 constexpr int kSplitMaxPhases = 8;   // row ranges of an iteration
 constexpr int kSplitMaxWarps = 24;   // per CTA
-constexpr size_t kSplitHeader = 128;
+constexpr size_t kSplitHeader = 144;  // mbarriers, failure flags, head
 constexpr int kSplitKeep = 10;       // longest row whose Q and dt addresses stay in registers
 constexpr int kSplitVnAhead = 8;     // dt requested before the first add
 constexpr int kSplitRowCost = 4;     // a row's fixed work, in edges
@@ -137,8 +137,9 @@ struct alignas(16) SplitHead {
     // rank's rows; rows {first edge | edge in the code << 16, state, suffix
     // column << 9 | shift, degree | suffix << 8}; columns {offset, ranks that
     // read it}; their dt {first | count << 16} per phase; every column's
-    // owner; task lists per (phase,) warp
-    int o_edge, o_row, o_col, o_beg, o_own, o_cnptr, o_cn, o_vnptr, o_vn, image_bytes;
+    // owner; task lists per (phase,) warp; bytes of dt and of posteriors that
+    // reach the rank per iteration
+    int o_edge, o_row, o_col, o_beg, o_own, o_cnptr, o_cn, o_vnptr, o_vn, o_bytes, image_bytes;
     int off_l, off_state, off_dt, off_acc, smem;  // shared memory
 };
 struct SplitJob {            // one codeword of a mixed batch
@@ -153,9 +154,11 @@ struct SplitArgs {
     uint8_t* packed;
     float* app;
     int32_t* iters;
+    int* error_flag;         // bounded-wait failures
     int n_cw, n_iter, n_w_iters, early_stop, llr_from_host;
     float alpha;
 };
+static_assert(kSplitHeader >= 32 + sizeof(SplitHead) && kSplitHeader % 16 == 0, "flags, then the head");
 // Cluster sizes tried: each holds more codewords at once than the one before
 // (GB300 at one CTA per SM: 7, 13, 23, 28, 36, 46, 76 and 152 clusters; a
 // GPC's SMs do not divide evenly by the other sizes).

@@ -43,6 +43,21 @@ namespace nrldpc {
 namespace {
 
 constexpr int kSplitThreads = kSplitMaxWarps * 32;
+// How a pass hands over to the next: kOne, a cluster of one CTA (small codes):
+// CTA barriers.  kCounted (one phase, no early stop): every CTA knows how many
+// bytes of dt, and of posteriors, will reach it, the stores count them on its
+// mbarriers, and it goes on when they are there.  kBarriers: cluster barriers,
+// which early stop needs for its failures (sent and counted beside the dt they
+// made BG2 Z=40 16 codewords 7% slower, 20.7 -> 22.2 us).  A cluster barrier
+// takes 400-650 clocks of which 300-500 are the fence, more with stores on the
+// way; counting instead, 10 iterations: BG1 Z=384 49.4 -> 42.8 us on 16 CTAs,
+// 57.6 -> 52.0 on 10, 100.6 -> 94.6 on 4, BG2 Z=208 60 codewords 74.1 -> 65.7.
+// No count can run into the next phase's: a CTA sends a column's dt only after
+// it has that column's posteriors, which the owner sends after its dt are
+// complete, and those include dt that their readers sent after the posteriors
+// before were complete; a thread opens each phase after all have seen the last.
+enum Mode { kOne, kCounted, kBarriers };
+
 constexpr uint32_t kHdBit = 0x80000000u;  // state info: hard decision of the suffix posterior read
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -84,6 +99,33 @@ __device__ __forceinline__ void stc_v4(uint32_t a, float4 v) {
     asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
                  : "memory");
 }
+// Remote store that counts its bytes on an mbarrier of the CTA it writes to.
+__device__ __forceinline__ void st_async(uint32_t a, uint32_t v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(a), "r"(v), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void mbar_init(uint32_t bar) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+}
+// Opens a phase that ends when `bytes` have arrived.
+__device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// Bounded wait for the phase of this parity; false when the limit ran out.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+    for (int i = 0; i < (1 << 16); i++) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
 // Barrier over every thread of the cluster; shared-memory writes before it
 // (local and remote) are seen after it.
 __device__ __forceinline__ void cluster_sync() {
@@ -120,7 +162,7 @@ __device__ __forceinline__ float min3(float a, float b, float c) {  // NaN opera
 // Rows of up to kSplitKeep edges keep Q and the dt addresses in registers (the
 // argmin is then found in the second half and the minima are taken in pairs,
 // as in row_update); longer rows track the argmin and form the address again.
-template <int D, bool WEIGHTED, bool ONE>
+template <int D, bool WEIGHTED, int MODE>
 __device__ __forceinline__ void cn_row(const uint4* edge, bool sfx, uint32_t s4, uint32_t l, uint32_t z4, uint4 st,
                                        uint4* st_out, const float* wprev, const float* wcur, float alpha, bool check,
                                        uint32_t& par) {
@@ -211,8 +253,10 @@ __device__ __forceinline__ void cn_row(const uint4* edge, bool sfx, uint32_t s4,
                 const uint32_t t = s4 + ea.y;
                 a = __viaddmin_u32(t, 0u - z4, t) + ea.x + l + ea.z;
             }
-            if (ONE)
+            if (MODE == kOne)
                 sts(a, d);
+            else if (MODE == kCounted)
+                st_async(a, __float_as_uint(d), edge[i].w);
             else
                 stc(a, d);
         }
@@ -240,13 +284,12 @@ struct SplitWeights<true> {
 };
 
 // Bound by SM issue in the check-node pass and, on large clusters, by the
-// distributed-shared-memory stores and the barriers (each waits for the stores
-// before it); 24 warps per CTA hide more of it than 16, and the 80 registers
-// that leaves hold a degree-19 row.  ONE: clusters of one CTA (small codes),
-// plain shared memory and CTA barriers.
-template <bool WEIGHTED, bool ONE>
+// distributed-shared-memory stores and the hand-overs; 24 warps per CTA hide
+// more of it than 16, and the 80 registers that leaves hold a degree-19 row.
+template <bool WEIGHTED, int MODE>
 __global__ void __launch_bounds__(kSplitThreads, 1)
     split_decode_kernel(const __grid_constant__ SplitArgs a, const __grid_constant__ typename SplitWeights<WEIGHTED>::type wt) {
+    constexpr bool ONE = MODE == kOne;
     extern __shared__ __align__(128) unsigned char smem[];
     const int rank = ONE ? 0 : static_cast<int>(cluster_rank()), C = ONE ? 1 : static_cast<int>(cluster_size());
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = blockDim.x, W = nt >> 5;
@@ -256,10 +299,25 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
         else
             cluster_sync();
     };
-    uint32_t* s_fail = reinterpret_cast<uint32_t*>(smem);  // [2] an unsatisfied row, by iteration parity
+    const uint32_t bar_dt = smem_u32(smem), bar_l = bar_dt + 8;  // mbarriers of the dt and the posteriors
+    uint32_t* s_fail = reinterpret_cast<uint32_t*>(smem + 16);   // [2] an unsatisfied row, by iteration parity
+    uint32_t ph_dt = 0, ph_l = 0;                                // parities waited for next
+    bool dead = false;  // a wait ran out: reported, and no further one
+    if (MODE == kCounted && tid == 0) {
+        mbar_init(bar_dt);
+        mbar_init(bar_l);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    auto wait = [&](uint32_t bar, uint32_t parity) {
+        if (!dead && !mbar_wait(bar, parity)) {
+            dead = true;
+            atomicExch(a.error_flag, kErrSplitTimeout);
+        }
+        __syncthreads();  // all threads have seen it before the next phase opens
+    };
     // the plan's head and this rank's tables; read where they are used, so
     // that the row bodies have the registers
-    SplitHead* s_head = reinterpret_cast<SplitHead*>(smem + 16);
+    SplitHead* s_head = reinterpret_cast<SplitHead*>(smem + 32);
     const volatile SplitHead& h = *s_head;
     unsigned char* image = smem + kSplitHeader;
     if (tid < 2) s_fail[tid] = 0;
@@ -313,6 +371,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
             for (int k = tid; k < h.n_edges; k += nt) {
                 const uint32_t to = edge[k].z, base = ONE ? dt_addr : mapa(dt_addr, to >> 24);
                 edge[k].z = base + (to & 0xffffffu) * z4 - (l_addr + edge[k].x);
+                if (MODE == kCounted) edge[k].w = mapa(bar_dt, to >> 24);
             }
             loaded = plan;
         }
@@ -320,14 +379,21 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
         int it = a.n_iter;
         bool conv = false;
         for (int t = 0; t < a.n_iter && !conv; t++) {
-            const bool check = a.early_stop && t > 0;
+            const bool check = MODE != kCounted && a.early_stop && t > 0;
             const float* wprev = nullptr;
             const float* wcur = nullptr;
             if constexpr (WEIGHTED) {
                 wprev = wt.w[t == 0 ? kMaxWIters : min(t - 1, a.n_w_iters - 1)];
                 wcur = wt.w[min(t, a.n_w_iters - 1)];
             }
-            for (int p = 0; p < P; p++) {
+            if (MODE == kCounted) {
+                if (t > 0) {
+                    wait(bar_l, ph_l);  // the posteriors of the last iteration
+                    ph_l ^= 1u;
+                }
+                if (tid == 0) mbar_expect(bar_dt, reinterpret_cast<const uint32_t*>(image + h.o_bytes)[0]);
+            }
+            for (int p = 0; p < (MODE == kCounted ? 1 : P); p++) {
                 const uint16_t* cnptr = reinterpret_cast<const uint16_t*>(image + h.o_cnptr) + p * lists + warp;
                 const uint16_t* cn = reinterpret_cast<const uint16_t*>(image + h.o_cn);
                 uint4* states = reinterpret_cast<uint4*>(smem + h.off_state);
@@ -351,7 +417,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
                         switch (rw.w & 255u) {
 #define NRLDPC_CN_CASE(D)                                                                                             \
     case D:                                                                                                           \
-        cn_row<D, WEIGHTED, ONE>(edge, sfx, 4u * s, l_addr, z4, st, state, WEIGHTED ? wprev + we : nullptr,           \
+        cn_row<D, WEIGHTED, MODE>(edge, sfx, 4u * s, l_addr, z4, st, state, WEIGHTED ? wprev + we : nullptr,           \
                                  WEIGHTED ? wcur + we : nullptr, a.alpha, check, bad);                                \
         break;
                             NRLDPC_CN_CASE(1) NRLDPC_CN_CASE(2) NRLDPC_CN_CASE(3) NRLDPC_CN_CASE(4)
@@ -374,12 +440,20 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
                             stc_u32(mapa(f, lane), 1u);
                     }
                 }
-                sync();  // the dt of this phase, and (last phase) the failures, are in place
+                // the dt of this phase, and (last phase) the failures, are in place
+                if (MODE == kCounted) {
+                    wait(bar_dt, ph_dt);
+                    ph_dt ^= 1u;
+                } else {
+                    sync();
+                }
                 if (check && p == P - 1 && s_fail[t & 1] == 0) {
                     conv = true;  // iteration t - 1 left a codeword: t iterations ran
                     it = t;
                     break;
                 }
+                if (MODE == kCounted && tid == 0)
+                    mbar_expect(bar_l, reinterpret_cast<const uint32_t*>(image + h.o_bytes)[1]);
                 const uint16_t* vnptr = reinterpret_cast<const uint16_t*>(image + h.o_vnptr) + warp;
                 const uint16_t* vn = reinterpret_cast<const uint16_t*>(image + h.o_vn);
                 const int v1 = warp < lists ? vnptr[1] : 0;
@@ -404,7 +478,12 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
                         for (int i = 0; i < kSplitVnAhead; i++)
                             if (i < m) v = __fadd_rn(v, x[i]);
                     }
-                    if (p < P - 1) {
+                    if (MODE == kCounted) {
+                        for (uint32_t m = cm.y; m; m &= m - 1) {
+                            const uint32_t q = __ffs(m) - 1;
+                            st_async(mapa(la, q), __float_as_uint(v), mapa(bar_l, q));
+                        }
+                    } else if (p < P - 1) {
                         *acc = v;
                     } else if (ONE) {
                         sts(la, v);
@@ -412,9 +491,16 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
                         for (uint32_t m = cm.y; m; m &= m - 1) stc(mapa(la, __ffs(m) - 1), v);
                     }
                 }
-                sync();  // posteriors (last phase) or dt buffers free for the next pass
+                if (MODE != kCounted) sync();  // posteriors (last phase) or dt buffers free for the next pass
                 if (tid == 0 && p == P - 1) s_fail[t & 1] = 0;  // written again two iterations on
             }
+        }
+        if (MODE == kCounted) {
+            if (!conv) {
+                wait(bar_l, ph_l);
+                ph_l ^= 1u;
+            }
+            sync();  // every CTA's posteriors and states are final
         }
         // Packed hard decisions (and posteriors): 32 positions per warp.
         const int n = h.n_bp, packed_bytes = h.packed_bytes, nc = h.n_core;
@@ -588,6 +674,7 @@ bool make_split_plan(const CodeTable& t, int ranks, size_t smem_limit, SplitHead
         h.o_cn = take(2 * n_cn);
         h.o_vnptr = take(2 * (static_cast<size_t>(W) + 1));
         h.o_vn = take(2 * n_cols * chunks);
+        h.o_bytes = take(8);
         h.image_bytes = static_cast<int>(at);
         auto up = [](size_t x) { return (x + 127) / 128 * 128; };
         const size_t l = up(kSplitHeader + at), st = up(l + 4 * static_cast<size_t>(t.core_floats)),
@@ -649,6 +736,17 @@ bool make_split_plan(const CodeTable& t, int ranks, size_t smem_limit, SplitHead
                 n += static_cast<int>(list[k][p].size());
             }
             spread(vl, W, 0, vnptr, vn);
+            // bytes that reach the rank in a one-phase iteration: dt of its
+            // columns, posteriors that its rows or its output read
+            auto* bytes = reinterpret_cast<uint32_t*>(im + h.o_bytes);
+            bytes[0] = 4u * static_cast<uint32_t>(t.z) * static_cast<uint32_t>(dt[k][0]);
+            uint32_t n_read = 0;
+            for (int c = 0; c < nc; c++) {
+                bool reads = col_rank[c] == k;
+                for (int j = 0; j < col_deg[c]; j++) reads |= row_rank[col_row[c][j]] == k;
+                n_read += reads;
+            }
+            bytes[1] = 4u * static_cast<uint32_t>(t.z) * n_read;
         }
         *head = h;
         return true;
@@ -657,12 +755,18 @@ bool make_split_plan(const CodeTable& t, int ranks, size_t smem_limit, SplitHead
 }
 
 namespace {
-const void* split_kernel(bool weighted, bool one) {
-    if (one)
-        return weighted ? reinterpret_cast<const void*>(&split_decode_kernel<true, true>)
-                        : reinterpret_cast<const void*>(&split_decode_kernel<false, true>);
-    return weighted ? reinterpret_cast<const void*>(&split_decode_kernel<true, false>)
-                    : reinterpret_cast<const void*>(&split_decode_kernel<false, false>);
+template <int MODE>
+const void* split_kernel_of(bool weighted) {
+    return weighted ? reinterpret_cast<const void*>(&split_decode_kernel<true, MODE>)
+                    : reinterpret_cast<const void*>(&split_decode_kernel<false, MODE>);
+}
+int mode_of(const SplitHead& h, int early_stop) {
+    return h.ranks == 1 ? kOne : h.phases == 1 && !early_stop ? kCounted : kBarriers;
+}
+const void* split_kernel(bool weighted, int mode) {
+    return mode == kOne       ? split_kernel_of<kOne>(weighted)
+           : mode == kCounted ? split_kernel_of<kCounted>(weighted)
+                              : split_kernel_of<kBarriers>(weighted);
 }
 void split_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, const SplitHead& h, int n_clusters,
                   cudaStream_t stream) {
@@ -679,8 +783,8 @@ void split_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, const Spli
 }  // namespace
 
 cudaError_t split_kernel_attributes(size_t smem) {
-    for (int w = 0; w < 4; w++) {
-        const void* k = split_kernel((w & 1) != 0, (w & 2) != 0);
+    for (int w = 0; w < 6; w++) {
+        const void* k = split_kernel((w & 1) != 0, w / 2);
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return e;
@@ -693,7 +797,7 @@ int split_max_clusters(const SplitHead& h) {
     cudaLaunchAttribute attr{};
     split_config(&cfg, &attr, h, 1, nullptr);
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, split_kernel(false, h.ranks == 1), &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&n, split_kernel(false, mode_of(h, 1)), &cfg) != cudaSuccess) {
         cudaGetLastError();  // clusters of this size are not available
         return 0;
     }
@@ -708,7 +812,7 @@ cudaError_t launch_split(const SplitHead& h, const SplitArgs& args, const Weight
     NoWeights none{};
     void* params[2] = {const_cast<SplitArgs*>(&args),
                        weights ? const_cast<WeightTable*>(weights) : static_cast<void*>(&none)};
-    return cudaLaunchKernelExC(&cfg, split_kernel(weights != nullptr, h.ranks == 1), params);
+    return cudaLaunchKernelExC(&cfg, split_kernel(weights != nullptr, mode_of(h, args.early_stop)), params);
 }
 
 }  // namespace nrldpc
