@@ -312,7 +312,7 @@ int max_cpb(const Batch* b, int id, int spt) {
     const int tpc = t.z / spt;
     const size_t room = b->smem_optin - kHeaderBytesBatch - kBatchTableBytes;
     int c = std::max(1, kMaxThreads / tpc);
-    while (c > 1 && group_smem_bytes(t, c) > room) c--;
+    while (c > 1 && group_smem_bytes(t, c, 0) > room) c--;
     return std::min(c, 48);
 }
 
@@ -593,7 +593,7 @@ int nrldpc_batch_set_jobs(nrldpc_batch* batch, const nrldpc_job* jobs, int n_job
             items.push_back(WorkItem{id, s, cnt, spt});
             threads = std::max(threads, (cnt * (t.z / spt) + 31) / 32 * 32);
             slot_words = std::max(slot_words, static_cast<size_t>(cnt) * 4 * t.rows * t.z);
-            bufs = std::max(bufs, group_smem_bytes(t, cnt));
+            bufs = std::max(bufs, group_smem_bytes(t, cnt, 0));
         }
         i = k;
     }

@@ -35,7 +35,8 @@ struct Handle {
     bool plan_ok = false;
     float alpha = 0.75f;
     int max_batch = 0;
-    int cpb = 1, threads = 32, ctas_per_sm = 1, sm_count = 1, max_grid = 1, minb = 1;
+    int cpb = 1, threads = 32, ctas_per_sm = 1, sm_count = 1, max_grid = 1;
+    DecodeKind kind = DecodeKind::kAny1;
     size_t smem = 0;
     // small batches: one codeword on a cluster of CTAs (split.cu), plans from
     // the largest cluster to the smallest
@@ -265,19 +266,18 @@ int init_impl(const int* base, int rows, int cols, int kb, const nrldpc_config* 
         delete h;
         return NRLDPC_ERR_BAD_CONFIG;
     }
+    const DecodeShape shape = decode_shape(h->tab, cpb, smem_limit, prop.sharedMemPerMultiprocessor);
     h->cpb = cpb;
-    h->threads = (cpb * z + 31) / 32 * 32;
-    h->smem = decode_smem_bytes(h->tab, cpb);
-    // two CTAs per SM when shared memory allows (the kernel then caps its
-    // registers for two); otherwise one CTA with the full register budget
-    h->minb = (2 * (h->smem + 1024) <= prop.sharedMemPerMultiprocessor) ? 2 : 1;
+    h->threads = shape.threads;
+    h->smem = shape.smem;
+    h->kind = shape.kind;
     // opt in to the device maximum, so handles of any size can coexist
-    if (map_cuda(decode_kernel_attributes(has_short_rows(h->tab), h->minb, smem_limit))) {
+    if (map_cuda(decode_kernel_attributes(h->kind, smem_limit))) {
         delete h;
         return NRLDPC_ERR_CUDA;
     }
-    h->ctas_per_sm = std::max(1, std::min(decode_max_ctas_per_sm(h->tab, false, h->minb, h->threads, h->smem),
-                                          decode_max_ctas_per_sm(h->tab, true, h->minb, h->threads, h->smem)));
+    h->ctas_per_sm = std::max(1, std::min(decode_max_ctas_per_sm(h->kind, false, h->threads, h->smem),
+                                          decode_max_ctas_per_sm(h->kind, true, h->threads, h->smem)));
     h->max_grid = h->ctas_per_sm * h->sm_count;
     const size_t state_elems =
         static_cast<size_t>(h->max_grid) * cpb * h->tab.rows * static_cast<size_t>(z);
@@ -363,7 +363,7 @@ int decode_impl(Handle* h, const float* llr, uint8_t* packed, int n_cw, int n_it
     const int grid = std::min(a.n_groups, h->max_grid);
     if (!counter && cudaMemsetAsync(h->scratch, 0, sizeof(int), stream) != cudaSuccess) return NRLDPC_ERR_CUDA;
     return map_cuda(launch_decode(h->tab, a, weighted ? h->weights : nullptr, grid, h->threads, h->smem,
-                                  h->schedule == NRLDPC_SCHEDULE_LAYERED, h->minb, stream));
+                                  h->schedule == NRLDPC_SCHEDULE_LAYERED, h->kind, stream));
 }
 
 // Host-buffer decode (fp32 LLRs, or narrow ones widened on the GPU: qtype 1

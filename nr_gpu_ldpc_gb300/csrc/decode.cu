@@ -36,7 +36,29 @@
 namespace nrldpc {
 namespace {
 
-constexpr int kKeepQMax = 10;  // longest row whose Q stay in registers (unweighted flooding)
+// What a kernel is compiled for (RowClass): the distance from Lold to Lnew,
+// the degrees that occur (bit d), which of them end in a suffix column (those
+// up to most_sfx; any_sfx of row_update where the class does not say), and the
+// longest row whose Q stay in registers in unweighted flooding.  In both NR
+// base graphs a row's degree tells whether it has a suffix column, so the row
+// bodies have no test for one; together with the fixed distance (each worth
+// about half; BG1 by steps 5.85 -> 5.72 -> 5.39 ms):
+//   us per call                       any code    class
+//   BG1 Z=384, 4,096 codewords, 10 it.    5860     5393
+//   the same, with weights                7400     6832
+//   layered, 6 iterations                 3440     3273
+//   BG1 Z=208, 3,000                      2771     2565
+//   BG2 Z=384, 3,000                      2997     2758
+//   BG2 Z=208, 1,001, early stop           607      563
+struct RowTraits {
+    uint32_t far, degrees;
+    int most_sfx, keep_q;
+};
+__host__ __device__ constexpr RowTraits row_traits(RowClass c) {
+    return c == RowClass::kBg1 ? RowTraits{kFarLong, 0x807f8u, 10, 10}
+         : c == RowClass::kBg2 ? RowTraits{kFarShort, 0x578u, 6, 8}
+                               : RowTraits{0u, 0xffffeu, -1, 10};
+}
 constexpr int kMaxCpb = 48;
 constexpr int kHeaderBytes = 1024;  // mbarrier, group id, per-slot flags
 // Weights of the current iteration in shared memory, one padded row of
@@ -173,14 +195,15 @@ __device__ __forceinline__ uint32_t lds_u8(uint32_t a) {
 // (kPair: not in the unweighted layered kernels, 1-2% slower with it).
 // Measured with the wrapped address below, BG1 Z=384 flooding 6.16 -> 6.00 ms
 // per 4,096 codewords, layered with weights 4.05 -> 3.97.
-template <int D, bool WEIGHTED, bool LAYERED, int MAXD>
-__device__ __forceinline__ void row_update(const CodeTable& tab, int e0, bool sfx, uint32_t s,
+template <int D, bool WEIGHTED, bool LAYERED, RowClass CLASS>
+__device__ __forceinline__ void row_update(const CodeTable& tab, int e0, bool any_sfx, uint32_t s,
                                            uint32_t s4old, uint32_t dnew, uint32_t z4,
                                            const float4* wprev, const float4* wcur, uint4 st, uint4* st_out,
                                            bool store, bool write_hd, uint32_t hd, float alpha) {
     constexpr int LAST = D - 1;
     constexpr bool kPlain = !WEIGHTED && !LAYERED;
-    constexpr bool kKeepQ = LAYERED || (kPlain && MAXD > kKeepQMax && D <= kKeepQMax);
+    constexpr bool kKeepQ = LAYERED || (kPlain && D <= row_traits(CLASS).keep_q);
+    const bool sfx = CLASS == RowClass::kAny ? any_sfx : D <= row_traits(CLASS).most_sfx;
     constexpr bool kPair = kKeepQ && (kPlain || WEIGHTED);
     uint32_t addr[D];
     float lv[D];
@@ -311,10 +334,9 @@ __device__ __forceinline__ void row_update(const CodeTable& tab, int e0, bool sf
     }
 }
 
-// Degree switch up to MAXD: 10 for BG2 and codes like it, whose kernels then
-// hold no registers for BG1's rows of 19 (1,001 codewords of BG2 Z=208 with
-// early stop 667 -> 625 us with the wrapped address).
-template <bool WEIGHTED, bool LAYERED, int MAXD>
+// Degree switch over the degrees of the class: BG2's kernels hold no registers
+// for BG1's rows of 19.
+template <bool WEIGHTED, bool LAYERED, RowClass CLASS>
 __device__ __forceinline__ void row_dispatch(int deg, const CodeTable& tab, int e0, bool sfx, uint32_t s,
                                              uint32_t s4old, uint32_t dnew, uint32_t z4,
                                              const float4* wprev, const float4* wcur, uint4 st, uint4* st_out,
@@ -322,9 +344,9 @@ __device__ __forceinline__ void row_dispatch(int deg, const CodeTable& tab, int 
     switch (deg) {
 #define NRLDPC_ROW_CASE(D)                                                                                        \
     case D:                                                                                                       \
-        if constexpr (D <= MAXD)                                                                                  \
-            row_update<D, WEIGHTED, LAYERED, MAXD>(tab, e0, sfx, s, s4old, dnew, z4, wprev, wcur, st, st_out,     \
-                                                   store, write_hd, hd, alpha);                                   \
+        if constexpr (row_traits(CLASS).degrees >> D & 1)                                                         \
+            row_update<D, WEIGHTED, LAYERED, CLASS>(tab, e0, sfx, s, s4old, dnew, z4, wprev, wcur, st, st_out,    \
+                                                    store, write_hd, hd, alpha);                                  \
         break;
         NRLDPC_ROW_CASE(1) NRLDPC_ROW_CASE(2) NRLDPC_ROW_CASE(3) NRLDPC_ROW_CASE(4)
         NRLDPC_ROW_CASE(5) NRLDPC_ROW_CASE(6) NRLDPC_ROW_CASE(7) NRLDPC_ROW_CASE(8)
@@ -429,7 +451,7 @@ __device__ __forceinline__ void write_outputs(const CodeTable& tab, const float*
 // with the row table).  BG1 Z=384 6.00 -> 5.86 ms per 4,096 codewords.  In
 // batch_decode_kernel the advancing addresses are 2-3% slower, the advancing
 // edge 1% faster.
-template <bool WEIGHTED, bool LAYERED, int SPT, int MAXD, bool STEP>
+template <bool WEIGHTED, bool LAYERED, int SPT, RowClass CLASS, bool STEP>
 __device__ __forceinline__ void iterate_rows(const CodeTable& tab, uint32_t s, uint32_t tpc, uint32_t s4old,
                                              uint32_t dnew, const float4* wpad, uint4* st_base,
                                              const float* gllr,
@@ -466,7 +488,7 @@ __device__ __forceinline__ void iterate_rows(const CodeTable& tab, uint32_t s, u
                 }
                 const bool sfx = tab.row_sfx[r] != 0;
                 if (act)
-                    row_dispatch<WEIGHTED, LAYERED, MAXD>(
+                    row_dispatch<WEIGHTED, LAYERED, CLASS>(
                         tab.row_deg[r], tab, kStepEdge ? e0 : tab.row_ptr[r], sfx, s, s4old, dnew, z4,
                         wpad + r * (kWPad / 4), wpad + (kMaxRows + r) * (kWPad / 4), s0,
                         (kPlain || store) ? here : nullptr, store, kPlain ? write_hd : (write_hd && sfx),
@@ -480,7 +502,7 @@ __device__ __forceinline__ void iterate_rows(const CodeTable& tab, uint32_t s, u
                 s2 = fetch(r + 2, s);
                 const bool sfx = tab.row_sfx[r] != 0;
                 if (act)
-                    row_dispatch<WEIGHTED, LAYERED, MAXD>(
+                    row_dispatch<WEIGHTED, LAYERED, CLASS>(
                         tab.row_deg[r], tab, e0, sfx, s, s4old, dnew, z4, wpad + r * (kWPad / 4),
                         wpad + (kMaxRows + r) * (kWPad / 4), s0, st_base + r * z + s, store, write_hd,
                         hd_base + static_cast<uint32_t>(r * z), alpha);
@@ -495,7 +517,7 @@ __device__ __forceinline__ void iterate_rows(const CodeTable& tab, uint32_t s, u
         auto run = [&](int r, uint32_t j, uint4 st) {
             const uint32_t sj = s + j * tpc;
             const bool sfx = tab.row_sfx[r] != 0;
-            row_dispatch<WEIGHTED, LAYERED, MAXD>(
+            row_dispatch<WEIGHTED, LAYERED, CLASS>(
                 tab.row_deg[r], tab, tab.row_ptr[r], sfx, sj, s4old + 4u * j * tpc, dnew, z4, wpad + r * (kWPad / 4),
                 wpad + (kMaxRows + r) * (kWPad / 4), st, st_base + r * z + sj, store, write_hd,
                 hd_base + j * tpc + static_cast<uint32_t>(r * z), alpha);
@@ -648,7 +670,7 @@ struct SlotOut {
 // Lold in place.  Early stop: after iteration t < n_iter - 1, a codeword
 // whose hard decisions satisfy every check stops with iters = t + 1 (the
 // oracle's rule, ldpc_oracle.c decode_one_f32).
-template <bool WEIGHTED, bool LAYERED, int MAXD, int SPT = 1, bool STEP = false>
+template <bool WEIGHTED, bool LAYERED, RowClass CLASS, int SPT = 1, bool STEP = false>
 __device__ __forceinline__ void run_group(const CodeTable& tab, int cpb, int slot, uint32_t s, uint32_t tpc,
                                           bool slot_done, float* buf0, uint8_t* hd0,
                                           int* s_fail, uint4* st_base, const float* gllr, SlotOut out,
@@ -657,10 +679,11 @@ __device__ __forceinline__ void run_group(const CodeTable& tab, int cpb, int slo
     const int z = tab.z, cf = tab.core_floats, tid = threadIdx.x;
     int* s_far = s_fail + kFarOffset;  // per slot: row of the last failed check
     float* lold = buf0 + static_cast<size_t>(slot) * cf;  // read by the check-node pass
-    float* lnew = LAYERED ? lold : lold + static_cast<size_t>(cpb) * cf;  // the posterior written
+    constexpr uint32_t kFar = row_traits(CLASS).far;
+    const uint32_t dnew = LAYERED ? 0u : kFar ? kFar : static_cast<uint32_t>(cpb) * static_cast<uint32_t>(cf) * 4u;
+    float* lnew = lold + dnew / 4;  // the posterior written
     const uint8_t* hd = hd0 + static_cast<size_t>(slot) * tab.rows * z;
     const uint32_t s4old = smem_addr(lold) + 4u * s;
-    const uint32_t dnew = LAYERED ? 0u : static_cast<uint32_t>(cpb) * static_cast<uint32_t>(cf) * 4u;
     const uint32_t hd_base = smem_addr(hd) + s;
     const int nt = static_cast<int>(tpc);  // threads of the slot
     // flooding: Lnew starts as the LLRs; unweighted, Lold as the LLRs with
@@ -697,7 +720,7 @@ __device__ __forceinline__ void run_group(const CodeTable& tab, int cpb, int slo
         const bool far_check = __syncthreads_or(!slot_done && s_far[slot] >= kFarRow);
         const bool act = !slot_done;
         const bool store = !last || out.app != nullptr;
-        iterate_rows<WEIGHTED, LAYERED, SPT, MAXD, STEP>(tab, s, tpc, s4old, dnew, wpad, st_base, gllr, hd_base, act,
+        iterate_rows<WEIGHTED, LAYERED, SPT, CLASS, STEP>(tab, s, tpc, s4old, dnew, wpad, st_base, gllr, hd_base, act,
                                                      first, store, early_stop || last, alpha);
         if (early_stop && !last) {  // the rows ended with a barrier
             // bit-sliced scratch: flooding in Lold (read again only after the
@@ -750,7 +773,7 @@ struct WeightParam<true> {
 
 // FROM_HOST: a.llr is pinned host memory (a separate instantiation, so the
 // device-resident kernels keep their register allocation).
-template <bool WEIGHTED, int MINB, bool LAYERED, bool FROM_HOST, int MAXD>
+template <bool WEIGHTED, int MINB, bool LAYERED, bool FROM_HOST, RowClass CLASS>
 __global__ void __launch_bounds__(kMaxThreads, MINB)
     decode_kernel(const __grid_constant__ CodeTable tab, const __grid_constant__ DecodeArgs a,
                   const __grid_constant__ typename WeightParam<WEIGHTED>::type wt) {
@@ -764,7 +787,8 @@ __global__ void __launch_bounds__(kMaxThreads, MINB)
     if constexpr (WEIGHTED) wtab = &wt.w[0][0];
 
     const int z = tab.z, n = tab.n_bp, cpb = a.cpb, rows = tab.rows, cf = tab.core_floats;
-    uint8_t* hd0 = reinterpret_cast<uint8_t*>(buf0 + 2 * static_cast<size_t>(cpb) * cf);
+    uint8_t* hd0 = reinterpret_cast<uint8_t*>(buf0) + group_hd_offset(4u * cpb * cf, (cpb * rows * z + 15) / 16 * 16,
+                                                                      row_traits(CLASS).far);
     const int tid = threadIdx.x;
     const int slot = tid / z;
     const uint32_t s = static_cast<uint32_t>(tid - slot * z);
@@ -829,7 +853,7 @@ __global__ void __launch_bounds__(kMaxThreads, MINB)
         const size_t cw = static_cast<size_t>(cw0 + (slot_done ? 0 : slot));
         SlotOut out{a.packed + cw * tab.packed_bytes, a.app ? a.app + cw * n : nullptr,
                     a.iters ? a.iters + cw : nullptr};
-        run_group<WEIGHTED, LAYERED, MAXD, 1, true>(tab, cpb, slot, s, static_cast<uint32_t>(z), slot_done, buf0,
+        run_group<WEIGHTED, LAYERED, CLASS, 1, true>(tab, cpb, slot, s, static_cast<uint32_t>(z), slot_done, buf0,
                                                     hd0, s_fail, st_base, a.llr + cw * n, out, a.n_iter,
                                                     a.early_stop, a.alpha, wtab, wpad, a.n_w_iters);
     }
@@ -897,62 +921,79 @@ __global__ void __launch_bounds__(kMaxThreads, 2)
         uint4* st_base = reinterpret_cast<uint4*>(a.state + static_cast<size_t>(blockIdx.x) * a.slot_words) +
                          static_cast<size_t>(valid_thread ? slot : 0) * tab.rows * z;
         if (item.spt == 2)
-            run_group<false, false, kMaxDeg, 2>(tab, cpb, slot, s, static_cast<uint32_t>(tpc), !valid_thread, buf0, hd0,
-                                       s_fail, st_base, a.llr + job.llr_offset, out, a.n_iter, a.early_stop, a.alpha,
-                                       nullptr, nullptr, 1);
+            run_group<false, false, RowClass::kAny, 2>(tab, cpb, slot, s, static_cast<uint32_t>(tpc), !valid_thread, buf0,
+                                                   hd0, s_fail, st_base, a.llr + job.llr_offset, out, a.n_iter,
+                                                   a.early_stop, a.alpha, nullptr, nullptr, 1);
         else
-            run_group<false, false, kMaxDeg>(tab, cpb, slot, s, static_cast<uint32_t>(tpc), !valid_thread, buf0, hd0,
-                                       s_fail, st_base, a.llr + job.llr_offset, out, a.n_iter, a.early_stop, a.alpha,
-                                       nullptr, nullptr, 1);
+            run_group<false, false, RowClass::kAny>(tab, cpb, slot, s, static_cast<uint32_t>(tpc), !valid_thread, buf0, hd0,
+                                                s_fail, st_base, a.llr + job.llr_offset, out, a.n_iter, a.early_stop,
+                                                a.alpha, nullptr, nullptr, 1);
     }
 }
 
 }  // namespace
 
-size_t decode_smem_bytes(const CodeTable& tab, int cpb) {
-    return kHeaderBytes + kWeightBytes + group_smem_bytes(tab, cpb);
+size_t decode_smem_bytes(const CodeTable& tab, int cpb, uint32_t far) {
+    return kHeaderBytes + kWeightBytes + group_smem_bytes(tab, cpb, far);
 }
 
-// The kernel for a code of row degrees up to 10 or up to 19; from_host: the
-// unweighted kernels that read host-resident LLRs.
-template <int MAXD, int MINB>
+// Two CTAs per SM when shared memory allows (the kernels then cap their
+// registers for two), otherwise one with the full register budget.  A class's
+// kernels are taken when every row is of the class, the buffers fit the fixed
+// distance and the larger CTA costs no resident one: so for every NR code at
+// the default codewords per CTA (192 < cpb * Z <= 384 but for the smallest Z),
+// while a CTA set to fewer would lose a third to a half of its neighbours.
+DecodeShape decode_shape(const CodeTable& tab, int cpb, size_t smem_block, size_t smem_sm) {
+    DecodeShape d;
+    d.cpb = cpb;
+    d.threads = (cpb * tab.z + 31) / 32 * 32;
+    d.smem = decode_smem_bytes(tab, cpb);
+    d.kind = 2 * (d.smem + 1024) <= smem_sm ? DecodeKind::kAny2 : DecodeKind::kAny1;
+    if (d.kind == DecodeKind::kAny1) return d;
+    const size_t half = static_cast<size_t>(cpb) * tab.core_floats * 4;
+    for (RowClass c : {RowClass::kBg1, RowClass::kBg2}) {
+        const RowTraits t = row_traits(c);
+        const size_t smem = decode_smem_bytes(tab, cpb, t.far);
+        bool fits = half <= t.far && smem <= smem_block &&
+                    decode_ctas(d.threads, smem, smem_sm) >= decode_ctas(d.threads, d.smem, smem_sm);
+        for (int r = 0; r < tab.rows; r++)
+            fits &= (t.degrees >> tab.row_deg[r] & 1) && (tab.row_sfx[r] != 0) == (tab.row_deg[r] <= t.most_sfx);
+        if (!fits) continue;
+        d.kind = c == RowClass::kBg1 ? DecodeKind::kBg1 : DecodeKind::kBg2;
+        d.smem = smem;
+        break;
+    }
+    return d;
+}
+
+// from_host: the unweighted kernels that read host-resident LLRs
+template <int MINB, RowClass CLASS>
 const void* kernel_of(bool weighted, bool layered, bool from_host) {
     if (from_host && !weighted)
-        return layered ? reinterpret_cast<const void*>(&decode_kernel<false, MINB, true, true, MAXD>)
-                       : reinterpret_cast<const void*>(&decode_kernel<false, MINB, false, true, MAXD>);
+        return layered ? reinterpret_cast<const void*>(&decode_kernel<false, MINB, true, true, CLASS>)
+                       : reinterpret_cast<const void*>(&decode_kernel<false, MINB, false, true, CLASS>);
     if (layered)
-        return weighted ? reinterpret_cast<const void*>(&decode_kernel<true, MINB, true, false, MAXD>)
-                        : reinterpret_cast<const void*>(&decode_kernel<false, MINB, true, false, MAXD>);
-    return weighted ? reinterpret_cast<const void*>(&decode_kernel<true, MINB, false, false, MAXD>)
-                    : reinterpret_cast<const void*>(&decode_kernel<false, MINB, false, false, MAXD>);
+        return weighted ? reinterpret_cast<const void*>(&decode_kernel<true, MINB, true, false, CLASS>)
+                        : reinterpret_cast<const void*>(&decode_kernel<false, MINB, true, false, CLASS>);
+    return weighted ? reinterpret_cast<const void*>(&decode_kernel<true, MINB, false, false, CLASS>)
+                    : reinterpret_cast<const void*>(&decode_kernel<false, MINB, false, false, CLASS>);
 }
 
-const void* select_kernel(bool short_rows, bool weighted, int minb, bool layered, bool from_host) {
-    if (short_rows) {
-        return minb >= 2 ? kernel_of<10, 2>(weighted, layered, from_host) : kernel_of<10, 1>(weighted, layered, from_host);
+const void* select_kernel(DecodeKind kind, bool weighted, bool layered, bool from_host) {
+    switch (kind) {
+        case DecodeKind::kAny1: return kernel_of<1, RowClass::kAny>(weighted, layered, from_host);
+        case DecodeKind::kAny2: return kernel_of<2, RowClass::kAny>(weighted, layered, from_host);
+        case DecodeKind::kBg1: return kernel_of<2, RowClass::kBg1>(weighted, layered, from_host);
+        default: return kernel_of<2, RowClass::kBg2>(weighted, layered, from_host);
     }
-    return minb >= 2 ? kernel_of<kMaxDeg, 2>(weighted, layered, from_host)
-                     : kernel_of<kMaxDeg, 1>(weighted, layered, from_host);
-}
-
-bool has_short_rows(const CodeTable& tab) {
-    for (int r = 0; r < tab.rows; r++)
-        if (tab.row_deg[r] > 10) return false;
-    return true;
-}
-
-cudaError_t launch_batch_decode(const BatchDecodeArgs& args, int grid, int threads, size_t smem,
-                                cudaStream_t stream) {
-    batch_decode_kernel<<<grid, threads, smem, stream>>>(args);
-    return cudaGetLastError();
 }
 
 const void* batch_decode_kernel_ptr() { return reinterpret_cast<const void*>(&batch_decode_kernel); }
 
-cudaError_t decode_kernel_attributes(bool short_rows, int minb, size_t smem) {
+cudaError_t decode_kernel_attributes(DecodeKind kind, size_t smem) {
     for (int k = 0; k < 6; k++) {  // plain, weighted, plain from host; both schedules
         const int w = k % 3;
-        const cudaError_t e = cudaFuncSetAttribute(select_kernel(short_rows, w == 1, minb, k >= 3, w == 2),
+        const cudaError_t e = cudaFuncSetAttribute(select_kernel(kind, w == 1, k >= 3, w == 2),
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return e;
     }
@@ -960,12 +1001,12 @@ cudaError_t decode_kernel_attributes(bool short_rows, int minb, size_t smem) {
 }
 
 // both schedules, device- and host-resident LLRs
-int decode_max_ctas_per_sm(const CodeTable& tab, bool weighted, int minb, int threads, size_t smem) {
+int decode_max_ctas_per_sm(DecodeKind kind, bool weighted, int threads, size_t smem) {
     int n = 1 << 30;
     for (int l = 0; l < 4; l++) {
         int k = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                &k, select_kernel(has_short_rows(tab), weighted, minb, l & 1, l >= 2), threads, smem) != cudaSuccess)
+                &k, select_kernel(kind, weighted, l & 1, l >= 2), threads, smem) != cudaSuccess)
             return 0;
         n = k < n ? k : n;
     }
@@ -973,11 +1014,11 @@ int decode_max_ctas_per_sm(const CodeTable& tab, bool weighted, int minb, int th
 }
 
 cudaError_t launch_decode(const CodeTable& tab, const DecodeArgs& args, const WeightTable* weights, int grid,
-                          int threads, size_t smem, bool layered, int minb, cudaStream_t stream) {
+                          int threads, size_t smem, bool layered, DecodeKind kind, cudaStream_t stream) {
     if (args.cpb < 1 || args.cpb > kMaxCpb) return cudaErrorInvalidValue;
     const bool weighted = weights != nullptr;
     if (weighted && args.llr_from_host) return cudaErrorInvalidValue;
-    const void* k = select_kernel(has_short_rows(tab), weighted, minb, layered, args.llr_from_host != 0);
+    const void* k = select_kernel(kind, weighted, layered, args.llr_from_host != 0);
     NoWeights none{};
     void* params[3] = {const_cast<CodeTable*>(&tab), const_cast<DecodeArgs*>(&args),
                        weighted ? const_cast<WeightTable*>(weights) : static_cast<void*>(&none)};

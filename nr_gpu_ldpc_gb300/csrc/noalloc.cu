@@ -70,10 +70,10 @@ int setup_device(int dev, DeviceSetup** out) {
         if (cudaGetSymbolAddress(&p, g_noalloc_state) != cudaSuccess ||
             cudaGetSymbolAddress(&q, g_noalloc_counters) != cudaSuccess ||
             cudaGetDeviceProperties(&prop, dev) != cudaSuccess ||
-            decode_kernel_attributes(false, 1, prop.sharedMemPerBlockOptin) != cudaSuccess ||
-            decode_kernel_attributes(false, 2, prop.sharedMemPerBlockOptin) != cudaSuccess ||
-            decode_kernel_attributes(true, 1, prop.sharedMemPerBlockOptin) != cudaSuccess ||
-            decode_kernel_attributes(true, 2, prop.sharedMemPerBlockOptin) != cudaSuccess) {
+            decode_kernel_attributes(DecodeKind::kAny1, prop.sharedMemPerBlockOptin) != cudaSuccess ||
+            decode_kernel_attributes(DecodeKind::kAny2, prop.sharedMemPerBlockOptin) != cudaSuccess ||
+            decode_kernel_attributes(DecodeKind::kBg1, prop.sharedMemPerBlockOptin) != cudaSuccess ||
+            decode_kernel_attributes(DecodeKind::kBg2, prop.sharedMemPerBlockOptin) != cudaSuccess) {
             cudaGetLastError();  // leave no sticky launch-side error behind; retried next call
             return NRLDPC_ERR_CUDA;
         }
@@ -107,11 +107,9 @@ int noalloc_decode(int bg, int z, float alpha, const float* d_llr, uint8_t* d_pa
     int cpb = std::max(1, kMaxThreads / z);
     while (cpb > 1 && decode_smem_bytes(tab, cpb) > s->smem_optin) cpb--;
     cpb = std::min(cpb, 48);
-    const size_t smem = decode_smem_bytes(tab, cpb);
-    if (smem > s->smem_optin) return NRLDPC_ERR_BAD_CONFIG;
-    const int threads = (cpb * z + 31) / 32 * 32;
-    const int minb = (2 * (smem + 1024) <= s->smem_per_sm) ? 2 : 1;
-    const int per_sm = decode_max_ctas_per_sm(tab, false, minb, threads, smem);
+    const DecodeShape shape = decode_shape(tab, cpb, s->smem_optin, s->smem_per_sm);
+    if (shape.smem > s->smem_optin) return NRLDPC_ERR_BAD_CONFIG;
+    const int per_sm = decode_max_ctas_per_sm(shape.kind, false, shape.threads, shape.smem);
     const size_t slot_bytes = static_cast<size_t>(cpb) * tab.rows * tab.z * kStateBytesPerRow;
     const size_t slots = kNoAllocScratchBytes / slot_bytes;
     if (slots < 1) return NRLDPC_ERR_SCRATCH_TOO_SMALL;
@@ -134,7 +132,7 @@ int noalloc_decode(int bg, int z, float alpha, const float* d_llr, uint8_t* d_pa
     const int grid = static_cast<int>(std::min<long>(a.n_groups, max_grid));
     // only the scheduler counter: the error word stays set until it is read
     if (cudaMemsetAsync(s->counters, 0, sizeof(int), st) != cudaSuccess) return NRLDPC_ERR_CUDA;
-    return launch_decode(tab, a, nullptr, grid, threads, smem, false, minb, st) == cudaSuccess ? NRLDPC_OK
+    return launch_decode(tab, a, nullptr, grid, shape.threads, shape.smem, false, shape.kind, st) == cudaSuccess ? NRLDPC_OK
                                                                                        : NRLDPC_ERR_CUDA;
 }
 

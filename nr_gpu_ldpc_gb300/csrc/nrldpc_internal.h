@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <cstddef>
+#include <algorithm>
 #include <cstdint>
 #include <vector>
 
@@ -79,6 +80,11 @@ struct DecodeArgs {
     uint32_t extra_tx;
 };
 
+// What decode_kernel is compiled for: any code, or one whose rows are like
+// BG1's or BG2's (decode.cu, row_traits)
+enum class RowClass { kAny, kBg1, kBg2 };
+// kAny1, kAny2: any code, one or two CTAs per SM in the register budget
+enum class DecodeKind { kAny1, kAny2, kBg1, kBg2 };
 enum DeviceError : int { kErrNone = 0, kErrLlrLoadTimeout = 1, kErrSplitTimeout = 2 };
 
 // Mixed-code batches (batch.cu): a work item is up to `count` codewords of
@@ -109,13 +115,24 @@ struct BatchDecodeArgs {
 };
 // Shared memory of one decode group of cpb codewords: Lold and Lnew over the
 // core columns, plus one hard-decision byte per lifted row for the suffix
-// columns.
-inline size_t group_smem_bytes(const CodeTable& t, int cpb) {
-    const size_t hd = (static_cast<size_t>(cpb) * t.rows * t.z + 15) / 16 * 16;
-    return 2 * static_cast<size_t>(cpb) * t.core_floats * sizeof(float) + hd;
+// columns.  Lnew is `far` bytes after Lold, the decisions in the gap when they
+// fit; far = 0: right after it, the decisions last.  At a distance that the
+// compiler knows, an edge's Lnew accesses are its Lold address and an
+// immediate offset.
+constexpr uint32_t kFarLong = kMaxThreads * 26 * 4;   // BG1's core columns at the most sub-rows per CTA
+constexpr uint32_t kFarShort = kMaxThreads * 14 * 4;  // BG2's
+__host__ __device__ inline uint32_t group_hd_offset(uint32_t half, uint32_t hd, uint32_t far) {
+    return far == 0 ? 2 * half : half + hd <= far ? half : far + half;
 }
-cudaError_t launch_batch_decode(const BatchDecodeArgs& args, int grid, int threads, size_t smem,
-                                cudaStream_t stream);
+inline size_t group_smem_bytes(const CodeTable& t, int cpb, uint32_t far) {
+    const size_t hd = (static_cast<size_t>(cpb) * t.rows * t.z + 15) / 16 * 16;
+    const size_t half = static_cast<size_t>(cpb) * t.core_floats * sizeof(float);
+    return far == 0 ? 2 * half + hd : far + half + (half + hd <= far ? 0 : hd);
+}
+// CTAs per SM by registers (80 a thread) and shared memory
+inline int decode_ctas(int threads, size_t smem, size_t smem_sm) {
+    return static_cast<int>(std::min<size_t>(65536 / (80 * threads), smem_sm / (smem + 1024)));
+}
 const void* batch_decode_kernel_ptr();
 
 // One codeword on a cluster of CTAs (split.cu).  A plan is a head and one
@@ -181,15 +198,21 @@ cudaError_t launch_split(const SplitHead& head, const SplitArgs& args, const Wei
                          cudaStream_t stream);
 
 // Host-side launchers (decode.cu / channel.cu).
-// minb: CTAs per SM the kernel's register budget assumes (1 or 2).
+// kind: which kernels serve a code and geometry (decode_shape).
 // weights: null for the plain decoder; layered: row-sequential schedule (no
 // reference counterpart) instead of flooding.
 cudaError_t launch_decode(const CodeTable& tab, const DecodeArgs& args, const WeightTable* weights, int grid,
-                          int threads, size_t smem, bool layered, int minb, cudaStream_t stream);
-size_t decode_smem_bytes(const CodeTable& tab, int cpb);
-bool has_short_rows(const CodeTable& tab);  // every row of degree up to 10: kernels with fewer registers
-cudaError_t decode_kernel_attributes(bool short_rows, int minb, size_t smem);
-int decode_max_ctas_per_sm(const CodeTable& tab, bool weighted, int minb, int threads, size_t smem);
+                          int threads, size_t smem, bool layered, DecodeKind kind, cudaStream_t stream);
+size_t decode_smem_bytes(const CodeTable& tab, int cpb, uint32_t far = 0);
+// CTA geometry of cpb codewords per CTA
+struct DecodeShape {
+    int cpb = 1, threads = 32;
+    size_t smem = 0;
+    DecodeKind kind = DecodeKind::kAny1;
+};
+DecodeShape decode_shape(const CodeTable& tab, int cpb, size_t smem_block, size_t smem_sm);
+cudaError_t decode_kernel_attributes(DecodeKind kind, size_t smem);
+int decode_max_ctas_per_sm(DecodeKind kind, bool weighted, int threads, size_t smem);
 
 // Learned weighted min-sum training kernels (wms.cu).
 size_t wms_smem_bytes(const CodeTable& tab, int cpb, bool layered);
