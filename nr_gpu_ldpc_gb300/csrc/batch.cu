@@ -24,7 +24,6 @@ using namespace nrldpc;
 
 namespace {
 
-constexpr int kNumZ = 51;
 constexpr int kNumCodes = 2 * kNumZ;
 constexpr int kBaseZ[8] = {2, 3, 5, 7, 9, 11, 13, 15};
 
@@ -254,7 +253,7 @@ struct Batch {
     float alpha = 0.75f;
     int max_jobs = 0;
     int sm_count = 1;
-    size_t smem_optin = 0;
+    size_t smem_optin = 0, smem_sm = 0;
     CodeTable h_tables[kNumCodes];
     bool code_ok[kNumCodes];
     int cpb[kNumCodes];
@@ -288,6 +287,7 @@ struct Batch {
     SplitHead split{};
     int split_clusters = 0;
     size_t slot_words = 0, smem = 0;
+    bool classes = false;  // of rows and layouts (batch_decode_kernel)
     int grid = 0, threads = kMaxThreads;
     uint32_t* d_state = nullptr;
     size_t state_words = 0;
@@ -446,6 +446,7 @@ int nrldpc_batch_create(int device, int max_jobs, float alpha, nrldpc_batch** ou
     b->max_jobs = max_jobs;
     b->sm_count = prop.multiProcessorCount;
     b->smem_optin = prop.sharedMemPerBlockOptin;
+    b->smem_sm = prop.sharedMemPerMultiprocessor;
     std::vector<PlanDev> plans(kNumCodes);
     for (int bg = 1; bg <= 2; bg++)
         for (int zi = 0; zi < kNumZ; zi++) {
@@ -480,7 +481,9 @@ int nrldpc_batch_create(int device, int max_jobs, float alpha, nrldpc_batch** ou
     if (cudaMemcpy(b->d_tables, b->h_tables, sizeof(CodeTable) * kNumCodes, cudaMemcpyHostToDevice) ||
         cudaMemcpy(b->d_plans, plans.data(), sizeof(PlanDev) * kNumCodes, cudaMemcpyHostToDevice) ||
         cudaMemset(b->d_scratch, 0, 256) ||
-        cudaFuncSetAttribute(batch_decode_kernel_ptr(), cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(batch_decode_kernel_ptr(false), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(b->smem_optin)) ||
+        cudaFuncSetAttribute(batch_decode_kernel_ptr(true), cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(b->smem_optin)) ||
         split_kernel_attributes(b->smem_optin)) {
         free_batch(b);
@@ -580,8 +583,9 @@ int nrldpc_batch_set_jobs(nrldpc_batch* batch, const nrldpc_job* jobs, int n_job
         return b->h_jobs[x].code < b->h_jobs[y].code;
     });
     std::vector<WorkItem> items;
-    size_t slot_words = 0, bufs = 0;
+    size_t slot_words = 0, bufs = 0, class_bufs = 0;
     int threads = 32;
+    bool classes = true;
     for (int i = 0; i < n_jobs;) {
         const int id = b->h_jobs[order[i]].code;
         int k = i;
@@ -594,6 +598,9 @@ int nrldpc_batch_set_jobs(nrldpc_batch* batch, const nrldpc_job* jobs, int n_job
             threads = std::max(threads, (cnt * (t.z / spt) + 31) / 32 * 32);
             slot_words = std::max(slot_words, static_cast<size_t>(cnt) * 4 * t.rows * t.z);
             bufs = std::max(bufs, group_smem_bytes(t, cnt, 0));
+            const uint32_t far = id < kNumZ ? kFarLong : kFarShort;
+            class_bufs = std::max(class_bufs, group_smem_bytes(t, cnt, far));
+            classes &= spt == 1 && 4l * cnt * t.core_floats <= far;
         }
         i = k;
     }
@@ -602,8 +609,13 @@ int nrldpc_batch_set_jobs(nrldpc_batch* batch, const nrldpc_job* jobs, int n_job
     b->slot_words = slot_words;
     b->smem = kHeaderBytesBatch + kBatchTableBytes + bufs;
     b->threads = threads;  // the widest work item's threads
+    // the classes' layouts when they cost no resident CTA (as decode_shape)
+    const size_t class_smem = kHeaderBytesBatch + kBatchTableBytes + class_bufs;
+    b->classes = classes && class_smem <= b->smem_optin &&
+                 decode_ctas(threads, class_smem, b->smem_sm) >= decode_ctas(threads, b->smem, b->smem_sm);
+    if (b->classes) b->smem = class_smem;
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_decode_kernel_ptr(), b->threads, b->smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_decode_kernel_ptr(b->classes), b->threads, b->smem);
     b->grid = std::max(1, std::min(b->n_items, std::max(per_sm, 1) * b->sm_count));
     const size_t need = static_cast<size_t>(b->grid) * std::max<size_t>(slot_words, 1);
     if (need > b->state_words) {
@@ -705,7 +717,7 @@ int nrldpc_batch_decode(nrldpc_batch* batch, const float* d_llr, uint8_t* d_pack
     k.alpha = b->alpha;
     void* params[1] = {&k};
     cudaKernelNodeParams kp{};
-    kp.func = const_cast<void*>(batch_decode_kernel_ptr());
+    kp.func = const_cast<void*>(batch_decode_kernel_ptr(b->classes));
     kp.gridDim = dim3(b->grid);
     kp.blockDim = dim3(b->threads);
     kp.sharedMemBytes = static_cast<unsigned int>(b->smem);

@@ -445,13 +445,11 @@ __device__ __forceinline__ void write_outputs(const CodeTable& tab, const float*
 // next row's two sub-rows requested while this row's run.
 //   store: write this iteration's state; write_hd: write the suffix hard
 //   decisions.
-// STEP (kernels of a single code): the addresses of the prefetch, the stored
-// state and the decision byte advance from row to row instead of being formed
-// from r; so does the row's first edge in all but weighted flooding (4% faster
-// with the row table).  BG1 Z=384 6.00 -> 5.86 ms per 4,096 codewords.  In
-// batch_decode_kernel the advancing addresses are 2-3% slower, the advancing
-// edge 1% faster.
-template <bool WEIGHTED, bool LAYERED, int SPT, RowClass CLASS, bool STEP>
+// SPT = 1: the addresses of the prefetch, the stored state and the decision
+// byte advance from row to row instead of being formed from r; so does the
+// row's first edge in all but weighted flooding (4% faster with the row
+// table).  BG1 Z=384 6.00 -> 5.86 ms per 4,096 codewords.
+template <bool WEIGHTED, bool LAYERED, int SPT, RowClass CLASS>
 __device__ __forceinline__ void iterate_rows(const CodeTable& tab, uint32_t s, uint32_t tpc, uint32_t s4old,
                                              uint32_t dnew, const float4* wpad, uint4* st_base,
                                              const float* gllr,
@@ -471,6 +469,7 @@ __device__ __forceinline__ void iterate_rows(const CodeTable& tab, uint32_t s, u
     // kernels get null addresses for the stores they skip (faster for them)
     constexpr bool kPlain = !WEIGHTED && !LAYERED;
     if constexpr (SPT == 1) {
+        constexpr bool kStepEdge = !WEIGHTED || LAYERED;
         uint4 s0 = fetch(0, s), s1 = fetch(1, s);
         const uint4* ahead = st_base + 2 * z + s;  // state of row r + 2
         uint4* here = st_base + s;                 // state of row r
@@ -478,36 +477,23 @@ __device__ __forceinline__ void iterate_rows(const CodeTable& tab, uint32_t s, u
         int e0 = 0;
         for (int r = 0; r < rows; r++) {
             uint4 s2 = make_uint4(0u, 0u, 0u, 0u);
-            if constexpr (STEP) {
-                constexpr bool kStepEdge = !WEIGHTED || LAYERED;
-                if (act && r + 2 < rows) {
-                    if (!first)
-                        s2 = __ldcg(ahead);
-                    else if (tab.row_sfx[r + 2])
-                        s2.w = __float_as_uint(__ldcs(gllr + edge_pos(tab, tab.row_ptr[r + 3] - 1, s)));
-                }
-                const bool sfx = tab.row_sfx[r] != 0;
-                if (act)
-                    row_dispatch<WEIGHTED, LAYERED, CLASS>(
-                        tab.row_deg[r], tab, kStepEdge ? e0 : tab.row_ptr[r], sfx, s, s4old, dnew, z4,
-                        wpad + r * (kWPad / 4), wpad + (kMaxRows + r) * (kWPad / 4), s0,
-                        (kPlain || store) ? here : nullptr, store, kPlain ? write_hd : (write_hd && sfx),
-                        (kPlain || (write_hd && sfx)) ? hd : 0u, alpha);
-                ahead += z;
-                here += z;
-                hd += static_cast<uint32_t>(z);
-                if (kStepEdge) e0 += tab.row_deg[r];
-            } else {
-                static_assert(kPlain);
-                s2 = fetch(r + 2, s);
-                const bool sfx = tab.row_sfx[r] != 0;
-                if (act)
-                    row_dispatch<WEIGHTED, LAYERED, CLASS>(
-                        tab.row_deg[r], tab, e0, sfx, s, s4old, dnew, z4, wpad + r * (kWPad / 4),
-                        wpad + (kMaxRows + r) * (kWPad / 4), s0, st_base + r * z + s, store, write_hd,
-                        hd_base + static_cast<uint32_t>(r * z), alpha);
-                e0 += tab.row_deg[r];
+            if (act && r + 2 < rows) {
+                if (!first)
+                    s2 = __ldcg(ahead);
+                else if (tab.row_sfx[r + 2])
+                    s2.w = __float_as_uint(__ldcs(gllr + edge_pos(tab, tab.row_ptr[r + 3] - 1, s)));
             }
+            const bool sfx = tab.row_sfx[r] != 0;
+            if (act)
+                row_dispatch<WEIGHTED, LAYERED, CLASS>(
+                    tab.row_deg[r], tab, kStepEdge ? e0 : tab.row_ptr[r], sfx, s, s4old, dnew, z4,
+                    wpad + r * (kWPad / 4), wpad + (kMaxRows + r) * (kWPad / 4), s0,
+                    (kPlain || store) ? here : nullptr, store, kPlain ? write_hd : (write_hd && sfx),
+                    (kPlain || (write_hd && sfx)) ? hd : 0u, alpha);
+            ahead += z;
+            here += z;
+            hd += static_cast<uint32_t>(z);
+            if (kStepEdge) e0 += tab.row_deg[r];
             s0 = s1;
             s1 = s2;
             if (tab.sync_after[r]) __syncthreads();
@@ -670,7 +656,7 @@ struct SlotOut {
 // Lold in place.  Early stop: after iteration t < n_iter - 1, a codeword
 // whose hard decisions satisfy every check stops with iters = t + 1 (the
 // oracle's rule, ldpc_oracle.c decode_one_f32).
-template <bool WEIGHTED, bool LAYERED, RowClass CLASS, int SPT = 1, bool STEP = false>
+template <bool WEIGHTED, bool LAYERED, RowClass CLASS, int SPT = 1>
 __device__ __forceinline__ void run_group(const CodeTable& tab, int cpb, int slot, uint32_t s, uint32_t tpc,
                                           bool slot_done, float* buf0, uint8_t* hd0,
                                           int* s_fail, uint4* st_base, const float* gllr, SlotOut out,
@@ -720,7 +706,7 @@ __device__ __forceinline__ void run_group(const CodeTable& tab, int cpb, int slo
         const bool far_check = __syncthreads_or(!slot_done && s_far[slot] >= kFarRow);
         const bool act = !slot_done;
         const bool store = !last || out.app != nullptr;
-        iterate_rows<WEIGHTED, LAYERED, SPT, CLASS, STEP>(tab, s, tpc, s4old, dnew, wpad, st_base, gllr, hd_base, act,
+        iterate_rows<WEIGHTED, LAYERED, SPT, CLASS>(tab, s, tpc, s4old, dnew, wpad, st_base, gllr, hd_base, act,
                                                      first, store, early_stop || last, alpha);
         if (early_stop && !last) {  // the rows ended with a barrier
             // bit-sliced scratch: flooding in Lold (read again only after the
@@ -853,7 +839,7 @@ __global__ void __launch_bounds__(kMaxThreads, MINB)
         const size_t cw = static_cast<size_t>(cw0 + (slot_done ? 0 : slot));
         SlotOut out{a.packed + cw * tab.packed_bytes, a.app ? a.app + cw * n : nullptr,
                     a.iters ? a.iters + cw : nullptr};
-        run_group<WEIGHTED, LAYERED, CLASS, 1, true>(tab, cpb, slot, s, static_cast<uint32_t>(z), slot_done, buf0,
+        run_group<WEIGHTED, LAYERED, CLASS>(tab, cpb, slot, s, static_cast<uint32_t>(z), slot_done, buf0,
                                                     hd0, s_fail, st_base, a.llr + cw * n, out, a.n_iter,
                                                     a.early_stop, a.alpha, wtab, wpad, a.n_w_iters);
     }
@@ -863,6 +849,11 @@ __global__ void __launch_bounds__(kMaxThreads, MINB)
 // codes.  Each item = up to cpb codewords of one code; the item's code table
 // is copied into shared memory and every codeword is fetched from its own
 // offset with its own bulk copy.
+// CLASSES: no item of the list has two sub-rows per thread, and every item has
+// the layout and the rows of its base graph's class (8,192 jobs of 14 codes
+// 5.92 -> 5.55 ms); its 3% over single-code launches are the table reads from
+// shared memory.
+template <bool CLASSES>
 __global__ void __launch_bounds__(kMaxThreads, 2)
     batch_decode_kernel(const __grid_constant__ BatchDecodeArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -894,7 +885,10 @@ __global__ void __launch_bounds__(kMaxThreads, 2)
         const CodeTable& tab = *stab;
         const int z = tab.z, cf = tab.core_floats, cpb = item.count;
         const int tpc = z / item.spt;  // threads per codeword: each owns spt sub-rows
-        uint8_t* hd0 = reinterpret_cast<uint8_t*>(buf0 + 2 * static_cast<size_t>(cpb) * cf);
+        const bool bg1 = item.code < kNumZ;
+        uint8_t* hd0 = reinterpret_cast<uint8_t*>(buf0) +
+                       group_hd_offset(4u * cpb * cf, (cpb * tab.rows * z + 15) / 16 * 16,
+                                       !CLASSES ? 0 : bg1 ? kFarLong : kFarShort);
         const int slot = tid / tpc;
         const uint32_t s = static_cast<uint32_t>(tid - slot * tpc);
         const bool valid_thread = slot < cpb;
@@ -920,14 +914,24 @@ __global__ void __launch_bounds__(kMaxThreads, 2)
         SlotOut out{a.packed + job.out_offset, nullptr, a.iters ? a.iters + jidx : nullptr};
         uint4* st_base = reinterpret_cast<uint4*>(a.state + static_cast<size_t>(blockIdx.x) * a.slot_words) +
                          static_cast<size_t>(valid_thread ? slot : 0) * tab.rows * z;
-        if (item.spt == 2)
-            run_group<false, false, RowClass::kAny, 2>(tab, cpb, slot, s, static_cast<uint32_t>(tpc), !valid_thread, buf0,
-                                                   hd0, s_fail, st_base, a.llr + job.llr_offset, out, a.n_iter,
-                                                   a.early_stop, a.alpha, nullptr, nullptr, 1);
-        else
-            run_group<false, false, RowClass::kAny>(tab, cpb, slot, s, static_cast<uint32_t>(tpc), !valid_thread, buf0, hd0,
-                                                s_fail, st_base, a.llr + job.llr_offset, out, a.n_iter, a.early_stop,
-                                                a.alpha, nullptr, nullptr, 1);
+        if constexpr (CLASSES) {
+            if (bg1)
+                run_group<false, false, RowClass::kBg1>(tab, cpb, slot, s, static_cast<uint32_t>(tpc), !valid_thread,
+                                                        buf0, hd0, s_fail, st_base, a.llr + job.llr_offset, out,
+                                                        a.n_iter, a.early_stop, a.alpha, nullptr, nullptr, 1);
+            else
+                run_group<false, false, RowClass::kBg2>(tab, cpb, slot, s, static_cast<uint32_t>(tpc), !valid_thread,
+                                                        buf0, hd0, s_fail, st_base, a.llr + job.llr_offset, out,
+                                                        a.n_iter, a.early_stop, a.alpha, nullptr, nullptr, 1);
+        } else if (item.spt == 2) {
+            run_group<false, false, RowClass::kAny, 2>(tab, cpb, slot, s, static_cast<uint32_t>(tpc), !valid_thread,
+                                                       buf0, hd0, s_fail, st_base, a.llr + job.llr_offset, out,
+                                                       a.n_iter, a.early_stop, a.alpha, nullptr, nullptr, 1);
+        } else {
+            run_group<false, false, RowClass::kAny>(tab, cpb, slot, s, static_cast<uint32_t>(tpc), !valid_thread, buf0,
+                                                    hd0, s_fail, st_base, a.llr + job.llr_offset, out, a.n_iter,
+                                                    a.early_stop, a.alpha, nullptr, nullptr, 1);
+        }
     }
 }
 
@@ -988,7 +992,10 @@ const void* select_kernel(DecodeKind kind, bool weighted, bool layered, bool fro
     }
 }
 
-const void* batch_decode_kernel_ptr() { return reinterpret_cast<const void*>(&batch_decode_kernel); }
+const void* batch_decode_kernel_ptr(bool classes) {
+    return classes ? reinterpret_cast<const void*>(&batch_decode_kernel<true>)
+                   : reinterpret_cast<const void*>(&batch_decode_kernel<false>);
+}
 
 cudaError_t decode_kernel_attributes(DecodeKind kind, size_t smem) {
     for (int k = 0; k < 6; k++) {  // plain, weighted, plain from host; both schedules

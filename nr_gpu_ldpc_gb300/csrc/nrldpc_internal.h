@@ -89,8 +89,9 @@ enum DeviceError : int { kErrNone = 0, kErrLlrLoadTimeout = 1, kErrSplitTimeout 
 
 // Mixed-code batches (batch.cu): a work item is up to `count` codewords of
 // one code, listed at order[start .. start+count).
+constexpr int kNumZ = 51;  // lifting sizes of each base graph
 struct WorkItem {
-    int32_t code;   // index into the table array
+    int32_t code;   // index into the table array: BG1 from 0, BG2 from kNumZ
     int32_t start;
     int32_t count;
     int32_t spt;    // sub-rows per thread: Z / spt threads per codeword (1 or 2)
@@ -133,7 +134,8 @@ inline size_t group_smem_bytes(const CodeTable& t, int cpb, uint32_t far) {
 inline int decode_ctas(int threads, size_t smem, size_t smem_sm) {
     return static_cast<int>(std::min<size_t>(65536 / (80 * threads), smem_sm / (smem + 1024)));
 }
-const void* batch_decode_kernel_ptr();
+// classes: one sub-row per thread, and the layout of each base graph's class
+const void* batch_decode_kernel_ptr(bool classes);
 
 // One codeword on a cluster of CTAs (split.cu).  A plan is a head and one
 // table image per rank, contiguous in device memory: which CTA owns which base

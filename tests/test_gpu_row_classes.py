@@ -7,6 +7,7 @@ import pytest
 import torch
 
 from nr_gpu_ldpc_gb300 import Decoder, codes
+from nr_gpu_ldpc_gb300.batch import Batch, make_jobs
 from oracle.oracle import OracleCode
 
 pytestmark = pytest.mark.gpu
@@ -55,3 +56,34 @@ def test_row_classes_against_oracle(gpu, bg, z, change, n):
         opl, _, _ = oc.layered_f32(llr, 2, threads=8)
         np.testing.assert_array_equal(pl.cpu().numpy(), opl)
         dec.close()
+
+
+@pytest.mark.parametrize("spt", [1, 2])
+def test_job_list_of_both_classes_equals_single_code_decodes(gpu, spt):
+    """spt 2 for one code of the list: the whole list takes the kernel for any
+    code."""
+    shapes = [(bg, z) for bg in (1, 2) for z in (2, 7, 56, 208, 384)]
+    per = 160
+    bg = np.repeat([s[0] for s in shapes], per)
+    z = np.repeat([s[1] for s in shapes], per)
+    jobs, n_llr, _, n_out = make_jobs(bg, z)
+    b = Batch(max_jobs=bg.size)
+    b.set_sub_rows_per_thread(2, 56, spt)
+    b.set_jobs(jobs)
+    llr = torch.randn(n_llr, generator=torch.Generator().manual_seed(3)).to(gpu) + 0.9
+    packed = torch.zeros(n_out, dtype=torch.uint8, device=gpu)
+    iters = torch.zeros(bg.size, dtype=torch.int32, device=gpu)
+    b.decode(llr, packed, 6, early_stop=True, iters=iters)
+    torch.cuda.synchronize()
+    for k, (g, size) in enumerate(shapes):
+        dec = Decoder(bg=g, z=size, max_batch=per)
+        at = jobs["llr_offset"][k * per: (k + 1) * per]
+        own = torch.stack([llr[o: o + dec.n_bp] for o in at.tolist()]).contiguous()
+        pk, it = dec.decode(own, 6, early_stop=True, want_iters=True)
+        torch.cuda.synchronize()
+        at = jobs["out_offset"][k * per: (k + 1) * per]
+        got = torch.stack([packed[o: o + dec.packed_bytes] for o in at.tolist()])
+        assert torch.equal(got, pk), (g, size)
+        assert torch.equal(iters[k * per: (k + 1) * per], it), (g, size)
+        dec.close()
+    b.close()
