@@ -36,29 +36,6 @@
 namespace nrldpc {
 namespace {
 
-// What a kernel is compiled for (RowClass): the distance from Lold to Lnew,
-// the degrees that occur (bit d), which of them end in a suffix column (those
-// up to most_sfx; any_sfx of row_update where the class does not say), and the
-// longest row whose Q stay in registers in unweighted flooding.  In both NR
-// base graphs a row's degree tells whether it has a suffix column, so the row
-// bodies have no test for one; together with the fixed distance (each worth
-// about half; BG1 by steps 5.85 -> 5.72 -> 5.39 ms):
-//   us per call                       any code    class
-//   BG1 Z=384, 4,096 codewords, 10 it.    5860     5393
-//   the same, with weights                7400     6832
-//   layered, 6 iterations                 3440     3273
-//   BG1 Z=208, 3,000                      2771     2565
-//   BG2 Z=384, 3,000                      2997     2758
-//   BG2 Z=208, 1,001, early stop           607      563
-struct RowTraits {
-    uint32_t far, degrees;
-    int most_sfx, keep_q;
-};
-__host__ __device__ constexpr RowTraits row_traits(RowClass c) {
-    return c == RowClass::kBg1 ? RowTraits{kFarLong, 0x807f8u, 10, 10}
-         : c == RowClass::kBg2 ? RowTraits{kFarShort, 0x578u, 6, 8}
-                               : RowTraits{0u, 0xffffeu, -1, 10};
-}
 constexpr int kMaxCpb = 48;
 constexpr int kHeaderBytes = 1024;  // mbarrier, group id, per-slot flags
 // Weights of the current iteration in shared memory, one padded row of
@@ -947,6 +924,15 @@ size_t decode_smem_bytes(const CodeTable& tab, int cpb, uint32_t far) {
 // distance and the larger CTA costs no resident one: so for every NR code at
 // the default codewords per CTA (192 < cpb * Z <= 384 but for the smallest Z),
 // while a CTA set to fewer would lose a third to a half of its neighbours.
+// The distance and the known suffix columns are worth about half each (BG1
+// Z=384 5.85 -> 5.72 -> 5.39 ms):
+//   us per call                       any code    class
+//   BG1 Z=384, 4,096 codewords, 10 it.    5860     5393
+//   the same, with weights                7400     6832
+//   layered, 6 iterations                 3440     3273
+//   BG1 Z=208, 3,000                      2771     2565
+//   BG2 Z=384, 3,000                      2997     2758
+//   BG2 Z=208, 1,001, early stop           607      563
 DecodeShape decode_shape(const CodeTable& tab, int cpb, size_t smem_block, size_t smem_sm) {
     DecodeShape d;
     d.cpb = cpb;
@@ -954,18 +940,13 @@ DecodeShape decode_shape(const CodeTable& tab, int cpb, size_t smem_block, size_
     d.smem = decode_smem_bytes(tab, cpb);
     d.kind = 2 * (d.smem + 1024) <= smem_sm ? DecodeKind::kAny2 : DecodeKind::kAny1;
     if (d.kind == DecodeKind::kAny1) return d;
-    const size_t half = static_cast<size_t>(cpb) * tab.core_floats * 4;
-    for (RowClass c : {RowClass::kBg1, RowClass::kBg2}) {
-        const RowTraits t = row_traits(c);
-        const size_t smem = decode_smem_bytes(tab, cpb, t.far);
-        bool fits = half <= t.far && smem <= smem_block &&
-                    decode_ctas(d.threads, smem, smem_sm) >= decode_ctas(d.threads, d.smem, smem_sm);
-        for (int r = 0; r < tab.rows; r++)
-            fits &= (t.degrees >> tab.row_deg[r] & 1) && (tab.row_sfx[r] != 0) == (tab.row_deg[r] <= t.most_sfx);
-        if (!fits) continue;
+    const RowClass c = row_class(tab);
+    const uint32_t far = row_traits(c).far;
+    const size_t smem = decode_smem_bytes(tab, cpb, far);
+    if (c != RowClass::kAny && 4ull * cpb * tab.core_floats <= far && smem <= smem_block &&
+        decode_ctas(d.threads, smem, smem_sm) >= decode_ctas(d.threads, d.smem, smem_sm)) {
         d.kind = c == RowClass::kBg1 ? DecodeKind::kBg1 : DecodeKind::kBg2;
         d.smem = smem;
-        break;
     }
     return d;
 }

@@ -80,8 +80,8 @@ struct DecodeArgs {
     uint32_t extra_tx;
 };
 
-// What decode_kernel is compiled for: any code, or one whose rows are like
-// BG1's or BG2's (decode.cu, row_traits)
+// What the row loops are compiled for: any code, or one whose rows are like
+// BG1's or BG2's (row_traits)
 enum class RowClass { kAny, kBg1, kBg2 };
 // kAny1, kAny2: any code, one or two CTAs per SM in the register budget
 enum class DecodeKind { kAny1, kAny2, kBg1, kBg2 };
@@ -122,6 +122,30 @@ struct BatchDecodeArgs {
 // immediate offset.
 constexpr uint32_t kFarLong = kMaxThreads * 26 * 4;   // BG1's core columns at the most sub-rows per CTA
 constexpr uint32_t kFarShort = kMaxThreads * 14 * 4;  // BG2's
+// What is known of a class: decode_kernel's distance from Lold to Lnew, the
+// degrees that occur (bit d), which of them end in a suffix column (those up
+// to most_sfx), and the longest row whose Q stay in registers in unweighted
+// flooding (decode.cu).  In both NR base graphs a row's degree tells whether
+// it has a suffix column, so the classes' row bodies have no test for one.
+struct RowTraits {
+    uint32_t far, degrees;
+    int most_sfx, keep_q;
+};
+__host__ __device__ constexpr RowTraits row_traits(RowClass c) {
+    return c == RowClass::kBg1 ? RowTraits{kFarLong, 0x807f8u, 10, 10}
+         : c == RowClass::kBg2 ? RowTraits{kFarShort, 0x578u, 6, 8}
+                               : RowTraits{0u, 0xffffeu, -1, 10};
+}
+inline RowClass row_class(const CodeTable& t) {
+    for (RowClass c : {RowClass::kBg1, RowClass::kBg2}) {
+        const RowTraits k = row_traits(c);
+        bool fits = true;
+        for (int r = 0; r < t.rows; r++)
+            fits &= (k.degrees >> t.row_deg[r] & 1) && (t.row_sfx[r] != 0) == (t.row_deg[r] <= k.most_sfx);
+        if (fits) return c;
+    }
+    return RowClass::kAny;
+}
 __host__ __device__ inline uint32_t group_hd_offset(uint32_t half, uint32_t hd, uint32_t far) {
     return far == 0 ? 2 * half : half + hd <= far ? half : far + half;
 }

@@ -149,6 +149,12 @@ __device__ __forceinline__ float wsel(const float4* w, int i) {
     return c == 0 ? v.x : c == 1 ? v.y : c == 2 ? v.z : v.w;
 }
 
+// whether a row of D edges ends in a suffix column
+template <RowClass CLASS>
+__device__ __forceinline__ bool suffix_row(int D, bool any_sfx) {
+    return CLASS == RowClass::kAny ? any_sfx : D <= row_traits(CLASS).most_sfx;
+}
+
 // sfx: the row's last edge is a suffix column, its posterior is st.w (read)
 // and the stored state's w (written); its loss term and seed are taken here.
 // Signs: R_old_i's is bit i of the previous Q signs XOR their parity; Q_i's
@@ -157,12 +163,13 @@ __device__ __forceinline__ float wsel(const float4* w, int i) {
 // D-1-i) and bit-reversed into the stored order (edge i at bit i).
 // l: shared address of the posteriors read; dnew: from there to the ones
 // written.
-template <int D, bool LAYERED>
+template <int D, bool LAYERED, RowClass CLASS>
 __device__ __forceinline__ void fwd_row(const CodeTable& tab, int e0, uint32_t s4, uint32_t z4, uint32_t l,
                                         uint32_t dnew, const float4* w_prev, const float4* w_cur, uint4 st,
-                                        uint4* st_out, bool sfx, bool ybit, float* seed_t, float scale,
+                                        uint4* st_out, bool any_sfx, bool ybit, float* seed_t, float scale,
                                         float* loss) {
     constexpr int LAST = D - 1;
+    const bool sfx = suffix_row<CLASS>(D, any_sfx);
     uint32_t addr[D];
     float lv[D], rold[D];
 #pragma unroll
@@ -235,15 +242,15 @@ __device__ __forceinline__ void fwd_row(const CodeTable& tab, int e0, uint32_t s
         default: break;                                                                          \
     }
 
-template <int MAXD, bool LAYERED>
+template <RowClass CLASS, int MAXD, bool LAYERED>
 __device__ __forceinline__ void fwd_dispatch(int deg, const CodeTable& tab, int e0, uint32_t s4, uint32_t z4,
                                              uint32_t l, uint32_t dnew, const float4* wp, const float4* wc, uint4 st,
                                              uint4* st_out, bool sfx, bool ybit, float* seed_t, float scale,
                                              float* loss) {
 #define NRLDPC_FWD_CASE(D)                                                                         \
     case D:                                                                                        \
-        if constexpr (D <= MAXD)                                                                   \
-            fwd_row<D, LAYERED>(tab, e0, s4, z4, l, dnew, wp, wc, st, st_out, sfx, ybit, seed_t, scale, loss); \
+        if constexpr (D <= MAXD && (row_traits(CLASS).degrees >> D & 1))                           \
+            fwd_row<D, LAYERED, CLASS>(tab, e0, s4, z4, l, dnew, wp, wc, st, st_out, sfx, ybit, seed_t, scale, loss); \
         break;
     NRLDPC_DEG_SWITCH(NRLDPC_FWD_CASE)
 #undef NRLDPC_FWD_CASE
@@ -270,7 +277,7 @@ struct WmsArgs {
 // little at degree 19, the BG2 ones do not).
 constexpr int kWmsMinBlocks = 2;
 
-template <int MAXD, bool LAYERED>
+template <RowClass CLASS, int MAXD, bool LAYERED>
 __global__ void __launch_bounds__(kMaxThreads, kWmsMinBlocks)
     wms_forward_kernel(const __grid_constant__ CodeTable tab, const __grid_constant__ WmsArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -351,7 +358,7 @@ __global__ void __launch_bounds__(kMaxThreads, kWmsMinBlocks)
             for (int r = 0; r < rows; r++) {
                 const uint4 p2 = fetch(r + 2);
                 if (act)
-                    fwd_dispatch<MAXD, LAYERED>(tab.row_deg[r], tab, tab.row_ptr[r], 4u * s, 4u * z, smem_u32(lold),
+                    fwd_dispatch<CLASS, MAXD, LAYERED>(tab.row_deg[r], tab, tab.row_ptr[r], 4u * s, 4u * z, smem_u32(lold),
                                                 smem_u32(lnew) - smem_u32(lold), wrow + r * (kWPad / 4), wrow + (kMaxRows + r) * (kWPad / 4), p0,
                                                 st_cur + r * z + s, tab.row_sfx[r] != 0,
                                                 (ysfx >> r) & 1u, seed_t, a.scale, &loss_part);
@@ -500,10 +507,11 @@ __device__ __forceinline__ void bwd_close(const BwdRow& r, int deg, uint32_t s4,
                         static_cast<uint32_t>(r.i2 < deg ? r.i2 : 31));
 }
 
-template <int D>
+template <int D, RowClass CLASS>
 __device__ __forceinline__ void bwd_row(uint32_t s4, uint32_t z4, bool act, uint32_t gl, uint32_t gl_next,
                                         const uint4* edges, float* gw_acc, uint4 st, uint4 gin,
-                                        uint4* gq_io, bool scatter, bool sfx, float sfx_seed) {
+                                        uint4* gq_io, bool scatter, bool any_sfx, float sfx_seed) {
+    const bool sfx = suffix_row<CLASS>(D, any_sfx);
     BwdRow r = bwd_open(st);
     float gwv[D];
 #pragma unroll
@@ -541,23 +549,23 @@ __device__ __forceinline__ void bwd_long_row(int deg, uint32_t s4, uint32_t z4, 
     bwd_close(r, deg, s4, z4, act, gl_next, edges, gq_io, scatter, sfx);
 }
 
-template <int MAXD>
+template <RowClass CLASS, int MAXD>
 __device__ __forceinline__ void bwd_dispatch(int deg, uint32_t s4, uint32_t z4, bool act, uint32_t gl, uint32_t gln,
                                              const uint4* edges, float* gw_acc, uint4 st, uint4 gin, uint4* gq, bool scatter,
                                              bool sfx, float sfx_seed) {
 #define NRLDPC_BWD_CASE(D)                                                                           \
     case D:                                                                                          \
-        if constexpr (D <= kUnrolled)                                                                \
-            bwd_row<D>(s4, z4, act, gl, gln, edges, gw_acc, st, gin, gq, scatter, sfx, sfx_seed);    \
+        if constexpr (D <= kUnrolled && (row_traits(CLASS).degrees >> D & 1))                        \
+            bwd_row<D, CLASS>(s4, z4, act, gl, gln, edges, gw_acc, st, gin, gq, scatter, sfx, sfx_seed);    \
         break;
     if (MAXD > kUnrolled && deg > kUnrolled)
-        bwd_long_row(deg, s4, z4, act, gl, gln, edges, gw_acc, st, gin, gq, scatter, sfx, sfx_seed);
+        bwd_long_row(deg, s4, z4, act, gl, gln, edges, gw_acc, st, gin, gq, scatter, CLASS == RowClass::kAny && sfx, sfx_seed);
     else
         NRLDPC_DEG_SWITCH(NRLDPC_BWD_CASE)
 #undef NRLDPC_BWD_CASE
 }
 
-template <int MAXD>
+template <RowClass CLASS, int MAXD>
 __global__ void __launch_bounds__(kMaxThreads, kWmsMinBlocks)
     wms_backward_kernel(const __grid_constant__ CodeTable tab, const __grid_constant__ WmsArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -625,7 +633,7 @@ __global__ void __launch_bounds__(kMaxThreads, kWmsMinBlocks)
                     const uint4 sv = act ? ring_st[k] : make_uint4(0u, 0u, 31u << 5, 0u);
                     const uint4 gv = act ? ring_gq[k] : make_uint4(0u, 0u, 31u, 31u);
                     const float sd = (act && tab.row_sfx[r]) ? ring_sd[k] : 0.0f;
-                    bwd_dispatch<MAXD>(tab.row_deg[r], 4u * s, 4u * z, act, smem_u32(gl), smem_u32(gln),
+                    bwd_dispatch<CLASS, MAXD>(tab.row_deg[r], 4u * s, 4u * z, act, smem_u32(gl), smem_u32(gln),
                                        edges + tab.row_ptr[r], gw_acc + tab.row_ptr[r], sv, gv,
                                        gq + r * z + s, t > 0, tab.row_sfx[r] != 0, sd);
                 }
@@ -651,7 +659,7 @@ __global__ void __launch_bounds__(kMaxThreads, kWmsMinBlocks)
                     uint4 s2, g2;
                     float d2;
                     fetch(r + 2, s2, g2, d2);
-                    bwd_dispatch<MAXD>(tab.row_deg[r], 4u * s, 4u * z, act, smem_u32(gl), smem_u32(gln),
+                    bwd_dispatch<CLASS, MAXD>(tab.row_deg[r], 4u * s, 4u * z, act, smem_u32(gl), smem_u32(gln),
                                        edges + tab.row_ptr[r], gw_acc + tab.row_ptr[r], s0, g0,
                                        gq + r * z + s, t > 0, tab.row_sfx[r] != 0, d0);
                     s0 = s1;
@@ -698,10 +706,11 @@ __device__ __forceinline__ void bwd_layered_close(const BwdRow& r, int deg, uint
 // h_row: shared address of the row's staged dloss/dR (edge i h_step bytes on).
 // dloss/dR^{t-1} = -dloss/dQ goes out edge by edge as if no edge were an
 // argmin; the two that are follow.
-template <int D>
+template <int D, RowClass CLASS>
 __device__ __forceinline__ void bwd_layered_row(uint32_t s4, uint32_t z4, bool act, uint32_t g, const uint4* edges,
                                                 float* gw_acc, uint4 st, uint32_t h_row, uint32_t h_step,
-                                                float* gh_row, bool write_h, bool sfx, float sfx_seed) {
+                                                float* gh_row, bool write_h, bool any_sfx, float sfx_seed) {
+    const bool sfx = suffix_row<CLASS>(D, any_sfx);
     const int z = static_cast<int>(z4 / 4);
     BwdRow r = bwd_open(st);
     float gwv[D], ga_last = 0.0f;
@@ -751,24 +760,25 @@ __device__ __forceinline__ void bwd_layered_long_row(int deg, uint32_t s4, uint3
     bwd_layered_close(r, deg, s4, z4, act, g, edges, gh_row, write_h, sfx, ga_last);
 }
 
-template <int MAXD>
+template <RowClass CLASS, int MAXD>
 __device__ __forceinline__ void bwd_layered_dispatch(int deg, uint32_t s4, uint32_t z4, bool act, uint32_t g,
                                                      const uint4* edges, float* gw_acc, uint4 st, uint32_t h_row,
                                                      uint32_t h_step, float* gh_row, bool has_h, bool write_h,
                                                      bool sfx, float sfx_seed) {
 #define NRLDPC_BWDL_CASE(D)                                                                                 \
     case D:                                                                                                 \
-        if constexpr (D <= kUnrolled)                                                                         \
-            bwd_layered_row<D>(s4, z4, act, g, edges, gw_acc, st, h_row, h_step, gh_row, write_h, sfx, sfx_seed); \
+        if constexpr (D <= kUnrolled && (row_traits(CLASS).degrees >> D & 1))                                 \
+            bwd_layered_row<D, CLASS>(s4, z4, act, g, edges, gw_acc, st, h_row, h_step, gh_row, write_h, sfx, sfx_seed); \
         break;
     if (MAXD > kUnrolled && deg > kUnrolled)
-        bwd_layered_long_row(deg, s4, z4, act, g, edges, gw_acc, st, gh_row, has_h, write_h, sfx, sfx_seed);
+        bwd_layered_long_row(deg, s4, z4, act, g, edges, gw_acc, st, gh_row, has_h, write_h,
+                             CLASS == RowClass::kAny && sfx, sfx_seed);
     else
         NRLDPC_DEG_SWITCH(NRLDPC_BWDL_CASE)
 #undef NRLDPC_BWDL_CASE
 }
 
-template <int MAXD>
+template <RowClass CLASS, int MAXD>
 __global__ void __launch_bounds__(kMaxThreads, kWmsMinBlocks)
     wms_backward_layered_kernel(const __grid_constant__ CodeTable tab, const __grid_constant__ WmsArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -836,7 +846,7 @@ __global__ void __launch_bounds__(kMaxThreads, kWmsMinBlocks)
                 cp_async_wait<1>();  // this thread's copies of row r have landed
                 const uint32_t h_row = ring + (r & 1) * (kUnrolled + 1) * h_step;
                 const float sd = tab.row_sfx[r] ? lds(h_row + kUnrolled * h_step) : 0.0f;
-                bwd_layered_dispatch<MAXD>(tab.row_deg[r], 4u * s, 4u * z, act, smem_u32(g), edges + tab.row_ptr[r],
+                bwd_layered_dispatch<CLASS, MAXD>(tab.row_deg[r], 4u * s, 4u * z, act, smem_u32(g), edges + tab.row_ptr[r],
                                            gw_acc + tab.row_ptr[r], staged_st[(r & 1) * blockDim.x], h_row, h_step,
                                            gh + static_cast<size_t>(tab.row_ptr[r]) * z + s, act && t < a.T - 1, t > 0,
                                            tab.row_sfx[r] != 0, sd);
@@ -892,17 +902,26 @@ size_t wms_smem_bytes(const CodeTable& tab, int cpb, bool layered) {
 namespace {
 // kernel k of the degree class: 0 forward flooding, 1 forward layered,
 // 2 adjoint flooding, 3 adjoint layered
-template <int MAXD>
+template <RowClass CLASS, int MAXD>
 const void* wms_kernel(int k) {
     switch (k) {
-        case 0: return reinterpret_cast<const void*>(&wms_forward_kernel<MAXD, false>);
-        case 1: return reinterpret_cast<const void*>(&wms_forward_kernel<MAXD, true>);
-        case 2: return reinterpret_cast<const void*>(&wms_backward_kernel<MAXD>);
-        default: return reinterpret_cast<const void*>(&wms_backward_layered_kernel<MAXD>);
+        case 0: return reinterpret_cast<const void*>(&wms_forward_kernel<CLASS, MAXD, false>);
+        case 1: return reinterpret_cast<const void*>(&wms_forward_kernel<CLASS, MAXD, true>);
+        case 2: return reinterpret_cast<const void*>(&wms_backward_kernel<CLASS, MAXD>);
+        default: return reinterpret_cast<const void*>(&wms_backward_layered_kernel<CLASS, MAXD>);
     }
 }
+// The kernels for the code's class of rows (forward and adjoint, us: BG2 Z=128
+// 4,096 codewords x 8 it. flooding 3481 -> 3343, BG1 Z=384 512 x 6 layered 1946
+// -> 1880), but BG1's flooding adjoint, whose compiled form for the class is
+// slower: BG1 Z=384 1,000 x 6 it. 2973 with the general kernels, 3287 with the
+// class's, 2952 with its forward and the general adjoint.
 const void* wms_kernel_for(const CodeTable& tab, int k) {
-    return max_row_degree(tab) <= 10 ? wms_kernel<10>(k) : wms_kernel<19>(k);
+    switch (row_class(tab)) {
+        case RowClass::kBg1: return k == 2 ? wms_kernel<RowClass::kAny, 19>(k) : wms_kernel<RowClass::kBg1, 19>(k);
+        case RowClass::kBg2: return wms_kernel<RowClass::kBg2, 10>(k);
+        default: return max_row_degree(tab) <= 10 ? wms_kernel<RowClass::kAny, 10>(k) : wms_kernel<RowClass::kAny, 19>(k);
+    }
 }
 }  // namespace
 
