@@ -163,9 +163,8 @@ __device__ __forceinline__ uint32_t lds_u8(uint32_t a) {
 // form measured fastest for its kernels).
 // LAYERED (no reference counterpart): one posterior buffer updated in place,
 // A = Q + R_new (dnew = 0), instead of Lnew += R_new - R_old.
-// kKeepQ (layered, and unweighted flooding of codes with longer rows for their
-// rows of up to kKeepQMax edges; the kernels for shorter codes are 4% slower
-// with it): Q stays in registers, so the edge that gets min2 is found in the
+// kKeepQ (layered, and unweighted flooding for rows of up to the class's
+// keep_q edges): Q stays in registers, so the edge that gets min2 is found in the
 // second half as any edge with |Q| == min1 -- the first argmin when the
 // minimum is unique, and when it is not, min2 == min1 and every such edge
 // gets the same message -- and the two minima are taken two edges at a time
@@ -277,7 +276,7 @@ __device__ __forceinline__ void row_update(const CodeTable& tab, int e0, bool an
         // Lnew read-modify-write with the loads kPipe edges ahead of the stores
         // (fewer live registers than loading the whole row first); the
         // suffix edge adds to the exact suffix posterior
-        constexpr int kPipe = 4;
+        constexpr int kPipe = row_traits(CLASS).ahead;
         float nv[D];
 #pragma unroll
         for (int i = 0; i < kPipe && i < D; i++)
@@ -897,9 +896,10 @@ __global__ void __launch_bounds__(kMaxThreads, 2)
                                                         buf0, hd0, s_fail, st_base, a.llr + job.llr_offset, out,
                                                         a.n_iter, a.early_stop, a.alpha, nullptr, nullptr, 1);
             else
-                run_group<false, false, RowClass::kBg2>(tab, cpb, slot, s, static_cast<uint32_t>(tpc), !valid_thread,
-                                                        buf0, hd0, s_fail, st_base, a.llr + job.llr_offset, out,
-                                                        a.n_iter, a.early_stop, a.alpha, nullptr, nullptr, 1);
+                run_group<false, false, RowClass::kBg2Mixed>(tab, cpb, slot, s, static_cast<uint32_t>(tpc), !valid_thread,
+                                                             buf0, hd0, s_fail, st_base, a.llr + job.llr_offset,
+                                                             out, a.n_iter, a.early_stop, a.alpha, nullptr,
+                                                             nullptr, 1);
         } else if (item.spt == 2) {
             run_group<false, false, RowClass::kAny, 2>(tab, cpb, slot, s, static_cast<uint32_t>(tpc), !valid_thread,
                                                        buf0, hd0, s_fail, st_base, a.llr + job.llr_offset, out,

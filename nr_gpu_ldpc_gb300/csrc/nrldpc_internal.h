@@ -81,8 +81,9 @@ struct DecodeArgs {
 };
 
 // What the row loops are compiled for: any code, or one whose rows are like
-// BG1's or BG2's (row_traits)
-enum class RowClass { kAny, kBg1, kBg2 };
+// BG1's or BG2's (row_traits); kBg2Mixed: BG2's in a kernel that also holds
+// BG1's
+enum class RowClass { kAny, kBg1, kBg2, kBg2Mixed };
 // kAny1, kAny2: any code, one or two CTAs per SM in the register budget
 enum class DecodeKind { kAny1, kAny2, kBg1, kBg2 };
 enum DeviceError : int { kErrNone = 0, kErrLlrLoadTimeout = 1, kErrSplitTimeout = 2 };
@@ -124,17 +125,22 @@ constexpr uint32_t kFarLong = kMaxThreads * 26 * 4;   // BG1's core columns at t
 constexpr uint32_t kFarShort = kMaxThreads * 14 * 4;  // BG2's
 // What is known of a class: decode_kernel's distance from Lold to Lnew, the
 // degrees that occur (bit d), which of them end in a suffix column (those up
-// to most_sfx), and the longest row whose Q stay in registers in unweighted
-// flooding (decode.cu).  In both NR base graphs a row's degree tells whether
-// it has a suffix column, so the classes' row bodies have no test for one.
+// to most_sfx), the longest row whose Q stay in registers in unweighted
+// flooding, and how many edges ahead of the store Lnew is read.  In both NR
+// base graphs a row's degree tells whether it has a suffix column, so the
+// classes' row bodies have no test for one.  BG2's kernels have the registers
+// to read a whole row of Lnew first (2.9% over 15 sizes, BG2 Z=208 1,001
+// codewords 563 -> 549 us, Z=256 with early stop 1% slower); the job lists'
+// kernel, whose registers BG1's rows take, is 1.4% slower with it.
 struct RowTraits {
     uint32_t far, degrees;
-    int most_sfx, keep_q;
+    int most_sfx, keep_q, ahead;
 };
 __host__ __device__ constexpr RowTraits row_traits(RowClass c) {
-    return c == RowClass::kBg1 ? RowTraits{kFarLong, 0x807f8u, 10, 10}
-         : c == RowClass::kBg2 ? RowTraits{kFarShort, 0x578u, 6, 8}
-                               : RowTraits{0u, 0xffffeu, -1, 10};
+    return c == RowClass::kBg1        ? RowTraits{kFarLong, 0x807f8u, 10, 10, 4}
+           : c == RowClass::kBg2      ? RowTraits{kFarShort, 0x578u, 6, 10, 10}
+           : c == RowClass::kBg2Mixed ? RowTraits{kFarShort, 0x578u, 6, 8, 4}
+                                      : RowTraits{0u, 0xffffeu, -1, 10, 4};
 }
 inline RowClass row_class(const CodeTable& t) {
     for (RowClass c : {RowClass::kBg1, RowClass::kBg2}) {
