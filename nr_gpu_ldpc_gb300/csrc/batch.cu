@@ -155,6 +155,7 @@ __global__ void __launch_bounds__(256) batch_gen_kernel(const __grid_constant__ 
 struct DerateArgs {
     const CodeTable* tables;
     const JobDev* jobs;
+    const int32_t* order;  // largest codes first
     const float* llr_e;
     float* llr;
     int n_jobs, parts, part;
@@ -162,25 +163,44 @@ struct DerateArgs {
 
 // Each job's output in `parts` parts of `part` positions or interleaver rows,
 // one CTA per (job, part) at a time: as many parts as it takes for a few jobs
-// to fill the GPU, one where the jobs do (nrldpc_batch_set_jobs).  Without repetition (e <= Nc) every bit k lands at one position of the
-// compressed buffer: a thread takes one interleaver row, reads its qm
+// to fill the GPU, one where the jobs do (nrldpc_batch_set_jobs); the largest
+// jobs first and every other round of CTAs backwards, so that the CTAs' shares
+// differ little.  Not interleaved and without repetition (e <= Nc): the output
+// in order, four positions a store, each position's LLR, zero or filler looked
+// up.  Interleaved: a thread takes one interleaver row, reads its qm
 // neighbouring LLRs (bits i, i + E/qm, ...) and writes each beside its
-// neighbours' -- reads and writes both in order, no division per bit.  With
-// repetition each position c collects bits k = k_first, k_first + Nc, ... in
-// order, the first copy taken as is, later ones added.  Bound by memory: one
-// CTA per job with a division chain per position took 29 us for 26 blocks of
-// BG1 Z=384 and 286 us for the 8,192-codeword mix (0.85 GB).
+// neighbours' -- no division per bit.  With repetition each position c
+// collects bits k = k_first, k_first + Nc, ... in order, the first copy taken
+// as is, later ones added.  Bound by the writes: the 8,192-codeword mix (0.40
+// GB written, 0.23 read) takes 154 us without its reads, 190 with them; in
+// input order, four bytes a store, it took 257, 1,000 codewords 73 (now 24).
 
 __global__ void __launch_bounds__(256) batch_derate_kernel(const __grid_constant__ DerateArgs a) {
     const float inf = __int_as_float(0x7f800000);
-    for (long w = blockIdx.x; w < static_cast<long>(a.n_jobs) * a.parts; w += gridDim.x) {
-        const int job = static_cast<int>(w / a.parts), from = static_cast<int>(w - static_cast<long>(job) * a.parts) * a.part;
-        const JobDev jb = a.jobs[job];
+    const long n_work = static_cast<long>(a.n_jobs) * a.parts;
+    for (long base = 0, back = 0; base < n_work; base += gridDim.x, back ^= 1) {
+        const long w = base + (back ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
+        if (w >= n_work) continue;
+        const int at = static_cast<int>(w / a.parts), from = static_cast<int>(w - static_cast<long>(at) * a.parts) * a.part;
+        const JobDev jb = a.jobs[a.order[at]];
         const int z = a.tables[jb.code].z, n = a.tables[jb.code].n_bp, K = a.tables[jb.code].kb * z, ncb = n - 2 * z;
         const int f0 = jb.k_prime - 2 * z, nf = K - jb.k_prime, nc = ncb - nf;
         const int c0 = jb.k0 < f0 ? jb.k0 : (jb.k0 < f0 + nf ? f0 : jb.k0 - nf);
         float* out = a.llr + jb.llr_offset;
         const float* in = a.llr_e + jb.e_offset;
+        if (jb.qm == 1 && jb.e <= nc && reinterpret_cast<uintptr_t>(out) % 16 == 0) {
+            auto value = [&](int j) {  // of position j of the mother codeword
+                if (j < 2 * z) return 0.0f;
+                if (j >= jb.k_prime && j < K) return inf;
+                int k = j - 2 * z - (j < K ? 0 : nf) - c0;
+                if (k < 0) k += nc;
+                return k < jb.e ? __ldcs(in + k) : 0.0f;
+            };
+            const int to = min(n, from + a.part);  // a multiple of 4, as 52 Z and 68 Z are
+            for (int j = from + 4 * threadIdx.x; j < to; j += 4 * blockDim.x)
+                *reinterpret_cast<float4*>(out + j) = make_float4(value(j), value(j + 1), value(j + 2), value(j + 3));
+            continue;
+        }
         if (from == 0) {
             for (int j = threadIdx.x; j < 2 * z; j += blockDim.x) out[j] = 0.0f;
             for (int j = jb.k_prime + threadIdx.x; j < K; j += blockDim.x) out[j] = inf;
@@ -569,7 +589,7 @@ int nrldpc_batch_set_jobs(nrldpc_batch* batch, const nrldpc_job* jobs, int n_job
         d.out_offset = j.out_offset;
         order[i] = i;
         const int nc = ncb - (K - kp);  // positions a bit can land on
-        longest = std::max(longest, e <= nc ? std::max(e / qm, nc - e) : nc);
+        longest = std::max(longest, e > nc ? nc : qm == 1 ? t.n_bp : std::max(e / qm, nc - e));
     }
     // eight CTAs per SM, in parts of at least 256 positions
     b->derate_part = std::max(256, (longest * static_cast<int>(std::min(n_jobs, 8 * b->sm_count)) / (8 * b->sm_count) + 255) / 256 * 256);
@@ -661,7 +681,7 @@ int nrldpc_batch_derate(nrldpc_batch* batch, const float* d_llr_e, float* d_llr,
     Batch* b = reinterpret_cast<Batch*>(batch);
     if (!b || !d_llr_e || !d_llr) return NRLDPC_ERR_INVALID_ARG;
     if (b->n_jobs == 0) return NRLDPC_OK;
-    DerateArgs a{b->d_tables, b->d_jobs_rm, d_llr_e, d_llr, b->n_jobs, b->derate_parts, b->derate_part};
+    DerateArgs a{b->d_tables, b->d_jobs_rm, b->d_order, d_llr_e, d_llr, b->n_jobs, b->derate_parts, b->derate_part};
     const int grid = static_cast<int>(std::min<long>(static_cast<long>(b->n_jobs) * b->derate_parts, 8L * b->sm_count));
     batch_derate_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(a);
     return map_cuda(cudaGetLastError());
