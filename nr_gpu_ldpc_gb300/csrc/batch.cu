@@ -269,6 +269,7 @@ __global__ void __launch_bounds__(256) batch_count_kernel(const __grid_constant_
 }
 
 struct Batch {
+    InFlight in_flight;
     int device = 0;
     float alpha = 0.75f;
     int max_jobs = 0;
@@ -352,6 +353,7 @@ void drop_graph(Batch* b) {
 
 void free_batch(Batch* b) {
     if (!b) return;
+    in_flight_leave(&b->in_flight);
     drop_graph(b);
     cudaFree(b->d_tables);
     cudaFree(b->d_plans);
@@ -506,6 +508,10 @@ int nrldpc_batch_create(int device, int max_jobs, float alpha, nrldpc_batch** ou
         cudaFuncSetAttribute(batch_decode_kernel_ptr(true), cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(b->smem_optin)) ||
         split_kernel_attributes(b->smem_optin)) {
+        free_batch(b);
+        return NRLDPC_ERR_CUDA;
+    }
+    if (!in_flight_join(&b->in_flight, device)) {
         free_batch(b);
         return NRLDPC_ERR_CUDA;
     }
@@ -705,7 +711,12 @@ int nrldpc_batch_decode(nrldpc_batch* batch, const float* d_llr, uint8_t* d_pack
     if (b->n_jobs == 0) return NRLDPC_OK;
     if (!d_llr || !d_packed) return NRLDPC_ERR_INVALID_ARG;
     if (reinterpret_cast<uintptr_t>(d_llr) % 16 != 0) return NRLDPC_ERR_ALIGNMENT;
-    if (b->split.ranks) {
+    // clusters while they and those of as many lists like this one as other
+    // decoders are busy have the GPU's SMs, the queue kernel else
+    if (b->split.ranks &&
+        static_cast<long>(b->n_jobs) * b->split.ranks *
+                in_flight_others(&b->in_flight, reinterpret_cast<cudaStream_t>(stream),
+                                 static_cast<long>(b->n_jobs) * b->split.ranks, b->sm_count) <= b->sm_count) {
         SplitArgs a{};
         a.plan = b->d_plans_split;
         a.jobs = b->d_split;
@@ -717,7 +728,10 @@ int nrldpc_batch_decode(nrldpc_batch* batch, const float* d_llr, uint8_t* d_pack
         a.n_iter = n_iter;
         a.early_stop = early_stop;
         a.alpha = b->alpha;
-        return map_cuda(launch_split(b->split, a, nullptr, b->split_clusters, reinterpret_cast<cudaStream_t>(stream)));
+        const int rc =
+            map_cuda(launch_split(b->split, a, nullptr, b->split_clusters, reinterpret_cast<cudaStream_t>(stream)));
+        in_flight_note(&b->in_flight, reinterpret_cast<cudaStream_t>(stream));
+        return rc;
     }
     BatchDecodeArgs& k = b->kargs;
     k.tables = b->d_tables;
@@ -759,7 +773,9 @@ int nrldpc_batch_decode(nrldpc_batch* batch, const float* d_llr, uint8_t* d_pack
     } else if (cudaGraphExecKernelNodeSetParams(b->exec, b->knode, &kp) != cudaSuccess) {
         return NRLDPC_ERR_CUDA;
     }
-    return map_cuda(cudaGraphLaunch(b->exec, reinterpret_cast<cudaStream_t>(stream)));
+    const int rc = map_cuda(cudaGraphLaunch(b->exec, reinterpret_cast<cudaStream_t>(stream)));
+    in_flight_note(&b->in_flight, reinterpret_cast<cudaStream_t>(stream));
+    return rc;
 }
 
 }  // extern "C"

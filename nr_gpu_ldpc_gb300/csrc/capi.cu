@@ -7,11 +7,74 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <vector>
 
 #include "../../include/nr_gpu_ldpc_gb300.h"
 #include "nrldpc_internal.h"
+
+namespace nrldpc {
+namespace {
+std::mutex g_in_flight_mu;
+std::vector<InFlight*> g_in_flight;  // one per live handle
+int g_crowd[64];                     // per device: the last count, falling
+}  // namespace
+
+bool in_flight_join(InFlight* me, int device) {
+    if (cudaEventCreateWithFlags(&me->done, cudaEventDisableTiming) != cudaSuccess) return false;
+    me->device = device;
+    std::lock_guard<std::mutex> lock(g_in_flight_mu);
+    g_in_flight.push_back(me);
+    return true;
+}
+
+void in_flight_leave(InFlight* me) {
+    if (!me->done) return;
+    {
+        std::lock_guard<std::mutex> lock(g_in_flight_mu);
+        g_in_flight.erase(std::remove(g_in_flight.begin(), g_in_flight.end(), me), g_in_flight.end());
+    }
+    cudaEventDestroy(me->done);
+}
+
+int in_flight_others(const InFlight* me, cudaStream_t stream, long sms, int sm_count) {
+    std::lock_guard<std::mutex> lock(g_in_flight_mu);
+    if (g_in_flight.size() < 2 || sms * static_cast<long>(g_in_flight.size()) <= sm_count) return 0;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return 0;
+    }
+    // a query must not disturb a capture of another thread
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    int busy = 0;
+    for (InFlight* f : g_in_flight) {
+        if (f == me || f->device != me->device || !f->recorded || f->stream == stream) continue;
+        if (cudaEventQuery(f->done) == cudaErrorNotReady)
+            busy++;
+        else
+            f->recorded = false;
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (busy) cudaGetLastError();  // not-ready is no error of the caller's
+    int& crowd = g_crowd[me->device & 63];
+    crowd = std::min(std::max(busy, crowd - 1), static_cast<int>(g_in_flight.size()) - 1);
+    return crowd;
+}
+
+void in_flight_note(InFlight* me, cudaStream_t stream) {
+    std::lock_guard<std::mutex> lock(g_in_flight_mu);
+    if (g_in_flight.size() < 2) return;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone &&
+        cudaEventRecord(me->done, stream) == cudaSuccess)
+        me->recorded = true, me->stream = stream;
+    else
+        cudaGetLastError();
+}
+}  // namespace nrldpc
 
 using namespace nrldpc;
 
@@ -30,6 +93,7 @@ constexpr size_t kDirectMaxRounds = 4;
 
 struct Handle {
     int device = 0;
+    InFlight in_flight;
     CodeTable tab{};
     EncodePlan plan{};
     bool plan_ok = false;
@@ -156,6 +220,7 @@ int base_matrix_impl(int bg, int ils, int* out, int* rows, int* cols) {
 
 void free_handle(Handle* h) {
     if (!h) return;
+    in_flight_leave(&h->in_flight);
     cudaFree(h->state);
     cudaFree(h->state2);
     cudaFree(h->scratch);
@@ -306,6 +371,10 @@ int init_impl(const int* base, int rows, int cols, int kb, const nrldpc_config* 
             free_handle(h);
             return NRLDPC_ERR_CUDA;
         }
+    if (!in_flight_join(&h->in_flight, cfg->device)) {
+        free_handle(h);
+        return NRLDPC_ERR_CUDA;
+    }
     *out = reinterpret_cast<nrldpc_handle*>(h);
     return NRLDPC_OK;
 }
@@ -323,7 +392,14 @@ int decode_impl(Handle* h, const float* llr, uint8_t* packed, int n_cw, int n_it
     if (n_cw > h->max_batch) return NRLDPC_ERR_TOO_LARGE;
     if (reinterpret_cast<uintptr_t>(llr) % 16 != 0) return NRLDPC_ERR_ALIGNMENT;
     if (weighted && (!h->weights || h->n_w_iters < 1)) return NRLDPC_ERR_INVALID_ARG;
-    const int plan = (h->schedule == NRLDPC_SCHEDULE_FLOODING && extra_tx == 0) ? split_choice(h, n_cw) : -1;
+    int plan = (h->schedule == NRLDPC_SCHEDULE_FLOODING && extra_tx == 0) ? split_choice(h, n_cw) : -1;
+    // six streams of 40 codewords of BG1 Z=384, 5 iterations, from host memory:
+    // 0.56 ms a round with every batch spread, 0.33 with this count (0.35 with
+    // decode_kernel alone)
+    if (plan >= 0)
+        if (const int busy = in_flight_others(&h->in_flight, stream, static_cast<long>(n_cw) * h->split[plan].ranks,
+                                              h->sm_count))
+            plan = split_choice(h, static_cast<int>(std::min<long>(n_cw * (1L + busy), 1 << 24)));
     if (plan >= 0) {
         SplitArgs a{};
         a.head = h->split[plan];
@@ -339,8 +415,10 @@ int decode_impl(Handle* h, const float* llr, uint8_t* packed, int n_cw, int n_it
         a.early_stop = early;
         a.llr_from_host = llr_from_host ? 1 : 0;
         a.alpha = h->alpha;
-        return map_cuda(launch_split(h->split[plan], a, weighted ? h->weights : nullptr,
-                                     std::min(n_cw, h->split_room[plan]), stream));
+        const int rc = map_cuda(launch_split(h->split[plan], a, weighted ? h->weights : nullptr,
+                                             std::min(n_cw, h->split_room[plan]), stream));
+        in_flight_note(&h->in_flight, stream);
+        return rc;
     }
     DecodeArgs a{};
     a.llr = llr;
@@ -362,8 +440,10 @@ int decode_impl(Handle* h, const float* llr, uint8_t* packed, int n_cw, int n_it
     a.extra_tx = extra_tx;
     const int grid = std::min(a.n_groups, h->max_grid);
     if (!counter && cudaMemsetAsync(h->scratch, 0, sizeof(int), stream) != cudaSuccess) return NRLDPC_ERR_CUDA;
-    return map_cuda(launch_decode(h->tab, a, weighted ? h->weights : nullptr, grid, h->threads, h->smem,
-                                  h->schedule == NRLDPC_SCHEDULE_LAYERED, h->kind, stream));
+    const int rc = map_cuda(launch_decode(h->tab, a, weighted ? h->weights : nullptr, grid, h->threads, h->smem,
+                                          h->schedule == NRLDPC_SCHEDULE_LAYERED, h->kind, stream));
+    if (!counter) in_flight_note(&h->in_flight, stream);
+    return rc;
 }
 
 // Host-buffer decode (fp32 LLRs, or narrow ones widened on the GPU: qtype 1

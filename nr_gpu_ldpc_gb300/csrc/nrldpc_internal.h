@@ -229,6 +229,25 @@ int split_max_clusters(const SplitHead& head);  // resident at once
 cudaError_t launch_split(const SplitHead& head, const SplitArgs& args, const WeightTable* weights, int n_clusters,
                          cudaStream_t stream);
 
+// Live decoders of the process and whether their last call is still running.
+// A small batch spread over the whole GPU is the fastest alone but takes about
+// twice the SM time of decode_kernel, so the choice counts the other decoders
+// of the device that are busy on other streams as as many batches like its
+// own.  The first call of a round sees the others idle, so the count falls by
+// one a call at most (a hint: either choice gives the same bits).
+struct InFlight {
+    int device = -1;
+    cudaEvent_t done = nullptr;  // after the last call
+    cudaStream_t stream = nullptr;
+    bool recorded = false;
+};
+bool in_flight_join(InFlight* me, int device);
+void in_flight_leave(InFlight* me);
+// Busy ones beside `me`; 0 while the stream is captured, and where as many
+// calls of `sms` SMs as there are decoders fit the GPU's.
+int in_flight_others(const InFlight* me, cudaStream_t stream, long sms, int sm_count);
+void in_flight_note(InFlight* me, cudaStream_t stream);  // after a call's launches
+
 // Host-side launchers (decode.cu / channel.cu).
 // kind: which kernels serve a code and geometry (decode_shape).
 // weights: null for the plain decoder; layered: row-sequential schedule (no
