@@ -264,8 +264,10 @@ int split_prepare(Handle* h, size_t smem_limit, std::vector<unsigned char>* byte
 // early stop, us (model): BG1 Z=384 on 16 / 10 / 4 / 3 CTAs 43 / 52 / 95 / 148
 // (47 / 57 / 98 / 150), BG2 Z=384 on 16 / 4 / 3 40 / 72 / 89 (42 / 80 / 96),
 // BG1 Z=96 on 4 / 2 / 1 CTAs 42 / 59 / 80 (47 / 64 / 98); decode_kernel at one
-// CTA per SM BG1 Z=384 / 208 / 96 299 / 245 / 204 (300 / 248 / 207), BG2 Z=384 /
-// 128 219 / 157, two CTAs per SM 1.5-1.65 times that.
+// CTA per SM BG1 Z=384 / 208 276 / 227 (295 / 244), BG2 Z=384 188 (216), two
+// CTAs per SM 1.4-1.6 times that.  Both estimates are high, by about as much:
+// with decode_kernel's alone brought down to its times, 13 of 112 sizes tried
+// changed sides and every one got slower (1.08-1.55 times).
 long fused_cost(const Handle* h, int n) {
     const long groups = (n + h->cpb - 1) / h->cpb, one = fused_row_walk(h->tab, h->threads / 32);
     long cost = groups / h->max_grid * (one * (4 + 2 * h->ctas_per_sm) / 5);
