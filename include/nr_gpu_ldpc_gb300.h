@@ -338,6 +338,17 @@ int nrldpc_device_error(nrldpc_handle* h);
 int nrldpc_selftest_wait_timeout(nrldpc_handle* h, const float* d_llr, uint8_t* d_packed, int n_cw,
                                  nrldpc_stream_t stream);
 
+/* The same for the waits of the small-batch decoder (one codeword on a cluster
+ * of CTAs that count the bytes they send each other): the first CTA of every
+ * cluster is told to expect 16 bytes more than are sent, with a short wait
+ * limit.  Every store that is sent arrives; the first CTA's wait runs out, then
+ * those of the CTAs that wait for it, the kernel records the timeout and each
+ * cluster leaves without writing d_packed.  Waits for the stream.
+ * NRLDPC_ERR_BAD_CONFIG for a code that has no such clusters.  The handle
+ * stays usable. */
+int nrldpc_selftest_split_timeout(nrldpc_handle* h, const float* d_llr, uint8_t* d_packed, int n_cw,
+                                  nrldpc_stream_t stream);
+
 const char* nrldpc_status_string(int status);
 
 #ifdef __cplusplus

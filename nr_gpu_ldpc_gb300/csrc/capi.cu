@@ -290,6 +290,19 @@ int split_choice(const Handle* h, int n) {
     return best;
 }
 
+SplitArgs split_args(const Handle* h, int plan, const float* llr, uint8_t* packed, int n_cw, int n_iter) {
+    SplitArgs a{};
+    a.head = h->split[plan];
+    a.plan = reinterpret_cast<const unsigned char*>(h->scratch) + h->split_at[plan];
+    a.llr = llr;
+    a.packed = packed;
+    a.error_flag = h->scratch + 1;
+    a.n_cw = n_cw;
+    a.n_iter = n_iter;
+    a.alpha = h->alpha;
+    return a;
+}
+
 int init_impl(const int* base, int rows, int cols, int kb, const nrldpc_config* cfg,
               nrldpc_handle** out) {
     if (!cfg || !out || cfg->max_batch < 1 || !(cfg->alpha > 0.0f) || cfg->cw_per_cta < 0)
@@ -403,20 +416,12 @@ int decode_impl(Handle* h, const float* llr, uint8_t* packed, int n_cw, int n_it
                                               h->sm_count))
             plan = split_choice(h, static_cast<int>(std::min<long>(n_cw * (1L + busy), 1 << 24)));
     if (plan >= 0) {
-        SplitArgs a{};
-        a.head = h->split[plan];
-        a.plan = reinterpret_cast<const unsigned char*>(h->scratch) + h->split_at[plan];
-        a.llr = llr;
-        a.packed = packed;
+        SplitArgs a = split_args(h, plan, llr, packed, n_cw, n_iter);
         a.app = app;
         a.iters = iters;
-        a.error_flag = h->scratch + 1;
-        a.n_cw = n_cw;
-        a.n_iter = n_iter;
         a.n_w_iters = h->n_w_iters;
         a.early_stop = early;
         a.llr_from_host = llr_from_host ? 1 : 0;
-        a.alpha = h->alpha;
         const int rc = map_cuda(launch_split(h->split[plan], a, weighted ? h->weights : nullptr,
                                              std::min(n_cw, h->split_room[plan]), stream));
         in_flight_note(&h->in_flight, stream);
@@ -680,6 +685,23 @@ int nrldpc_selftest_wait_timeout(nrldpc_handle* handle, const float* d_llr, uint
     // 16 bytes more than the copies deliver, 1024 wait iterations
     return decode_impl(reinterpret_cast<Handle*>(handle), d_llr, d_packed, n_cw, 1, 0, nullptr, nullptr, false,
                        reinterpret_cast<cudaStream_t>(stream), false, nullptr, nullptr, 1024, 16);
+}
+
+int nrldpc_selftest_split_timeout(nrldpc_handle* handle, const float* d_llr, uint8_t* d_packed, int n_cw,
+                                  nrldpc_stream_t stream) {
+    Handle* h = reinterpret_cast<Handle*>(handle);
+    if (!h || !d_llr || !d_packed || n_cw < 1) return NRLDPC_ERR_INVALID_ARG;
+    if (n_cw > h->max_batch) return NRLDPC_ERR_TOO_LARGE;
+    if (reinterpret_cast<uintptr_t>(d_llr) % 16 != 0) return NRLDPC_ERR_ALIGNMENT;
+    for (size_t k = 0; k < h->split.size(); k++) {
+        if (!split_counts(h->split[k], 0)) continue;
+        return map_cuda(launch_split_timeout(h->split[k],
+                                             split_args(h, static_cast<int>(k), d_llr, d_packed, n_cw, 2),
+                                             reinterpret_cast<unsigned char*>(h->scratch) + h->split_at[k],
+                                             std::min(n_cw, h->split_room[k]),
+                                             reinterpret_cast<cudaStream_t>(stream)));
+    }
+    return NRLDPC_ERR_BAD_CONFIG;
 }
 
 int nrldpc_decode_weighted(nrldpc_handle* handle, const float* d_llr, uint8_t* d_packed, int n_cw,

@@ -175,6 +175,7 @@ constexpr int kSplitMaxRanks = 16;   // CTAs per cluster
 constexpr int kSplitMaxPhases = 8;   // row ranges of an iteration
 constexpr int kSplitMaxWarps = 24;   // per CTA
 constexpr size_t kSplitHeader = 144;  // mbarriers, failure flags, head
+constexpr int kSplitWaitLimit = 1 << 20;  // polls, as decode_kernel's
 constexpr int kSplitKeep = 10;       // longest row whose Q and dt addresses stay in registers
 constexpr int kSplitVnAhead = 8;     // dt requested before the first add
 constexpr int kSplitRowCost = 4;     // a row's fixed work, in edges
@@ -206,6 +207,7 @@ struct SplitArgs {
     int* error_flag;         // bounded-wait failures
     int n_cw, n_iter, n_w_iters, early_stop, llr_from_host;
     float alpha;
+    int32_t wait_limit = kSplitWaitLimit;  // polls before a wait gives up
 };
 static_assert(kSplitHeader >= 32 + sizeof(SplitHead) && kSplitHeader % 16 == 0, "flags, then the head");
 // Cluster sizes tried: each holds more codewords at once than the one before
@@ -226,6 +228,11 @@ bool make_split_plan(const CodeTable& tab, int ranks, size_t smem_limit, SplitHe
                      std::vector<unsigned char>* out);
 cudaError_t split_kernel_attributes(size_t smem);
 int split_max_clusters(const SplitHead& head);  // resident at once
+bool split_counts(const SplitHead& head, int early_stop);  // whether its passes wait for counted bytes
+// launch_split with a short wait limit and, for its time, the first CTA of
+// every cluster of the plan expecting 16 bytes more than it is sent.
+cudaError_t launch_split_timeout(const SplitHead& head, SplitArgs args, unsigned char* plan, int n_clusters,
+                                 cudaStream_t stream);
 cudaError_t launch_split(const SplitHead& head, const SplitArgs& args, const WeightTable* weights, int n_clusters,
                          cudaStream_t stream);
 

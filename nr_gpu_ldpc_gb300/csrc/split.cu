@@ -56,6 +56,9 @@ constexpr int kSplitThreads = kSplitMaxWarps * 32;
 // it has that column's posteriors, which the owner sends after its dt are
 // complete, and those include dt that their readers sent after the posteriors
 // before were complete; a thread opens each phase after all have seen the last.
+// The waits are bounded (kSplitWaitLimit polls): where one runs out the
+// cluster reports it, and leaves without writing its codeword or taking
+// another.
 enum Mode { kOne, kCounted, kBarriers };
 
 constexpr uint32_t kHdBit = 0x80000000u;  // state info: hard decision of the suffix posterior read
@@ -111,19 +114,24 @@ __device__ __forceinline__ void mbar_init(uint32_t bar) {
 __device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ bool mbar_poll(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
 // Bounded wait for the phase of this parity; false when the limit ran out.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    for (int i = 0; i < (1 << 16); i++) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (ok) return true;
-    }
+// (The first poll stands outside the loop: 1.3 us less in 10 iterations of one
+// BG1 Z=384 codeword than all of them inside.)
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int limit) {
+    if (mbar_poll(bar, parity)) return true;
+    for (int i = 1; i < limit; i++)
+        if (mbar_poll(bar, parity)) return true;
     return false;
 }
 // Barrier over every thread of the cluster; shared-memory writes before it
@@ -300,19 +308,23 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
             cluster_sync();
     };
     const uint32_t bar_dt = smem_u32(smem), bar_l = bar_dt + 8;  // mbarriers of the dt and the posteriors
-    uint32_t* s_fail = reinterpret_cast<uint32_t*>(smem + 16);   // [2] an unsatisfied row, by iteration parity
+    // [2] an unsatisfied row, by iteration parity; [2] a wait of some thread of the cluster ran out
+    uint32_t* s_fail = reinterpret_cast<uint32_t*>(smem + 16);
     uint32_t ph_dt = 0, ph_l = 0;                                // parities waited for next
-    bool dead = false;  // a wait ran out: reported, and no further one
     if (MODE == kCounted && tid == 0) {
         mbar_init(bar_dt);
         mbar_init(bar_l);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    auto wait = [&](uint32_t bar, uint32_t parity) {
-        if (!dead && !mbar_wait(bar, parity)) {
-            dead = true;
-            atomicExch(a.error_flag, kErrSplitTimeout);
-        }
+    // Warps with task lists (a mixed batch's CTA may have more); 0 in a thread
+    // of which a wait ran out: it waits and sends no more, and thread 0 opens no
+    // further phase (an arrival on one that has not ended is undefined).  What
+    // others still send to the CTA is counted on the open phases, two passes'
+    // bytes at most: then they lack what it owes them.
+    int lists = 1;
+    auto wait = [&](uint32_t bar, uint32_t& parity) {
+        if (lists && !mbar_wait(bar, parity, a.wait_limit)) lists = 0;
+        parity ^= 1u;
         __syncthreads();  // all threads have seen it before the next phase opens
     };
     // the plan's head and this rank's tables; read where they are used, so
@@ -320,7 +332,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
     SplitHead* s_head = reinterpret_cast<SplitHead*>(smem + 32);
     const volatile SplitHead& h = *s_head;
     unsigned char* image = smem + kSplitHeader;
-    if (tid < 2) s_fail[tid] = 0;
+    if (tid < 3) s_fail[tid] = 0;
     const unsigned char* loaded = nullptr;
     for (int item = blockIdx.x / C; item < a.n_cw; item += gridDim.x / C) {
         const unsigned char* plan = a.plan;
@@ -345,7 +357,8 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
             const unsigned char* src = plan + sizeof(SplitHead) + static_cast<size_t>(rank) * h.image_bytes;
             for (int k = tid; k < h.image_bytes / 16; k += nt) cp_async16(smem_u32(image) + 16u * k, src + 16 * k);
         }
-        const int z = h.z, P = h.phases, lists = h.warps;  // warps with task lists (a mixed batch's CTA may have more)
+        const int z = h.z, P = h.phases;
+        lists = h.warps;
         const uint32_t z4 = 4u * static_cast<uint32_t>(z);
         if (!a.jobs) {
             llr += static_cast<size_t>(cw) * h.n_bp;
@@ -387,11 +400,9 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
                 wcur = wt.w[min(t, a.n_w_iters - 1)];
             }
             if (MODE == kCounted) {
-                if (t > 0) {
-                    wait(bar_l, ph_l);  // the posteriors of the last iteration
-                    ph_l ^= 1u;
-                }
-                if (tid == 0) mbar_expect(bar_dt, reinterpret_cast<const uint32_t*>(image + h.o_bytes)[0]);
+                if (t > 0) wait(bar_l, ph_l);  // the posteriors of the last iteration
+                if (tid == 0 && lists)
+                    mbar_expect(bar_dt, reinterpret_cast<const uint32_t*>(image + h.o_bytes)[0]);
             }
             for (int p = 0; p < (MODE == kCounted ? 1 : P); p++) {
                 const uint16_t* cnptr = reinterpret_cast<const uint16_t*>(image + h.o_cnptr) + p * lists + warp;
@@ -443,7 +454,6 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
                 // the dt of this phase, and (last phase) the failures, are in place
                 if (MODE == kCounted) {
                     wait(bar_dt, ph_dt);
-                    ph_dt ^= 1u;
                 } else {
                     sync();
                 }
@@ -452,7 +462,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
                     it = t;
                     break;
                 }
-                if (MODE == kCounted && tid == 0)
+                if (MODE == kCounted && tid == 0 && lists)
                     mbar_expect(bar_l, reinterpret_cast<const uint32_t*>(image + h.o_bytes)[1]);
                 const uint16_t* vnptr = reinterpret_cast<const uint16_t*>(image + h.o_vnptr) + warp;
                 const uint16_t* vn = reinterpret_cast<const uint16_t*>(image + h.o_vn);
@@ -496,11 +506,23 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
             }
         }
         if (MODE == kCounted) {
-            if (!conv) {
-                wait(bar_l, ph_l);
-                ph_l ^= 1u;
+            wait(bar_l, ph_l);
+            if (!lists)
+                for (int q = 0; q < C; q++) stc_u32(mapa(smem_u32(&s_fail[2]), q), 1u);
+            sync();  // every CTA's posteriors and states are final, and none sends any more
+            if (s_fail[2]) {
+                // what was sent to a CTA whose wait ran out may be under way: as
+                // many polls again before any leaves
+                if (!lists) {
+                    atomicExch(a.error_flag, kErrSplitTimeout);
+                    for (int i = 0; i < a.wait_limit; i++) {
+                        mbar_poll(bar_dt, 0);
+                        mbar_poll(bar_l, 0);
+                    }
+                }
+                sync();
+                return;
             }
-            sync();  // every CTA's posteriors and states are final
         }
         // Packed hard decisions (and posteriors): 32 positions per warp.
         const int n = h.n_bp, packed_bytes = h.packed_bytes, nc = h.n_core;
@@ -804,6 +826,8 @@ int split_max_clusters(const SplitHead& h) {
     return n;
 }
 
+bool split_counts(const SplitHead& h, int early_stop) { return mode_of(h, early_stop) == kCounted; }
+
 cudaError_t launch_split(const SplitHead& h, const SplitArgs& args, const WeightTable* weights, int n_clusters,
                          cudaStream_t stream) {
     cudaLaunchConfig_t cfg{};
@@ -813,6 +837,21 @@ cudaError_t launch_split(const SplitHead& h, const SplitArgs& args, const Weight
     void* params[2] = {const_cast<SplitArgs*>(&args),
                        weights ? const_cast<WeightTable*>(weights) : static_cast<void*>(&none)};
     return cudaLaunchKernelExC(&cfg, split_kernel(weights != nullptr, mode_of(h, args.early_stop)), params);
+}
+
+cudaError_t launch_split_timeout(const SplitHead& h, SplitArgs args, unsigned char* plan, int n_clusters,
+                                 cudaStream_t stream) {
+    uint32_t bytes = 0;  // of dt that reach the first CTA, in its table image
+    void* at = plan + sizeof(SplitHead) + h.o_bytes;
+    cudaError_t e = cudaMemcpyAsync(&bytes, at, sizeof(bytes), cudaMemcpyDeviceToHost, stream);
+    if (e != cudaSuccess || (e = cudaStreamSynchronize(stream)) != cudaSuccess) return e;
+    const uint32_t more = bytes + 16;
+    args.wait_limit = 1024;
+    e = cudaMemcpyAsync(at, &more, sizeof(more), cudaMemcpyHostToDevice, stream);
+    if (e == cudaSuccess) e = launch_split(h, args, nullptr, n_clusters, stream);
+    const cudaError_t back = cudaMemcpyAsync(at, &bytes, sizeof(bytes), cudaMemcpyHostToDevice, stream);
+    const cudaError_t done = cudaStreamSynchronize(stream);
+    return e != cudaSuccess ? e : back != cudaSuccess ? back : done;
 }
 
 }  // namespace nrldpc
