@@ -371,6 +371,7 @@ int init_impl(const int* base, int rows, int cols, int kb, const nrldpc_config* 
         cudaMalloc(&h->state2, state_elems * kStateBytesPerRow) != cudaSuccess ||
         cudaMalloc(&h->scratch, scratch.size()) != cudaSuccess ||
         cudaMemcpy(h->scratch, scratch.data(), scratch.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+        uploads_landed() != cudaSuccess ||
         cudaMalloc(&h->stage_llr, n_llr * sizeof(float)) != cudaSuccess ||
         cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&h->lane_stream, cudaStreamNonBlocking) != cudaSuccess ||

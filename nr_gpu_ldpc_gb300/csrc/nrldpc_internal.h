@@ -255,6 +255,11 @@ void in_flight_leave(InFlight* me);
 int in_flight_others(const InFlight* me, cudaStream_t stream, long sms, int sm_count);
 void in_flight_note(InFlight* me, cudaStream_t stream);  // after a call's launches
 
+// A copy from pageable memory and a memset may return before the device has the
+// data, and work on other streams than the legacy one is not ordered after
+// them: waited for before a handle is given out.
+inline cudaError_t uploads_landed() { return cudaStreamSynchronize(cudaStreamLegacy); }
+
 // Host-side launchers (decode.cu / channel.cu).
 // kind: which kernels serve a code and geometry (decode_shape).
 // weights: null for the plain decoder; layered: row-sequential schedule (no

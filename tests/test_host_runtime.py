@@ -1,0 +1,108 @@
+"""Host code of the library on a CUDA runtime without a GPU
+(tests/cpp/fake_cudart.cpp): what is launched, copied and allocated when."""
+import ctypes as C
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+from nr_gpu_ldpc_gb300 import _lib, build
+from nr_gpu_ldpc_gb300.batch import make_jobs
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+pytestmark = pytest.mark.skipif(shutil.which("g++") is None, reason="g++ not present")
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    objs = [os.path.join(build.BUILD, s.replace(".cu", ".o")) for s in build.SOURCES]
+    build.build(force=not all(map(os.path.exists, objs)))
+    so = str(tmp_path_factory.mktemp("fake") / "libfake.so")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-I",
+                    os.path.join(CUDA, "include"), os.path.join(HERE, "cpp", "fake_cudart.cpp"), *objs, "-o", so],
+                   check=True, capture_output=True, text=True)
+    lib = C.CDLL(so)
+    for name, (res, args) in _lib.SIGNATURES.items():
+        fn = getattr(lib, name)
+        fn.restype, fn.argtypes = res, args
+    lib.fake_last_launch.restype = C.c_char_p
+    lib.fake_unfinished.restype = C.c_long
+    for f in ("fake_stream_busy", "fake_stream_capturing"):
+        getattr(lib, f).argtypes = [C.c_void_p, C.c_int]
+    return lib
+
+
+@pytest.fixture
+def rt(fake):
+    fake.fake_reset()
+    return fake
+
+
+class Handle:
+    """A decoder handle and buffers for n codewords."""
+
+    def __init__(self, rt, bg=1, z=384, n=64, device=0):
+        cfg = _lib.ConfigC(bg=bg, z=z, max_batch=n, alpha=0.75, device=device, cw_per_cta=0)
+        self.rt, self.h = rt, C.c_void_p()
+        assert rt.nrldpc_init(C.byref(cfg), C.byref(self.h)) == 0
+        cols = 68 if bg == 1 else 52
+        self.buf = np.zeros(n * cols * z + 4, np.float32)
+        self.llr = (self.buf.ctypes.data + 15) // 16 * 16
+        self.out = np.zeros(n * (cols * z + 7) // 8 + 8, np.uint8)
+
+    def decode(self, n, stream, early=0):
+        assert self.rt.nrldpc_decode(self.h, self.llr, self.out.ctypes.data, n, 5, early, None, None, stream) == 0
+        return b"split" in self.rt.fake_last_launch()
+
+    def close(self):
+        self.rt.nrldpc_destroy(self.h)
+
+
+class List:
+    """A job list handle."""
+
+    def __init__(self, rt, max_jobs=512):
+        self.rt, self.h = rt, C.c_void_p()
+        assert rt.nrldpc_batch_create(0, max_jobs, 0.75, C.byref(self.h)) == 0
+
+    def set_jobs(self, bg, z):
+        self.jobs, n_llr, _, n_out = make_jobs(np.broadcast_to(bg, np.shape(z)), np.asarray(z))
+        self.buf = np.zeros(n_llr + 4, np.float32)
+        self.llr = (self.buf.ctypes.data + 15) // 16 * 16
+        self.out = np.zeros(n_out, np.uint8)
+        return self.rt.nrldpc_batch_set_jobs(self.h, self.jobs.ctypes.data, self.jobs.size)
+
+    def decode(self, stream):
+        assert self.rt.nrldpc_batch_decode(self.h, self.llr, self.out.ctypes.data, 5, 0, None, stream) == 0
+        return b"split" in self.rt.fake_last_launch()
+
+    def close(self):
+        self.rt.nrldpc_batch_destroy(self.h)
+
+
+STREAM = [0x100, 0x200, 0x300, 0x400, 0x500, 0x600]  # non-blocking streams, made up
+
+
+def test_nothing_runs_before_its_tables_and_lists_have_landed(rt):
+    # work on a non-blocking stream is not ordered after a pageable copy or a
+    # memset, which only the legacy stream waits for
+    d = Handle(rt)
+    assert rt.fake_unfinished() == 0
+    b = List(rt)
+    assert rt.fake_unfinished() == 0
+    e = np.zeros(1 << 24, np.uint8)
+    for z in ([384] * 5, [384] * 5 + [40] * 20, [64] * 400):
+        for call in (lambda: b.decode(STREAM[0]),
+                     lambda: rt.nrldpc_batch_derate(b.h, e.ctypes.data, b.llr, STREAM[0]),
+                     lambda: rt.nrldpc_batch_gen(b.h, 1, 0, e.ctypes.data, None, STREAM[0]),
+                     lambda: rt.nrldpc_batch_count_errors(b.h, b.out.ctypes.data, b.out.ctypes.data, e.ctypes.data,
+                                                          STREAM[0])):
+            assert b.set_jobs(1, z) == 0
+            before = rt.fake_launches()
+            call()
+            assert rt.fake_launches() == before + 1 and rt.fake_early_launches() == 0
+    d.close()
+    b.close()
