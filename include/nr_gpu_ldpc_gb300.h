@@ -250,6 +250,15 @@ int nrldpc_batch_derate(nrldpc_batch* b, const float* d_llr_e, float* d_llr, nrl
  * replayed from a CUDA graph; d_iters (may be NULL) indexed by job. */
 int nrldpc_batch_decode(nrldpc_batch* b, const float* d_llr, uint8_t* d_packed, int n_iter,
                         int early_stop, int32_t* d_iters, nrldpc_stream_t stream);
+/* Last device-side error recorded by a bounded wait of a list's decode (0 if
+ * none, else NRLDPC_ERR_TIMEOUT: jobs of that decode have no result); clears it. */
+int nrldpc_batch_device_error(nrldpc_batch* b);
+/* Self-test of a short list's bounded waits, as nrldpc_selftest_split_timeout
+ * for a handle: the loaded jobs of the list's first code are not decoded and
+ * nrldpc_batch_device_error then reports the timeout.  NRLDPC_ERR_BAD_CONFIG
+ * for a list that does not run on such clusters. */
+int nrldpc_selftest_batch_timeout(nrldpc_batch* b, const float* d_llr, uint8_t* d_packed,
+                                  nrldpc_stream_t stream);
 /* d_counts[2] += {bit errors, frame errors} over each job's k_prime info bits. */
 int nrldpc_batch_count_errors(nrldpc_batch* b, const uint8_t* d_packed, const uint8_t* d_cw,
                               unsigned long long* d_counts, nrldpc_stream_t stream);

@@ -74,6 +74,8 @@ SIGNATURES = {
     "nrldpc_batch_derate": (_i, [_vp, _vp, _vp, _vp]),
     "nrldpc_batch_decode": (_i, [_vp, _vp, _vp, _i, _i, _vp, _vp]),
     "nrldpc_batch_count_errors": (_i, [_vp, _vp, _vp, _vp, _vp]),
+    "nrldpc_batch_device_error": (_i, [_vp]),
+    "nrldpc_selftest_batch_timeout": (_i, [_vp, _vp, _vp, _vp]),
     "nrldpc_rm_k0": (_i, [_i, _i, _i]),
     "nrldpc_crc": (_i, [_vp, _i, _i, _i, _i, _vp, _vp]),
     "nrldpc_segment": (_i, [_i, _i, C.POINTER(SegmentInfoC)]),

@@ -143,3 +143,8 @@ class Batch:
                    self.lib.nrldpc_batch_count_errors(self._h, _dev_ptr(packed), _dev_ptr(cw), _dev_ptr(counts),
                                                       _stream_ptr(stream)))
         return counts
+
+    def device_error(self) -> int:
+        """0, or the error of a device-side wait that ran out in a decode
+        since the last call (negative; cleared)."""
+        return self.lib.nrldpc_batch_device_error(self._h)

@@ -309,6 +309,7 @@ struct Batch {
     SplitJob* d_split = nullptr;
     SplitHead split{};
     int split_clusters = 0;
+    size_t split_count_at = 0;  // of the bytes that the first CTA of the list's first code expects (self-test)
     size_t slot_words = 0, smem = 0;
     bool classes = false;  // of rows and layouts (batch_decode_kernel)
     int grid = 0, threads = kMaxThreads;
@@ -365,6 +366,19 @@ void free_batch(Batch* b) {
     cudaFree(b->d_state);
     cudaFree(b->d_scratch);
     delete b;
+}
+
+SplitArgs split_args(const Batch* b, const float* llr, uint8_t* packed, int n_iter) {
+    SplitArgs a{};
+    a.plan = b->d_plans_split;
+    a.jobs = b->d_split;
+    a.llr = llr;
+    a.packed = packed;
+    a.error_flag = b->d_scratch + 1;
+    a.n_cw = b->n_jobs;
+    a.n_iter = n_iter;
+    a.alpha = b->alpha;
+    return a;
 }
 
 // Before work on `stream` reads the lists and plans: their copies come from
@@ -450,6 +464,8 @@ int choose_split(Batch* b, const std::vector<int32_t>& order, const std::vector<
             return NRLDPC_ERR_CUDA;
         b->plans_sent = b->h_plans.size();
     }
+    const Batch::Plan& first = b->plans[b->h_jobs[order[0]].code * kSplitSizes + best];
+    b->split_count_at = first.at + sizeof(SplitHead) + first.head.o_bytes;
     jobs->resize(n);
     for (int i = 0; i < n; i++) {
         const JobDev& d = b->h_jobs[order[i]];
@@ -743,17 +759,9 @@ int nrldpc_batch_decode(nrldpc_batch* batch, const float* d_llr, uint8_t* d_pack
         static_cast<long>(b->n_jobs) * b->split.ranks *
                 in_flight_others(&b->in_flight, reinterpret_cast<cudaStream_t>(stream),
                                  static_cast<long>(b->n_jobs) * b->split.ranks, b->sm_count) <= b->sm_count) {
-        SplitArgs a{};
-        a.plan = b->d_plans_split;
-        a.jobs = b->d_split;
-        a.llr = d_llr;
-        a.packed = d_packed;
+        SplitArgs a = split_args(b, d_llr, d_packed, n_iter);
         a.iters = d_iters;
-        a.error_flag = b->d_scratch + 1;
-        a.n_cw = b->n_jobs;
-        a.n_iter = n_iter;
         a.early_stop = early_stop;
-        a.alpha = b->alpha;
         const int rc =
             map_cuda(launch_split(b->split, a, nullptr, b->split_clusters, reinterpret_cast<cudaStream_t>(stream)));
         in_flight_note(&b->in_flight, reinterpret_cast<cudaStream_t>(stream));
@@ -802,6 +810,27 @@ int nrldpc_batch_decode(nrldpc_batch* batch, const float* d_llr, uint8_t* d_pack
     const int rc = map_cuda(cudaGraphLaunch(b->exec, reinterpret_cast<cudaStream_t>(stream)));
     in_flight_note(&b->in_flight, reinterpret_cast<cudaStream_t>(stream));
     return rc;
+}
+
+int nrldpc_batch_device_error(nrldpc_batch* batch) {
+    Batch* b = reinterpret_cast<Batch*>(batch);
+    if (!b) return NRLDPC_ERR_INVALID_ARG;
+    int v = 0;
+    if (cudaMemcpy(&v, b->d_scratch + 1, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return NRLDPC_ERR_CUDA;
+    if (v) cudaMemset(b->d_scratch + 1, 0, sizeof(int));
+    return v ? NRLDPC_ERR_TIMEOUT : NRLDPC_OK;
+}
+
+int nrldpc_selftest_batch_timeout(nrldpc_batch* batch, const float* d_llr, uint8_t* d_packed,
+                                  nrldpc_stream_t stream) {
+    Batch* b = reinterpret_cast<Batch*>(batch);
+    if (!b || !d_llr || !d_packed) return NRLDPC_ERR_INVALID_ARG;
+    if (reinterpret_cast<uintptr_t>(d_llr) % 16 != 0) return NRLDPC_ERR_ALIGNMENT;
+    if (b->n_jobs == 0 || !b->split.ranks || !split_counts(b->split, 0)) return NRLDPC_ERR_BAD_CONFIG;
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    if (wait_lists(b, st) != cudaSuccess) return NRLDPC_ERR_CUDA;
+    return map_cuda(launch_split_timeout(b->split, split_args(b, d_llr, d_packed, 2),
+                                         b->d_plans_split + b->split_count_at, b->split_clusters, st));
 }
 
 }  // extern "C"

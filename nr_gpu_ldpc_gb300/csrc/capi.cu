@@ -698,7 +698,8 @@ int nrldpc_selftest_split_timeout(nrldpc_handle* handle, const float* d_llr, uin
         if (!split_counts(h->split[k], 0)) continue;
         return map_cuda(launch_split_timeout(h->split[k],
                                              split_args(h, static_cast<int>(k), d_llr, d_packed, n_cw, 2),
-                                             reinterpret_cast<unsigned char*>(h->scratch) + h->split_at[k],
+                                             reinterpret_cast<unsigned char*>(h->scratch) + h->split_at[k] +
+                                                 sizeof(SplitHead) + h->split[k].o_bytes,
                                              std::min(n_cw, h->split_room[k]),
                                              reinterpret_cast<cudaStream_t>(stream)));
     }

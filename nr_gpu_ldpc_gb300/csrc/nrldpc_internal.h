@@ -229,9 +229,9 @@ bool make_split_plan(const CodeTable& tab, int ranks, size_t smem_limit, SplitHe
 cudaError_t split_kernel_attributes(size_t smem);
 int split_max_clusters(const SplitHead& head);  // resident at once
 bool split_counts(const SplitHead& head, int early_stop);  // whether its passes wait for counted bytes
-// launch_split with a short wait limit and, for its time, the first CTA of
-// every cluster of the plan expecting 16 bytes more than it is sent.
-cudaError_t launch_split_timeout(const SplitHead& head, SplitArgs args, unsigned char* plan, int n_clusters,
+// launch_split with a short wait limit and, for its time, 16 bytes more in the
+// count at `expected`, of the bytes that reach a plan's first CTA.
+cudaError_t launch_split_timeout(const SplitHead& head, SplitArgs args, void* expected, int n_clusters,
                                  cudaStream_t stream);
 cudaError_t launch_split(const SplitHead& head, const SplitArgs& args, const WeightTable* weights, int n_clusters,
                          cudaStream_t stream);

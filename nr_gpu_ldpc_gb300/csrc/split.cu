@@ -839,17 +839,16 @@ cudaError_t launch_split(const SplitHead& h, const SplitArgs& args, const Weight
     return cudaLaunchKernelExC(&cfg, split_kernel(weights != nullptr, mode_of(h, args.early_stop)), params);
 }
 
-cudaError_t launch_split_timeout(const SplitHead& h, SplitArgs args, unsigned char* plan, int n_clusters,
+cudaError_t launch_split_timeout(const SplitHead& h, SplitArgs args, void* expected, int n_clusters,
                                  cudaStream_t stream) {
-    uint32_t bytes = 0;  // of dt that reach the first CTA, in its table image
-    void* at = plan + sizeof(SplitHead) + h.o_bytes;
-    cudaError_t e = cudaMemcpyAsync(&bytes, at, sizeof(bytes), cudaMemcpyDeviceToHost, stream);
+    uint32_t bytes = 0;
+    cudaError_t e = cudaMemcpyAsync(&bytes, expected, sizeof(bytes), cudaMemcpyDeviceToHost, stream);
     if (e != cudaSuccess || (e = cudaStreamSynchronize(stream)) != cudaSuccess) return e;
     const uint32_t more = bytes + 16;
     args.wait_limit = 1024;
-    e = cudaMemcpyAsync(at, &more, sizeof(more), cudaMemcpyHostToDevice, stream);
+    e = cudaMemcpyAsync(expected, &more, sizeof(more), cudaMemcpyHostToDevice, stream);
     if (e == cudaSuccess) e = launch_split(h, args, nullptr, n_clusters, stream);
-    const cudaError_t back = cudaMemcpyAsync(at, &bytes, sizeof(bytes), cudaMemcpyHostToDevice, stream);
+    const cudaError_t back = cudaMemcpyAsync(expected, &bytes, sizeof(bytes), cudaMemcpyHostToDevice, stream);
     const cudaError_t done = cudaStreamSynchronize(stream);
     return e != cudaSuccess ? e : back != cudaSuccess ? back : done;
 }

@@ -9,6 +9,7 @@ import pytest
 import torch
 
 from nr_gpu_ldpc_gb300 import Decoder, _lib, codes
+from nr_gpu_ldpc_gb300.batch import Batch, make_jobs
 from oracle.oracle import OracleCode
 
 pytestmark = pytest.mark.gpu
@@ -44,3 +45,22 @@ def test_code_without_such_clusters(gpu):
     assert _lib.load().nrldpc_selftest_split_timeout(dec._h, C.c_void_p(llr.data_ptr()), C.c_void_p(out.data_ptr()),
                                                      1, None) == -2  # NRLDPC_ERR_BAD_CONFIG
     dec.close()
+
+
+@pytest.mark.parametrize("bg,z,n", [(1, 384, 1), (1, 384, 12), (2, 208, 9)])
+def test_wait_that_runs_out_in_a_job_list(gpu, bg, z, n):
+    jobs, n_llr, _, n_out = make_jobs(np.full(n, bg), z)
+    llr = torch.empty(n_llr, device=gpu).normal_(generator=torch.Generator(device=gpu).manual_seed(3)) * 2 + 2
+    b = Batch(max_jobs=n)
+    b.set_jobs(jobs)
+    want, out = (torch.full((n_out,), 0xA5, dtype=torch.uint8, device=gpu) for _ in range(2))
+    b.decode(llr, want, 5)
+    assert b.device_error() == 0
+    assert _lib.load().nrldpc_selftest_batch_timeout(b._h, C.c_void_p(llr.data_ptr()), C.c_void_p(out.data_ptr()),
+                                                     C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    torch.cuda.synchronize()
+    assert b.device_error() == -6 and b.device_error() == 0
+    assert torch.all(out == 0xA5)
+    b.decode(llr, out, 5)
+    assert torch.equal(out, want) and b.device_error() == 0
+    b.close()
