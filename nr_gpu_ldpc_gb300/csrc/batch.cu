@@ -402,7 +402,7 @@ cudaError_t wait_lists(Batch* b, cudaStream_t stream) {
 int choose_split(Batch* b, const std::vector<int32_t>& order, const std::vector<WorkItem>& items,
                  std::vector<SplitJob>* jobs) {
     static const int kRoom[kSplitSizes] = {7, 13, 23, 28, 36, 46, 76, 152};  // at one CTA per SM of 152
-    const int n = b->n_jobs;
+    const int n = static_cast<int>(order.size());
     if (n > 2L * kRoom[kSplitSizes - 1] * b->sm_count / 152) return NRLDPC_OK;
     long fused_sum = 0, least = 0;
     for (const WorkItem& it : items) {
@@ -664,7 +664,7 @@ int nrldpc_batch_set_jobs(nrldpc_batch* batch, const nrldpc_job* jobs, int n_job
         }
         i = k;
     }
-    b->n_jobs = n_jobs;
+    b->n_jobs = 0;  // until everything is in place: the list before no longer is
     b->n_items = static_cast<int>(items.size());
     b->slot_words = slot_words;
     b->smem = kHeaderBytesBatch + kBatchTableBytes + bufs;
@@ -707,6 +707,7 @@ int nrldpc_batch_set_jobs(nrldpc_batch* batch, const nrldpc_job* jobs, int n_job
         cudaEventRecord(b->lists_sent, cudaStreamLegacy) != cudaSuccess)
         return NRLDPC_ERR_CUDA;
     b->lists_landed = false;
+    b->n_jobs = n_jobs;
     return NRLDPC_OK;
 }
 

@@ -106,3 +106,21 @@ def test_nothing_runs_before_its_tables_and_lists_have_landed(rt):
             assert rt.fake_launches() == before + 1 and rt.fake_early_launches() == 0
     d.close()
     b.close()
+
+
+@pytest.mark.parametrize("bg,z", [(1, [384] * 400), ([1, 2] * 5, [2, 7, 16, 40, 64, 128, 208, 256, 320, 384])])
+def test_list_that_could_not_be_loaded_is_not_run(rt, bg, z):
+    for after in range(8):  # the allocation that fails
+        b = List(rt)
+        assert b.set_jobs(1, [384] * 2) == 0 and b.decode(STREAM[0])
+        rt.fake_fail_malloc(after)
+        rc = b.set_jobs(bg, z)
+        rt.fake_fail_malloc(-1)
+        before = rt.fake_launches()
+        b.decode(STREAM[0])
+        assert rt.fake_launches() == (before if rc else before + 1)
+        assert b.set_jobs(1, [384] * 2) == 0 and b.decode(STREAM[0])
+        b.close()
+        if rc == 0:
+            break
+    assert rc == 0 and after > 0
