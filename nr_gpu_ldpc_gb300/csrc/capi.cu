@@ -7,6 +7,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <new>
 #include <vector>
@@ -16,31 +17,39 @@
 
 namespace nrldpc {
 namespace {
-std::mutex g_in_flight_mu;
-std::vector<InFlight*> g_in_flight;  // one per live handle
-int g_crowd[64];                     // per device: the last count, falling
+// The decoders of one device
+struct Flights {
+    std::vector<InFlight*> live;
+    int crowd = 0;  // the last count, falling
+};
+std::mutex g_flights_mu;
+std::map<int, Flights> g_flights;  // a device's entry goes with its last decoder
 }  // namespace
 
 bool in_flight_join(InFlight* me, int device) {
     if (cudaEventCreateWithFlags(&me->done, cudaEventDisableTiming) != cudaSuccess) return false;
     me->device = device;
-    std::lock_guard<std::mutex> lock(g_in_flight_mu);
-    g_in_flight.push_back(me);
+    std::lock_guard<std::mutex> lock(g_flights_mu);
+    g_flights[device].live.push_back(me);
     return true;
 }
 
 void in_flight_leave(InFlight* me) {
     if (!me->done) return;
     {
-        std::lock_guard<std::mutex> lock(g_in_flight_mu);
-        g_in_flight.erase(std::remove(g_in_flight.begin(), g_in_flight.end(), me), g_in_flight.end());
+        std::lock_guard<std::mutex> lock(g_flights_mu);
+        std::vector<InFlight*>& live = g_flights[me->device].live;
+        live.erase(std::remove(live.begin(), live.end(), me), live.end());
+        if (live.empty()) g_flights.erase(me->device);
     }
     cudaEventDestroy(me->done);
 }
 
 int in_flight_others(const InFlight* me, cudaStream_t stream, long sms, int sm_count) {
-    std::lock_guard<std::mutex> lock(g_in_flight_mu);
-    if (g_in_flight.size() < 2 || sms * static_cast<long>(g_in_flight.size()) <= sm_count) return 0;
+    std::lock_guard<std::mutex> lock(g_flights_mu);
+    Flights& d = g_flights[me->device];
+    const int others = static_cast<int>(d.live.size()) - 1;
+    if (others < 1 || sms * (others + 1L) <= sm_count) return 0;
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
@@ -50,8 +59,8 @@ int in_flight_others(const InFlight* me, cudaStream_t stream, long sms, int sm_c
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     cudaThreadExchangeStreamCaptureMode(&mode);
     int busy = 0;
-    for (InFlight* f : g_in_flight) {
-        if (f == me || f->device != me->device || !f->recorded || f->stream == stream) continue;
+    for (InFlight* f : d.live) {
+        if (f == me || !f->recorded || f->stream == stream) continue;
         if (cudaEventQuery(f->done) == cudaErrorNotReady)
             busy++;
         else
@@ -59,14 +68,13 @@ int in_flight_others(const InFlight* me, cudaStream_t stream, long sms, int sm_c
     }
     cudaThreadExchangeStreamCaptureMode(&mode);
     if (busy) cudaGetLastError();  // not-ready is no error of the caller's
-    int& crowd = g_crowd[me->device & 63];
-    crowd = std::min(std::max(busy, crowd - 1), static_cast<int>(g_in_flight.size()) - 1);
-    return crowd;
+    d.crowd = std::min(std::max(busy, d.crowd - 1), others);
+    return d.crowd;
 }
 
 void in_flight_note(InFlight* me, cudaStream_t stream) {
-    std::lock_guard<std::mutex> lock(g_in_flight_mu);
-    if (g_in_flight.size() < 2) return;
+    std::lock_guard<std::mutex> lock(g_flights_mu);
+    if (g_flights[me->device].live.size() < 2) return;
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone &&
         cudaEventRecord(me->done, stream) == cudaSuccess)

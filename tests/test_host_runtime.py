@@ -124,3 +124,24 @@ def test_list_that_could_not_be_loaded_is_not_run(rt, bg, z):
         if rc == 0:
             break
     assert rc == 0 and after > 0
+
+
+# BG1 Z=384, 40 codewords: alone on clusters, beside others on decode_kernel
+
+
+def test_busy_neighbours_are_counted_per_device(rt):
+    far = [Handle(rt, device=1) for _ in range(3)]
+    d = Handle(rt)
+    for k, f in enumerate(far):
+        f.decode(40, STREAM[k])
+        rt.fake_stream_busy(STREAM[k], 1)
+    records = rt.fake_records()
+    assert d.decode(40, STREAM[3])  # no neighbour on its own device
+    assert rt.fake_records() == records  # nor anything to note for one
+    near = [Handle(rt) for _ in range(2)]
+    for k, f in enumerate(near):
+        f.decode(40, STREAM[4 + k])
+        rt.fake_stream_busy(STREAM[4 + k], 1)
+    assert not d.decode(40, STREAM[3])
+    for h in (*far, *near, d):
+        h.close()
