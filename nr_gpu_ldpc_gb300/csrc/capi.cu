@@ -433,7 +433,7 @@ int decode_impl(Handle* h, const float* llr, uint8_t* packed, int n_cw, int n_it
         a.llr_from_host = llr_from_host ? 1 : 0;
         const int rc = map_cuda(launch_split(h->split[plan], a, weighted ? h->weights : nullptr,
                                              std::min(n_cw, h->split_room[plan]), stream));
-        in_flight_note(&h->in_flight, stream);
+        if (!counter) in_flight_note(&h->in_flight, stream);  // chunks: host_decode, once
         return rc;
     }
     DecodeArgs a{};
@@ -547,6 +547,7 @@ int host_decode(Handle* h, const void* h_llr, int qtype, float scale, uint8_t* h
     if (cudaEventRecord(h->ev_lane, h->lane_stream) != cudaSuccess ||
         cudaStreamWaitEvent(s, h->ev_lane, 0) != cudaSuccess)
         return NRLDPC_ERR_CUDA;
+    in_flight_note(&h->in_flight, s);
     return rc;
 }
 

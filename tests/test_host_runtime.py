@@ -57,6 +57,9 @@ class Handle:
         assert self.rt.nrldpc_decode(self.h, self.llr, self.out.ctypes.data, n, 5, early, None, None, stream) == 0
         return b"split" in self.rt.fake_last_launch()
 
+    def decode_host_q(self, n, stream):
+        assert self.rt.nrldpc_decode_host_async_q(self.h, self.llr, 2, 0.5, self.out.ctypes.data, n, 5, 0, stream) == 0
+
     def close(self):
         self.rt.nrldpc_destroy(self.h)
 
@@ -144,4 +147,15 @@ def test_busy_neighbours_are_counted_per_device(rt):
         rt.fake_stream_busy(STREAM[4 + k], 1)
     assert not d.decode(40, STREAM[3])
     for h in (*far, *near, d):
+        h.close()
+
+
+def test_staged_host_calls_are_busy_neighbours(rt):
+    small, big = Handle(rt), [Handle(rt, n=3000) for _ in range(2)]
+    assert small.decode(40, STREAM[0])
+    for k, h in enumerate(big):
+        h.decode_host_q(3000, STREAM[1 + k])
+        rt.fake_stream_busy(STREAM[1 + k], 1)
+    assert not small.decode(40, STREAM[0])
+    for h in (small, *big):
         h.close()
