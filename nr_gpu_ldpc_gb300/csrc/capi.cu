@@ -21,6 +21,7 @@ namespace {
 struct Flights {
     std::vector<InFlight*> live;
     int crowd = 0;  // the last count, falling
+    const InFlight* last = nullptr;  // whose call was the last
 };
 std::mutex g_flights_mu;
 std::map<int, Flights> g_flights;  // a device's entry goes with its last decoder
@@ -40,6 +41,7 @@ void in_flight_leave(InFlight* me) {
         std::lock_guard<std::mutex> lock(g_flights_mu);
         std::vector<InFlight*>& live = g_flights[me->device].live;
         live.erase(std::remove(live.begin(), live.end(), me), live.end());
+        if (g_flights[me->device].last == me) g_flights[me->device].last = nullptr;
         if (live.empty()) g_flights.erase(me->device);
     }
     cudaEventDestroy(me->done);
@@ -68,13 +70,16 @@ int in_flight_others(const InFlight* me, cudaStream_t stream, long sms, int sm_c
     }
     cudaThreadExchangeStreamCaptureMode(&mode);
     if (busy) cudaGetLastError();  // not-ready is no error of the caller's
-    d.crowd = std::min(std::max(busy, d.crowd - 1), others);
+    // two calls of one decoder in a row with the others idle: it is alone
+    d.crowd = busy == 0 && d.last == me ? 0 : std::min(std::max(busy, d.crowd - 1), others);
     return d.crowd;
 }
 
 void in_flight_note(InFlight* me, cudaStream_t stream) {
     std::lock_guard<std::mutex> lock(g_flights_mu);
-    if (g_flights[me->device].live.size() < 2) return;
+    Flights& d = g_flights[me->device];
+    if (d.live.size() < 2) return;
+    d.last = me;
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone &&
         cudaEventRecord(me->done, stream) == cudaSuccess)

@@ -241,7 +241,8 @@ cudaError_t launch_split(const SplitHead& head, const SplitArgs& args, const Wei
 // twice the SM time of decode_kernel, so the choice counts the other decoders
 // of the device that are busy on other streams as as many batches like its
 // own.  The first call of a round sees the others idle, so the count falls by
-// one a call at most (a hint: either choice gives the same bits).
+// one a call at most, unless one decoder calls twice in a row beside idle ones
+// (a hint: either choice gives the same bits).
 struct InFlight {
     int device = -1;
     cudaEvent_t done = nullptr;  // after the last call

@@ -159,3 +159,17 @@ def test_staged_host_calls_are_busy_neighbours(rt):
     assert not small.decode(40, STREAM[0])
     for h in (small, *big):
         h.close()
+
+
+def test_lone_caller_is_back_on_clusters_after_a_burst(rt):
+    hs = [Handle(rt) for _ in range(6)]
+    for k, h in enumerate(hs):
+        h.decode(40, STREAM[k])
+        rt.fake_stream_busy(STREAM[k], 1)
+    assert not hs[0].decode(40, 0x700)
+    for s in STREAM:
+        rt.fake_stream_busy(s, 0)
+    hs[0].decode(40, STREAM[0])
+    assert hs[0].decode(40, STREAM[0])
+    for h in hs:
+        h.close()
