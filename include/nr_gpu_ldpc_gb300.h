@@ -150,6 +150,15 @@ int nrldpc_decode_weighted(nrldpc_handle* h, const float* d_llr, uint8_t* d_pack
                            int n_iter, int early_stop, float* d_app, int32_t* d_iters,
                            nrldpc_stream_t stream);
 
+/* Decoders that run beside this one's calls, on other streams of its device.  A
+ * small batch alone is spread over the whole GPU (several CTAs a codeword),
+ * the fastest for itself but at twice the GPU time; beside others it is not.
+ * n = -1 (default): the decoders of the process whose last call still runs are
+ * counted, and in a call that is captured into a graph all others of the
+ * device.  n >= 0 says it instead: 0 for graphs that are replayed alone.
+ * Results do not depend on it. */
+int nrldpc_set_neighbours(nrldpc_handle* h, int n);
+
 /* Message-passing schedule of a handle's decodes (nrldpc_decode,
  * nrldpc_decode_weighted, the host-buffer calls).  FLOODING (default) is the
  * reference's: every check row reads the previous iteration's posterior
@@ -250,6 +259,8 @@ int nrldpc_batch_derate(nrldpc_batch* b, const float* d_llr_e, float* d_llr, nrl
  * replayed from a CUDA graph; d_iters (may be NULL) indexed by job. */
 int nrldpc_batch_decode(nrldpc_batch* b, const float* d_llr, uint8_t* d_packed, int n_iter,
                         int early_stop, int32_t* d_iters, nrldpc_stream_t stream);
+/* As nrldpc_set_neighbours, for short job lists. */
+int nrldpc_batch_set_neighbours(nrldpc_batch* b, int n);
 /* Last device-side error recorded by a bounded wait of a list's decode (0 if
  * none, else NRLDPC_ERR_TIMEOUT: jobs of that decode have no result); clears it. */
 int nrldpc_batch_device_error(nrldpc_batch* b);

@@ -54,6 +54,7 @@ SIGNATURES = {
     "nrldpc_decode_host_async": (_i, [_vp, _vp, _vp, _i, _i, _i, _vp]),
     "nrldpc_decode_host_async_q": (_i, [_vp, _vp, _i, _f, _vp, _i, _i, _i, _vp]),
     "nrldpc_set_schedule": (_i, [_vp, _i]),
+    "nrldpc_set_neighbours": (_i, [_vp, _i]),
     "nrldpc_set_host_transfer": (_i, [_vp, _i]),
     "nrldpc_set_weights": (_i, [_vp, _vp, _i]),
     "nrldpc_decode_weighted": (_i, [_vp, _vp, _vp, _i, _i, _i, _vp, _vp, _vp]),
@@ -74,6 +75,7 @@ SIGNATURES = {
     "nrldpc_batch_derate": (_i, [_vp, _vp, _vp, _vp]),
     "nrldpc_batch_decode": (_i, [_vp, _vp, _vp, _i, _i, _vp, _vp]),
     "nrldpc_batch_count_errors": (_i, [_vp, _vp, _vp, _vp, _vp]),
+    "nrldpc_batch_set_neighbours": (_i, [_vp, _i]),
     "nrldpc_batch_device_error": (_i, [_vp]),
     "nrldpc_selftest_batch_timeout": (_i, [_vp, _vp, _vp, _vp]),
     "nrldpc_rm_k0": (_i, [_i, _i, _i]),

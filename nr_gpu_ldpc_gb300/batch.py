@@ -144,6 +144,10 @@ class Batch:
                                                       _stream_ptr(stream)))
         return counts
 
+    def set_neighbours(self, n: int) -> None:
+        """As Decoder.set_neighbours, for short lists."""
+        _lib.check("nrldpc_batch_set_neighbours", self.lib.nrldpc_batch_set_neighbours(self._h, int(n)))
+
     def device_error(self) -> int:
         """0, or the error of a device-side wait that ran out in a decode
         since the last call (negative; cleared)."""

@@ -813,6 +813,13 @@ int nrldpc_batch_decode(nrldpc_batch* batch, const float* d_llr, uint8_t* d_pack
     return rc;
 }
 
+int nrldpc_batch_set_neighbours(nrldpc_batch* batch, int n) {
+    Batch* b = reinterpret_cast<Batch*>(batch);
+    if (!b || n < -1) return NRLDPC_ERR_INVALID_ARG;
+    b->in_flight.neighbours = n;
+    return NRLDPC_OK;
+}
+
 int nrldpc_batch_device_error(nrldpc_batch* batch) {
     Batch* b = reinterpret_cast<Batch*>(batch);
     if (!b) return NRLDPC_ERR_INVALID_ARG;

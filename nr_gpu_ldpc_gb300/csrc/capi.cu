@@ -48,6 +48,7 @@ void in_flight_leave(InFlight* me) {
 }
 
 int in_flight_others(const InFlight* me, cudaStream_t stream, long sms, int sm_count) {
+    if (me->neighbours >= 0) return me->neighbours;
     std::lock_guard<std::mutex> lock(g_flights_mu);
     Flights& d = g_flights[me->device];
     const int others = static_cast<int>(d.live.size()) - 1;
@@ -55,7 +56,7 @@ int in_flight_others(const InFlight* me, cudaStream_t stream, long sms, int sm_c
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
-        return 0;
+        return others;
     }
     // a query must not disturb a capture of another thread
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
@@ -764,6 +765,13 @@ int nrldpc_set_host_transfer(nrldpc_handle* handle, int mode) {
     if (!h || (mode != NRLDPC_HOST_AUTO && mode != NRLDPC_HOST_COPY && mode != NRLDPC_HOST_DIRECT))
         return NRLDPC_ERR_INVALID_ARG;
     h->host_mode = mode;
+    return NRLDPC_OK;
+}
+
+int nrldpc_set_neighbours(nrldpc_handle* handle, int n) {
+    Handle* h = reinterpret_cast<Handle*>(handle);
+    if (!h || n < -1) return NRLDPC_ERR_INVALID_ARG;
+    h->in_flight.neighbours = n;
     return NRLDPC_OK;
 }
 

@@ -248,11 +248,15 @@ struct InFlight {
     cudaEvent_t done = nullptr;  // after the last call
     cudaStream_t stream = nullptr;
     bool recorded = false;
+    int neighbours = -1;  // what the caller says instead of the count
 };
 bool in_flight_join(InFlight* me, int device);
 void in_flight_leave(InFlight* me);
-// Busy ones beside `me`; 0 while the stream is captured, and where as many
-// calls of `sms` SMs as there are decoders fit the GPU's.
+// Busy ones beside `me`; 0 where as many calls of `sms` SMs as there are
+// decoders fit the GPU's.  While the stream is captured, all others: what runs
+// beside a replay is not known then.  Six graphs of 40 BG1 Z=384 codewords, 5
+// iterations, replayed on six streams: 0.400 ms a round spread, 0.208 on
+// decode_kernel; one of them alone 0.081 and 0.148.
 int in_flight_others(const InFlight* me, cudaStream_t stream, long sms, int sm_count);
 void in_flight_note(InFlight* me, cudaStream_t stream);  // after a call's launches
 

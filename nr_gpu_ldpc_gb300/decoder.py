@@ -144,6 +144,12 @@ class Decoder:
         code = {"auto": 0, "copy": 1, "direct": 2}.get(mode, mode)
         _lib.check("nrldpc_set_host_transfer", self._lib.nrldpc_set_host_transfer(self._h, int(code)))
 
+    def set_neighbours(self, n: int) -> None:
+        """Decoders that run beside this one's calls on other streams: -1
+        (default) counts them, and in a captured call takes all others of the
+        device; 0 for graphs that are replayed alone."""
+        _lib.check("nrldpc_set_neighbours", self._lib.nrldpc_set_neighbours(self._h, int(n)))
+
     # ---- schedule -------------------------------------------------------------------
     FLOODING, LAYERED = 0, 1
 

@@ -173,3 +173,25 @@ def test_lone_caller_is_back_on_clusters_after_a_burst(rt):
     assert hs[0].decode(40, STREAM[0])
     for h in hs:
         h.close()
+
+
+def test_captured_calls_presume_the_other_decoders_beside_them(rt):
+    # what runs beside a replay is not known when the call is captured
+    hs = [Handle(rt)]
+    rt.fake_stream_capturing(STREAM[0], 1)
+    assert hs[0].decode(40, STREAM[0])  # the only decoder
+    hs += [Handle(rt) for _ in range(5)]
+    assert not hs[0].decode(40, STREAM[0])
+    lists = List(rt)
+    assert lists.set_jobs(1, [384] * 40) == 0
+    assert not lists.decode(STREAM[0])
+    for h, close in ((hs[0], rt.nrldpc_set_neighbours), (lists, rt.nrldpc_batch_set_neighbours)):
+        assert close(h.h, 0) == 0  # the caller knows better
+    assert hs[0].decode(40, STREAM[0]) and lists.decode(STREAM[0])
+    rt.fake_stream_capturing(STREAM[0], 0)
+    assert rt.nrldpc_set_neighbours(hs[0].h, 5) == 0 and not hs[0].decode(40, STREAM[0])
+    assert rt.nrldpc_set_neighbours(hs[0].h, -1) == 0 and hs[0].decode(40, STREAM[0])
+    assert rt.nrldpc_set_neighbours(hs[0].h, -2) == -1  # NRLDPC_ERR_INVALID_ARG
+    lists.close()
+    for h in hs:
+        h.close()
