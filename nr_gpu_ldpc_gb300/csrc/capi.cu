@@ -25,6 +25,14 @@ struct Flights {
 };
 std::mutex g_flights_mu;
 std::map<int, Flights> g_flights;  // a device's entry goes with its last decoder
+
+// true also where that cannot be told
+bool is_captured(cudaStream_t stream, bool pending) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+    if (!pending) cudaGetLastError();
+    return true;
+}
 }  // namespace
 
 bool in_flight_join(InFlight* me, int device) {
@@ -53,11 +61,10 @@ int in_flight_others(const InFlight* me, cudaStream_t stream, long sms, int sm_c
     Flights& d = g_flights[me->device];
     const int others = static_cast<int>(d.live.size()) - 1;
     if (others < 1 || sms * (others + 1L) <= sm_count) return 0;
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
-        cudaGetLastError();
-        return others;
-    }
+    // an error of the caller's that it has not read yet stays for it to read
+    const bool pending = cudaPeekAtLastError() != cudaSuccess;
+    if (is_captured(stream, pending)) return others;
+    if (pending) return std::min(d.crowd, others);  // a query's not-ready would take its place
     // a query must not disturb a capture of another thread
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     cudaThreadExchangeStreamCaptureMode(&mode);
@@ -81,12 +88,11 @@ void in_flight_note(InFlight* me, cudaStream_t stream) {
     Flights& d = g_flights[me->device];
     if (d.live.size() < 2) return;
     d.last = me;
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone &&
-        cudaEventRecord(me->done, stream) == cudaSuccess)
-        me->recorded = true, me->stream = stream;
-    else
-        cudaGetLastError();
+    const bool pending = cudaPeekAtLastError() != cudaSuccess;
+    if (is_captured(stream, pending)) return;
+    me->recorded = cudaEventRecord(me->done, stream) == cudaSuccess;
+    me->stream = stream;
+    if (!me->recorded && !pending) cudaGetLastError();
 }
 }  // namespace nrldpc
 

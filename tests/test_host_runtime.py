@@ -195,3 +195,18 @@ def test_captured_calls_presume_the_other_decoders_beside_them(rt):
     lists.close()
     for h in hs:
         h.close()
+
+
+def test_error_of_the_caller_survives_a_decode(rt):
+    hs = [Handle(rt) for _ in range(6)]
+    for k, h in enumerate(hs):
+        h.decode(40, STREAM[k])
+        rt.fake_stream_busy(STREAM[k], 1)
+    rt.fake_set_error(1)  # cudaErrorInvalidValue of an earlier call
+    hs[0].decode(40, 0x700)
+    assert rt.fake_peek_error() == 1
+    rt.fake_set_error(0)
+    hs[0].decode(40, 0x700)
+    assert rt.fake_peek_error() == 0  # and none of the decoder's own
+    for h in hs:
+        h.close()
