@@ -901,24 +901,26 @@ size_t wms_smem_bytes(const CodeTable& tab, int cpb, bool layered) {
 
 namespace {
 // kernel k of the degree class: 0 forward flooding, 1 forward layered,
-// 2 adjoint flooding, 3 adjoint layered
+// 2 adjoint flooding, 3 adjoint layered.  BG1's flooding adjoint is the general
+// one: the class's compiled form is slower (BG1 Z=384 1,000 x 6 it., us: 2973
+// with the general kernels, 3287 with the class's, 2952 with its forward and the
+// general adjoint).
 template <RowClass CLASS, int MAXD>
 const void* wms_kernel(int k) {
+    constexpr RowClass kFloodingAdjoint = CLASS == RowClass::kBg1 ? RowClass::kAny : CLASS;
     switch (k) {
         case 0: return reinterpret_cast<const void*>(&wms_forward_kernel<CLASS, MAXD, false>);
         case 1: return reinterpret_cast<const void*>(&wms_forward_kernel<CLASS, MAXD, true>);
-        case 2: return reinterpret_cast<const void*>(&wms_backward_kernel<CLASS, MAXD>);
+        case 2: return reinterpret_cast<const void*>(&wms_backward_kernel<kFloodingAdjoint, MAXD>);
         default: return reinterpret_cast<const void*>(&wms_backward_layered_kernel<CLASS, MAXD>);
     }
 }
 // The kernels for the code's class of rows (forward and adjoint, us: BG2 Z=128
 // 4,096 codewords x 8 it. flooding 3481 -> 3343, BG1 Z=384 512 x 6 layered 1946
-// -> 1880), but BG1's flooding adjoint, whose compiled form for the class is
-// slower: BG1 Z=384 1,000 x 6 it. 2973 with the general kernels, 3287 with the
-// class's, 2952 with its forward and the general adjoint.
+// -> 1880).
 const void* wms_kernel_for(const CodeTable& tab, int k) {
     switch (row_class(tab)) {
-        case RowClass::kBg1: return k == 2 ? wms_kernel<RowClass::kAny, 19>(k) : wms_kernel<RowClass::kBg1, 19>(k);
+        case RowClass::kBg1: return wms_kernel<RowClass::kBg1, 19>(k);
         case RowClass::kBg2: return wms_kernel<RowClass::kBg2, 10>(k);
         default: return max_row_degree(tab) <= 10 ? wms_kernel<RowClass::kAny, 10>(k) : wms_kernel<RowClass::kAny, 19>(k);
     }
