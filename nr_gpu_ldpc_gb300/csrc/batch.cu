@@ -294,18 +294,17 @@ struct Batch {
     int32_t* d_order = nullptr;
     WorkItem* d_items = nullptr;
     int derate_parts = 1, derate_part = 256;
-    // few jobs: one codeword on a cluster of CTAs (split.cu).  Plans are made
-    // when a job list first needs them and kept (102 codes x 8 cluster sizes,
-    // 10 KB each, at most); split: the current list's launch, ranks 0: none
+    // few jobs: one codeword on a cluster of CTAs (split.cu).  A plan's tables
+    // are made when a job list first runs on it, and kept; split: the current
+    // list's launch, ranks 0: none
     struct Plan {
-        int state = 0;  // 1: made, -1: the code does not fit such clusters
-        int32_t at = 0;
+        int state = 0;  // 1: head known, -1: the code does not fit such clusters
+        int32_t at = -1;  // its place in d_plans_split
         SplitHead head;
     };
     std::vector<Plan> plans;  // [code][cluster size]
-    std::vector<unsigned char> h_plans;
     unsigned char* d_plans_split = nullptr;
-    size_t plans_room = 0, plans_sent = 0;
+    size_t plans_bytes = 0;
     SplitJob* d_split = nullptr;
     SplitHead split{};
     int split_clusters = 0;
@@ -322,6 +321,10 @@ struct Batch {
     cudaGraphNode_t knode = nullptr;
     BatchDecodeArgs kargs{};
 };
+
+// Room for the plans of every code and cluster size (6.6 MB), so that no list
+// allocates or frees device memory for them.
+constexpr size_t kPlansRoom = 8u << 20;
 
 constexpr size_t kListBytes =
     sizeof(JobDev) + sizeof(nrldpc_job) + sizeof(int32_t) + sizeof(WorkItem) + sizeof(SplitJob);
@@ -403,6 +406,7 @@ int choose_split(Batch* b, const std::vector<int32_t>& order, const std::vector<
                  std::vector<SplitJob>* jobs) {
     static const int kRoom[kSplitSizes] = {7, 13, 23, 28, 36, 46, 76, 152};  // at one CTA per SM of 152
     const int n = static_cast<int>(order.size());
+    SplitDeal deal;
     if (n > 2L * kRoom[kSplitSizes - 1] * b->sm_count / 152) return NRLDPC_OK;
     long fused_sum = 0, least = 0;
     for (const WorkItem& it : items) {
@@ -428,8 +432,8 @@ int choose_split(Batch* b, const std::vector<int32_t>& order, const std::vector<
             const int code = b->h_jobs[order[i]].code;
             Batch::Plan& p = b->plans[code * kSplitSizes + s];
             if (p.state == 0) {
-                p.at = static_cast<int32_t>(b->h_plans.size());
-                p.state = make_split_plan(b->h_tables[code], ranks, b->smem_optin, &p.head, &b->h_plans) ? 1 : -1;
+                p.state = deal_split(b->h_tables[code], ranks, b->smem_optin, &deal) ? 1 : -1;
+                if (p.state > 0) p.head = deal.head;
             }
             fits = p.state > 0;
             launch.warps = std::max(launch.warps, p.head.warps);
@@ -450,19 +454,25 @@ int choose_split(Batch* b, const std::vector<int32_t>& order, const std::vector<
         if (room >= n) break;
     }
     if (best < 0) return NRLDPC_OK;
-    if (b->h_plans.size() > b->plans_room) {  // grows with the codes seen
-        cudaFree(b->d_plans_split);
-        b->d_plans_split = nullptr;
-        b->plans_room = b->plans_sent = 0;
-        const size_t room = 2 * b->h_plans.size();
-        if (cudaMalloc(&b->d_plans_split, room) != cudaSuccess) return NRLDPC_ERR_NO_MEMORY;
-        b->plans_room = room;
+    std::vector<unsigned char> fresh;  // tables that no list has run on yet
+    std::vector<Batch::Plan*> placed;
+    for (const int32_t j : order) {
+        const CodeTable& t = b->h_tables[b->h_jobs[j].code];
+        Batch::Plan& p = b->plans[b->h_jobs[j].code * kSplitSizes + best];
+        if (p.at >= 0) continue;
+        p.at = static_cast<int32_t>(b->plans_bytes + fresh.size());
+        placed.push_back(&p);
+        if (deal_split(t, kSplitRanks[best], b->smem_optin, &deal)) make_split_plan(t, deal, &fresh);
     }
-    if (b->plans_sent < b->h_plans.size()) {
-        if (cudaMemcpy(b->d_plans_split + b->plans_sent, b->h_plans.data() + b->plans_sent,
-                       b->h_plans.size() - b->plans_sent, cudaMemcpyHostToDevice) != cudaSuccess)
-            return NRLDPC_ERR_CUDA;
-        b->plans_sent = b->h_plans.size();
+    if (!fresh.empty()) {
+        const bool room = b->plans_bytes + fresh.size() <= kPlansRoom;
+        if (!room || cudaMemcpy(b->d_plans_split + b->plans_bytes, fresh.data(), fresh.size(),
+                                cudaMemcpyHostToDevice) != cudaSuccess) {
+            for (Batch::Plan* p : placed) p->at = -1;
+            b->split.ranks = 0;  // the persistent kernel needs none
+            return room ? NRLDPC_ERR_CUDA : NRLDPC_OK;
+        }
+        b->plans_bytes += fresh.size();
     }
     const Batch::Plan& first = b->plans[b->h_jobs[order[0]].code * kSplitSizes + best];
     b->split_count_at = first.at + sizeof(SplitHead) + first.head.o_bytes;
@@ -529,6 +539,7 @@ int nrldpc_batch_create(int device, int max_jobs, float alpha, nrldpc_batch** ou
     if (cudaMalloc(&b->d_tables, sizeof(CodeTable) * kNumCodes) != cudaSuccess ||
         cudaMalloc(&b->d_plans, sizeof(PlanDev) * kNumCodes) != cudaSuccess ||
         cudaMalloc(&b->d_lists, kListBytes * max_jobs + 5 * 256) != cudaSuccess ||
+        cudaMalloc(&b->d_plans_split, kPlansRoom) != cudaSuccess ||
         cudaMalloc(&b->d_scratch, 256) != cudaSuccess) {
         free_batch(b);
         return NRLDPC_ERR_NO_MEMORY;

@@ -257,28 +257,6 @@ void free_handle(Handle* h) {
     delete h;
 }
 
-// Plans for the cluster sizes that fit; their bytes go behind the handle's
-// scratch words in device memory.
-int split_prepare(Handle* h, size_t smem_limit, std::vector<unsigned char>* bytes) {
-    if (split_kernel_attributes(smem_limit) != cudaSuccess) return NRLDPC_ERR_CUDA;
-    const int tasks = h->tab.rows * ((h->tab.z + 31) / 32);
-    for (int ranks : kSplitRanks) {
-        if (ranks > 1 && tasks < ranks * kSplitMinTasks) continue;
-        SplitHead p;
-        const size_t at = bytes->size();
-        if (!make_split_plan(h->tab, ranks, smem_limit, &p, bytes)) continue;
-        const int room = split_max_clusters(p);
-        if (room < 1) {
-            bytes->resize(at);
-            continue;
-        }
-        h->split.push_back(p);
-        h->split_room.push_back(room);
-        h->split_at.push_back(at);
-    }
-    return NRLDPC_OK;
-}
-
 // Plan for n codewords, or -1 for decode_kernel: the smaller of two time
 // estimates (split_cost, fused_row_walk).  GB300 times, 10 iterations without
 // early stop, us (model): BG1 Z=384 on 16 / 10 / 4 / 3 CTAs 43 / 52 / 95 / 148
@@ -308,6 +286,43 @@ int split_choice(const Handle* h, int n) {
         }
     }
     return best;
+}
+
+// Plans for the cluster sizes that some batch can pick, of up to eight decoders
+// side by side; their bytes go behind the handle's scratch words in device
+// memory.  They are part of a handle's creation: BG1 Z=384 for 40 codewords 679
+// us with the tables of every size, 494 with these, 419 without plans.
+int split_prepare(Handle* h, size_t smem_limit, std::vector<unsigned char>* bytes) {
+    if (split_kernel_attributes(smem_limit) != cudaSuccess) return NRLDPC_ERR_CUDA;
+    const int tasks = h->tab.rows * ((h->tab.z + 31) / 32);
+    std::vector<SplitDeal> deals;
+    deals.reserve(kSplitSizes);
+    for (int ranks : kSplitRanks) {
+        if (ranks > 1 && tasks < ranks * kSplitMinTasks) continue;
+        deals.emplace_back();
+        const int room = deal_split(h->tab, ranks, smem_limit, &deals.back()) ? split_max_clusters(deals.back().head) : 0;
+        if (room < 1) {
+            deals.pop_back();
+            continue;
+        }
+        h->split.push_back(deals.back().head);
+        h->split_room.push_back(room);
+    }
+    bool picked[kSplitSizes] = {};
+    const long most = std::min(8L * h->max_batch, 8L * h->sm_count);
+    for (int n = 1; n <= most; n++)
+        if (const int k = split_choice(h, n); k >= 0) picked[k] = true;
+    size_t kept = 0;
+    for (size_t k = 0; k < deals.size(); k++) {
+        if (!picked[k]) continue;
+        h->split[kept] = h->split[k];
+        h->split_room[kept++] = h->split_room[k];
+        h->split_at.push_back(bytes->size());
+        make_split_plan(h->tab, deals[k], bytes);
+    }
+    h->split.resize(kept);
+    h->split_room.resize(kept);
+    return NRLDPC_OK;
 }
 
 SplitArgs split_args(const Handle* h, int plan, const float* llr, uint8_t* packed, int n_cw, int n_iter) {

@@ -224,8 +224,20 @@ inline long split_cost(const SplitHead& h) { return 667L * h.phases + h.load; }
 inline long fused_row_walk(const CodeTable& t, long warps) {
     return t.rows * (29 + 21 * warps / 10) + t.n_edges * (81 + 4 * warps) / 10;
 }
-bool make_split_plan(const CodeTable& tab, int ranks, size_t smem_limit, SplitHead* head,
-                     std::vector<unsigned char>* out);
+// Which CTA owns which base row and core column.
+struct SplitDeal {
+    SplitHead head;
+    uint8_t col_deg[kMaxCols], col_row[kMaxCols][kMaxRows];  // each column's rows and edges, ascending
+    uint16_t col_edge[kMaxCols][kMaxRows];
+    uint8_t col_rank[kMaxCols], row_rank[kMaxRows], row_at[kMaxRows];  // owners; a row's place there
+    uint8_t cols[kSplitMaxRanks][kMaxCols], rows[kSplitMaxRanks][kMaxRows];  // of each rank, in order
+    int n_cols[kSplitMaxRanks], n_rows[kSplitMaxRanks];
+    int row_beg[kSplitMaxRanks][kSplitMaxPhases + 1];  // first row of each phase
+    int col_beg[kMaxCols][kSplitMaxPhases], col_cnt[kMaxCols][kSplitMaxPhases];  // a column's dt places per phase
+    int dt_of[kMaxEdges], n_dt[kSplitMaxRanks][kSplitMaxPhases];
+};
+bool deal_split(const CodeTable& tab, int ranks, size_t smem_limit, SplitDeal* deal);
+void make_split_plan(const CodeTable& tab, const SplitDeal& deal, std::vector<unsigned char>* out);
 cudaError_t split_kernel_attributes(size_t smem);
 int split_max_clusters(const SplitHead& head);  // resident at once
 bool split_counts(const SplitHead& head, int early_stop);  // whether its passes wait for counted bytes

@@ -561,48 +561,74 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
     }
 }
 
-// Lists of task[i] (cost[i], largest first) for n_bins warps, each task to
-// the least loaded: ptr[0..n_bins] and the tasks bin by bin.
-void spread(const std::vector<std::pair<int, int>>& tasks, int n_bins, int from, uint16_t* ptr, uint16_t* out) {
-    int load[kSplitMaxWarps] = {0}, count[kSplitMaxWarps + 1] = {0}, bin[kMaxCols * 12];
-    for (size_t i = 0; i < tasks.size(); i++) {
-        int b = 0;
-        for (int j = 1; j < n_bins; j++)
-            if (load[j] < load[b]) b = j;
-        bin[i] = b;
-        load[b] += tasks[i].first;
-        count[b + 1]++;
-    }
+// Task lists of n_bins warps: items in the order given (largest cost first),
+// each `chunks` tasks of its cost, every task to the least loaded warp (the
+// first of several).  ptr[0..n_bins] and the tasks (item << 4 | chunk) bin by
+// bin, from out[from] on; returns the end.
+int spread(const uint8_t* items, const int* cost, int n, int chunks, int n_bins, int from, uint16_t* ptr,
+           uint16_t* out) {
+    constexpr int kLoads = 2048;  // above any load: an even share and one task (asserted below)
+    uint32_t at_load[kLoads] = {0};  // the warps that have this load
+    int count[kSplitMaxWarps + 1] = {0}, least = 0;
+    uint8_t bin[kMaxCols * 12];
+    at_load[0] = (1u << n_bins) - 1u;
+    for (int i = 0, task = 0; i < n; i++)
+        for (int c = 0; c < chunks; c++, task++) {
+            while (!at_load[least]) least++;
+            const int b = __builtin_ctz(at_load[least]);
+            at_load[least] &= at_load[least] - 1;
+            at_load[least + cost[i]] |= 1u << b;
+            bin[task] = static_cast<uint8_t>(b);
+            count[b + 1]++;
+        }
+    static_assert(kMaxCols * 12 * (kMaxRows + kSplitColCost) / kSplitMaxWarps + kMaxRows + kSplitColCost < kLoads,
+                  "the columns' tasks; the rows' are fewer and cost less");
     for (int b = 0; b < n_bins; b++) {
         count[b + 1] += count[b];
         ptr[b] = static_cast<uint16_t>(from + count[b]);
     }
     ptr[n_bins] = static_cast<uint16_t>(from + count[n_bins]);
-    for (size_t i = 0; i < tasks.size(); i++) out[from + count[bin[i]]++] = static_cast<uint16_t>(tasks[i].second);
+    for (int i = 0, task = 0; i < n; i++)
+        for (int c = 0; c < chunks; c++, task++)
+            out[from + count[bin[task]]++] = static_cast<uint16_t>(items[i] << 4 | c);
+    return from + n * chunks;
 }
+static_assert(kSplitMaxWarps < 32 && kMaxRows <= kMaxCols && kMaxDeg + kSplitRowCost <= kMaxRows + kSplitColCost,
+              "a bit per warp; rows' tasks within the bounds of columns'");
 
 }  // namespace
 
-// Rows and columns to CTAs, tasks to warps and the shared-memory layout for
-// clusters of `ranks` CTAs: appends the head and one table image per rank to
-// `out`.  False when the code does not fit such clusters.
-bool make_split_plan(const CodeTable& t, int ranks, size_t smem_limit, SplitHead* head,
-                     std::vector<unsigned char>* out) {
+// Rows and columns to CTAs and the shared-memory layout, first half of a plan:
+// enough to compare cluster sizes by.  False when the code does not fit
+// clusters of `ranks` CTAs.
+bool deal_split(const CodeTable& t, int ranks, size_t smem_limit, SplitDeal* deal) {
+    SplitDeal& d = *deal;
     const int chunks = (t.z + 31) / 32, rows = t.rows, nc = t.n_core;
-    int core[kMaxRows], col_deg[kMaxCols] = {0}, col_row[kMaxCols][kMaxRows], col_edge[kMaxCols][kMaxRows], total = 0;
+    auto share = [ranks](int n) { return static_cast<size_t>((n + ranks - 1) / ranks); };
+    // the posteriors and an even share of the states have to fit whatever the phases
+    const size_t least = kSplitHeader + 4 * static_cast<size_t>(t.core_floats) + 16 * share(rows) * t.z;
+    if (least > smem_limit) return false;
+    int core[kMaxRows], total = 0, row_order[kMaxRows];
+    uint8_t col_order[kMaxCols];
+    std::memset(d.col_deg, 0, sizeof(d.col_deg));
     for (int r = 0; r < rows; r++) {  // rows and edges of each column, ascending
         core[r] = t.row_deg[r] - (t.row_sfx[r] ? 1 : 0);
         total += core[r];
+        row_order[r] = r;
         for (int e = t.row_ptr[r]; e < t.row_ptr[r + 1]; e++) {
             const int c = t.edge_col[e];
-            col_row[c][col_deg[c]] = r;
-            col_edge[c][col_deg[c]++] = e;
+            d.col_row[c][d.col_deg[c]] = static_cast<uint8_t>(r);
+            d.col_edge[c][d.col_deg[c]++] = static_cast<uint16_t>(e);
         }
     }
-    // the posteriors and an even share of the states have to fit whatever the phases
-    if (4 * static_cast<size_t>(t.core_floats) + 16 * static_cast<size_t>((rows + ranks - 1) / ranks) * t.z > smem_limit)
-        return false;
+    for (int c = 0; c < nc; c++) col_order[c] = static_cast<uint8_t>(c);
+    std::stable_sort(col_order, col_order + nc, [&](int x, int y) { return d.col_deg[x] > d.col_deg[y]; });
+    std::stable_sort(row_order, row_order + rows, [&](int x, int y) { return t.row_deg[x] > t.row_deg[y]; });
     for (int P = 1; P <= kSplitMaxPhases && P <= rows; P++) {
+        // nor can even shares of the dt, the edges and (phases) the sums that do not fit
+        if (least + 4 * share((total + P - 1) / P) * t.z + 16 * share(t.n_edges) + (P > 1 ? 128 * share(nc) * chunks : 0) >
+            smem_limit)
+            continue;
         // phases: contiguous rows, about the same edges each
         int phase_of[kMaxRows], sum = 0;
         for (int r = 0; r < rows; r++) {
@@ -611,64 +637,55 @@ bool make_split_plan(const CodeTable& t, int ranks, size_t smem_limit, SplitHead
         }
         // columns to ranks, largest degree first, to the rank with the least
         // dt; dt places of a column's edges, ascending rows, per phase
-        int col_rank[kMaxCols], col_beg[kMaxCols][kSplitMaxPhases], col_cnt[kMaxCols][kSplitMaxPhases];
-        int dt_of[kMaxEdges], deg_sum[kSplitMaxRanks] = {0}, dt[kSplitMaxRanks][kSplitMaxPhases] = {{0}}, max_dt = 0;
-        std::vector<int> cols(nc), local_cols[kSplitMaxRanks];
-        for (int c = 0; c < nc; c++) cols[c] = c;
-        std::stable_sort(cols.begin(), cols.end(), [&](int x, int y) { return col_deg[x] > col_deg[y]; });
-        for (int c : cols) {
+        int deg_sum[kSplitMaxRanks] = {0}, max_dt = 0;
+        std::memset(d.n_dt, 0, sizeof(d.n_dt));
+        std::memset(d.n_cols, 0, sizeof(d.n_cols));
+        for (int i = 0; i < nc; i++) {
+            const int c = col_order[i];
             int k = 0;
             for (int j = 1; j < ranks; j++)
                 if (deg_sum[j] < deg_sum[k]) k = j;
-            col_rank[c] = k;
-            deg_sum[k] += col_deg[c] + kSplitColCost;
-            local_cols[k].push_back(c);
-            for (int p = 0; p < P; p++) col_beg[c][p] = dt[k][p];
-            for (int i = 0; i < col_deg[c]; i++) dt_of[col_edge[c][i]] = dt[k][phase_of[col_row[c][i]]]++;
+            d.col_rank[c] = static_cast<uint8_t>(k);
+            deg_sum[k] += d.col_deg[c] + kSplitColCost;
+            d.cols[k][d.n_cols[k]++] = static_cast<uint8_t>(c);
+            for (int p = 0; p < P; p++) d.col_beg[c][p] = d.n_dt[k][p];
+            for (int j = 0; j < d.col_deg[c]; j++) d.dt_of[d.col_edge[c][j]] = d.n_dt[k][phase_of[d.col_row[c][j]]]++;
             for (int p = 0; p < P; p++) {
-                col_cnt[c][p] = dt[k][p] - col_beg[c][p];
-                max_dt = std::max(max_dt, dt[k][p]);
+                d.col_cnt[c][p] = d.n_dt[k][p] - d.col_beg[c][p];
+                max_dt = std::max(max_dt, d.n_dt[k][p]);
             }
         }
         // rows of a phase to ranks, largest degree first, to the rank with
         // the least work in the phase (then the fewest rows so far)
-        int row_rank[kMaxRows], row_at[kMaxRows];
-        std::vector<int> local_rows[kSplitMaxRanks];
-        std::vector<std::pair<int, int>> list[kSplitMaxRanks][kSplitMaxPhases];
-        int busiest = 0;  // summed over the phases
+        std::memset(d.n_rows, 0, sizeof(d.n_rows));
+        int busiest = 0, most = 0;  // work summed over the phases, rows of a rank's phase
         for (int p = 0; p < P; p++) {
-            std::vector<int> order;
-            for (int r = 0; r < rows; r++)
-                if (phase_of[r] == p) order.push_back(r);
-            std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return t.row_deg[x] > t.row_deg[y]; });
             int load[kSplitMaxRanks] = {0};
-            for (int r : order) {
+            for (int k = 0; k < ranks; k++) d.row_beg[k][p] = d.n_rows[k];
+            for (int i = 0; i < rows; i++) {
+                const int r = row_order[i];
+                if (phase_of[r] != p) continue;
                 int k = 0;
                 for (int j = 1; j < ranks; j++)
-                    if (load[j] < load[k] || (load[j] == load[k] && local_rows[j].size() < local_rows[k].size())) k = j;
-                row_rank[r] = k;
-                row_at[r] = static_cast<int>(local_rows[k].size());
-                local_rows[k].push_back(r);
+                    if (load[j] < load[k] || (load[j] == load[k] && d.n_rows[j] < d.n_rows[k])) k = j;
+                d.row_rank[r] = static_cast<uint8_t>(k);
+                d.row_at[r] = static_cast<uint8_t>(d.n_rows[k]);
+                d.rows[k][d.n_rows[k]++] = static_cast<uint8_t>(r);
                 load[k] += t.row_deg[r] + kSplitRowCost;
-                for (int c = 0; c < chunks; c++)
-                    list[k][p].push_back({t.row_deg[r] + kSplitRowCost, (row_at[r] << 4) | c});
             }
+            for (int k = 0; k < ranks; k++) most = std::max(most, d.n_rows[k] - d.row_beg[k][p]);
             busiest += chunks * *std::max_element(load, load + ranks);
         }
-        size_t n_rows = 0, n_cols = 0, most = 0, n_edges = 0, n_cn = 0;
+        size_t n_rows = 0, n_cols = 0, n_edges = 0;
         for (int k = 0; k < ranks; k++) {
-            size_t e = 0, cn = 0;
-            for (int r : local_rows[k]) e += t.row_deg[r];
-            for (int p = 0; p < P; p++) {
-                most = std::max(most, list[k][p].size());
-                cn += list[k][p].size();
-            }
+            size_t e = 0;
+            for (int i = 0; i < d.n_rows[k]; i++) e += t.row_deg[d.rows[k][i]];
+            d.row_beg[k][P] = d.n_rows[k];
             n_edges = std::max(n_edges, e);
-            n_cn = std::max(n_cn, cn);
-            n_rows = std::max(n_rows, local_rows[k].size());
-            n_cols = std::max(n_cols, local_cols[k].size());
+            n_rows = std::max(n_rows, static_cast<size_t>(d.n_rows[k]));
+            n_cols = std::max(n_cols, static_cast<size_t>(d.n_cols[k]));
         }
-        const int W = std::max(4, std::min(kSplitMaxWarps, static_cast<int>(std::max(most, n_cols * chunks))));
+        const int W = std::max(4, std::min(kSplitMaxWarps, std::max(most, static_cast<int>(n_cols)) * chunks));
         // image layout (the same for every rank) and shared memory
         size_t at = 0;
         auto take = [&](size_t bytes) {
@@ -693,87 +710,92 @@ bool make_split_plan(const CodeTable& t, int ranks, size_t smem_limit, SplitHead
         h.o_beg = take(4 * n_cols * P);
         h.o_own = take(4 * static_cast<size_t>(t.cols));
         h.o_cnptr = take(2 * (static_cast<size_t>(P) * W + 1));
-        h.o_cn = take(2 * n_cn);
+        h.o_cn = take(2 * n_rows * chunks);
         h.o_vnptr = take(2 * (static_cast<size_t>(W) + 1));
         h.o_vn = take(2 * n_cols * chunks);
         h.o_bytes = take(8);
         h.image_bytes = static_cast<int>(at);
         auto up = [](size_t x) { return (x + 127) / 128 * 128; };
         const size_t l = up(kSplitHeader + at), st = up(l + 4 * static_cast<size_t>(t.core_floats)),
-                     d = up(st + 16 * n_rows * t.z), acc = up(d + 4 * static_cast<size_t>(max_dt) * t.z),
+                     dt = up(st + 16 * n_rows * t.z), acc = up(dt + 4 * static_cast<size_t>(max_dt) * t.z),
                      end = acc + (P > 1 ? 128 * n_cols * chunks : 0);
         if (end > smem_limit) continue;
         h.off_l = static_cast<int>(l);
         h.off_state = static_cast<int>(st);
-        h.off_dt = static_cast<int>(d);
+        h.off_dt = static_cast<int>(dt);
         h.off_acc = static_cast<int>(acc);
         h.smem = static_cast<int>(end);
-        // the images
-        const size_t base = out->size();
-        out->resize(base + sizeof(SplitHead) + static_cast<size_t>(ranks) * at, 0);
-        std::memcpy(out->data() + base, &h, sizeof(h));
-        for (int k = 0; k < ranks; k++) {
-            unsigned char* im = out->data() + base + sizeof(SplitHead) + static_cast<size_t>(k) * at;
-            auto* edge = reinterpret_cast<uint4*>(im + h.o_edge);
-            auto* row = reinterpret_cast<uint4*>(im + h.o_row);
-            auto* col = reinterpret_cast<uint4*>(im + h.o_col);
-            auto* beg = reinterpret_cast<uint32_t*>(im + h.o_beg);
-            auto* own = reinterpret_cast<uint32_t*>(im + h.o_own);
-            auto* cnptr = reinterpret_cast<uint16_t*>(im + h.o_cnptr);
-            auto* cn = reinterpret_cast<uint16_t*>(im + h.o_cn);
-            auto* vnptr = reinterpret_cast<uint16_t*>(im + h.o_vnptr);
-            auto* vn = reinterpret_cast<uint16_t*>(im + h.o_vn);
-            uint32_t m = 0;
-            for (size_t i = 0; i < local_rows[k].size(); i++) {
-                const int r = local_rows[k][i], last = t.row_ptr[r + 1] - 1;
-                row[i] = make_uint4(m | (static_cast<uint32_t>(t.row_ptr[r]) << 16), static_cast<uint32_t>(i) * t.z,
-                                    ((static_cast<uint32_t>(t.edge_col[last]) * t.z) << 9) | t.edge_shift[last],
-                                    t.row_deg[r] | (t.row_sfx[r] ? 256u : 0u));
-                for (int e = t.row_ptr[r]; e <= last; e++, m++) {
-                    const int c = t.edge_col[e];
-                    edge[m] = make_uint4(t.eaddr[e].x, t.eaddr[e].y, 0u, 0u);
-                    if (c < nc) edge[m].z = (static_cast<uint32_t>(col_rank[c]) << 24) | static_cast<uint32_t>(dt_of[e]);
-                }
-            }
-            std::vector<std::pair<int, int>> vl;
-            for (size_t i = 0; i < local_cols[k].size(); i++) {
-                const int c = local_cols[k][i];
-                uint32_t need = 1u << k;  // its owner (for the output) and every rank with a row that reads it
-                for (int j = 0; j < col_deg[c]; j++) need |= 1u << row_rank[col_row[c][j]];
-                col[i] = make_uint4(4u * static_cast<uint32_t>(c) * t.z, need, 0u, 0u);
-                for (int p = 0; p < P; p++)
-                    beg[i * P + p] = static_cast<uint32_t>(col_beg[c][p]) | (static_cast<uint32_t>(col_cnt[c][p]) << 16);
-                for (int j = 0; j < chunks; j++)
-                    vl.push_back({col_deg[c] + kSplitColCost, (static_cast<int>(i) << 4) | j});
-            }
-            for (int c = 0; c < nc; c++) own[c] = static_cast<uint32_t>(col_rank[c]) << 28;
-            for (int c = nc; c < t.cols; c++) {
-                const int r = t.sfx_row[c];
-                own[c] = (static_cast<uint32_t>(row_rank[r]) << 28) | (static_cast<uint32_t>(row_at[r] * t.z) << 9) |
-                         t.edge_shift[t.row_ptr[r + 1] - 1];
-            }
-            int n = 0;
-            for (int p = 0; p < P; p++) {
-                spread(list[k][p], W, n, cnptr + p * W, cn);
-                n += static_cast<int>(list[k][p].size());
-            }
-            spread(vl, W, 0, vnptr, vn);
-            // bytes that reach the rank in a one-phase iteration: dt of its
-            // columns, posteriors that its rows or its output read
-            auto* bytes = reinterpret_cast<uint32_t*>(im + h.o_bytes);
-            bytes[0] = 4u * static_cast<uint32_t>(t.z) * static_cast<uint32_t>(dt[k][0]);
-            uint32_t n_read = 0;
-            for (int c = 0; c < nc; c++) {
-                bool reads = col_rank[c] == k;
-                for (int j = 0; j < col_deg[c]; j++) reads |= row_rank[col_row[c][j]] == k;
-                n_read += reads;
-            }
-            bytes[1] = 4u * static_cast<uint32_t>(t.z) * n_read;
-        }
-        *head = h;
+        d.head = h;
         return true;
     }
     return false;
+}
+
+// Second half: the head and one table image per rank, appended to `out`.
+void make_split_plan(const CodeTable& t, const SplitDeal& d, std::vector<unsigned char>* out) {
+    const SplitHead& h = d.head;
+    const int chunks = (t.z + 31) / 32, nc = t.n_core, ranks = h.ranks, P = h.phases, W = h.warps;
+    const size_t base = out->size(), at = static_cast<size_t>(h.image_bytes);
+    out->resize(base + sizeof(SplitHead) + ranks * at, 0);
+    std::memcpy(out->data() + base, &h, sizeof(h));
+    int row_cost[kMaxRows], col_cost[kMaxCols];
+    uint8_t index[kMaxCols];
+    uint32_t need[kMaxCols];  // every rank that reads a column: its owner, for the output, and those with a row on it
+    for (int c = 0; c < nc; c++) {
+        need[c] = 1u << d.col_rank[c];
+        for (int j = 0; j < d.col_deg[c]; j++) need[c] |= 1u << d.row_rank[d.col_row[c][j]];
+    }
+    for (int c = 0; c < kMaxCols; c++) index[c] = static_cast<uint8_t>(c);
+    for (int k = 0; k < ranks; k++) {
+        unsigned char* im = out->data() + base + sizeof(SplitHead) + k * at;
+        auto* edge = reinterpret_cast<uint4*>(im + h.o_edge);
+        auto* row = reinterpret_cast<uint4*>(im + h.o_row);
+        auto* col = reinterpret_cast<uint4*>(im + h.o_col);
+        auto* beg = reinterpret_cast<uint32_t*>(im + h.o_beg);
+        auto* own = reinterpret_cast<uint32_t*>(im + h.o_own);
+        auto* cnptr = reinterpret_cast<uint16_t*>(im + h.o_cnptr);
+        auto* cn = reinterpret_cast<uint16_t*>(im + h.o_cn);
+        auto* vnptr = reinterpret_cast<uint16_t*>(im + h.o_vnptr);
+        auto* vn = reinterpret_cast<uint16_t*>(im + h.o_vn);
+        uint32_t m = 0;
+        for (int i = 0; i < d.n_rows[k]; i++) {
+            const int r = d.rows[k][i], last = t.row_ptr[r + 1] - 1;
+            row_cost[i] = t.row_deg[r] + kSplitRowCost;
+            row[i] = make_uint4(m | (static_cast<uint32_t>(t.row_ptr[r]) << 16), static_cast<uint32_t>(i) * t.z,
+                                ((static_cast<uint32_t>(t.edge_col[last]) * t.z) << 9) | t.edge_shift[last],
+                                t.row_deg[r] | (t.row_sfx[r] ? 256u : 0u));
+            for (int e = t.row_ptr[r]; e <= last; e++, m++) {
+                const int c = t.edge_col[e];
+                edge[m] = make_uint4(t.eaddr[e].x, t.eaddr[e].y, 0u, 0u);
+                if (c < nc) edge[m].z = (static_cast<uint32_t>(d.col_rank[c]) << 24) | static_cast<uint32_t>(d.dt_of[e]);
+            }
+        }
+        for (int i = 0; i < d.n_cols[k]; i++) {
+            const int c = d.cols[k][i];
+            col_cost[i] = d.col_deg[c] + kSplitColCost;
+            col[i] = make_uint4(4u * static_cast<uint32_t>(c) * t.z, need[c], 0u, 0u);
+            for (int p = 0; p < P; p++)
+                beg[i * P + p] = static_cast<uint32_t>(d.col_beg[c][p]) | (static_cast<uint32_t>(d.col_cnt[c][p]) << 16);
+        }
+        for (int c = 0; c < nc; c++) own[c] = static_cast<uint32_t>(d.col_rank[c]) << 28;
+        for (int c = nc; c < t.cols; c++) {
+            const int r = t.sfx_row[c];
+            own[c] = (static_cast<uint32_t>(d.row_rank[r]) << 28) | (static_cast<uint32_t>(d.row_at[r] * t.z) << 9) |
+                     t.edge_shift[t.row_ptr[r + 1] - 1];
+        }
+        for (int p = 0, n = 0; p < P; p++) {
+            const int from = d.row_beg[k][p];
+            n = spread(index + from, row_cost + from, d.row_beg[k][p + 1] - from, chunks, W, n, cnptr + p * W, cn);
+        }
+        spread(index, col_cost, d.n_cols[k], chunks, W, 0, vnptr, vn);
+        // bytes that reach the rank in a one-phase iteration: dt of its
+        // columns, posteriors that its rows or its output read
+        auto* bytes = reinterpret_cast<uint32_t*>(im + h.o_bytes);
+        bytes[0] = 4u * static_cast<uint32_t>(t.z) * static_cast<uint32_t>(d.n_dt[k][0]);
+        uint32_t n_read = 0;
+        for (int c = 0; c < nc; c++) n_read += need[c] >> k & 1u;
+        bytes[1] = 4u * static_cast<uint32_t>(t.z) * n_read;
+    }
 }
 
 namespace {

@@ -21,6 +21,7 @@ bool g_relaxed = false;
 cudaStream_t g_config = nullptr;
 const void* g_node = nullptr;  // the kernel of the last graph made or changed
 long g_unfinished = 0;  // bytes that pageable copies may still have on the way
+long g_uploaded = 0;    // bytes copied to the device
 int g_early = 0;        // launches that are not ordered after them
 cudaError_t g_last = cudaSuccess;
 
@@ -44,7 +45,7 @@ void fake_reset() {
     g_launch.clear();
     g_early = g_cluster = g_launches = g_frees = g_mallocs = g_records = g_occupancy = 0;
     g_fail_malloc = -1;
-    g_unfinished = 0;
+    g_unfinished = g_uploaded = 0;
     g_last = cudaSuccess;
 }
 void fake_stream_busy(void* s, int busy) {
@@ -68,6 +69,7 @@ int fake_mallocs() { return g_mallocs; }
 int fake_records() { return g_records; }
 int fake_occupancy_queries() { return g_occupancy; }
 long fake_unfinished() { return g_unfinished; }
+long fake_uploaded() { return g_uploaded; }
 int fake_early_launches() { return g_early; }
 
 // ---- memory ----
@@ -86,7 +88,10 @@ cudaError_t cudaFree(void* p) {
 // A copy from pageable memory may return before its data has reached the device.
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind k) {
     std::memcpy(d, s, n);
-    if (k == cudaMemcpyHostToDevice) g_unfinished += static_cast<long>(n);
+    if (k == cudaMemcpyHostToDevice) {
+        g_unfinished += static_cast<long>(n);
+        g_uploaded += static_cast<long>(n);
+    }
     return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {

@@ -29,7 +29,7 @@ def fake(tmp_path_factory):
         fn = getattr(lib, name)
         fn.restype, fn.argtypes = res, args
     lib.fake_last_launch.restype = C.c_char_p
-    lib.fake_unfinished.restype = C.c_long
+    lib.fake_unfinished.restype = lib.fake_uploaded.restype = C.c_long
     for f in ("fake_stream_busy", "fake_stream_capturing"):
         getattr(lib, f).argtypes = [C.c_void_p, C.c_int]
     return lib
@@ -210,3 +210,33 @@ def test_error_of_the_caller_survives_a_decode(rt):
     assert rt.fake_peek_error() == 0  # and none of the decoder's own
     for h in hs:
         h.close()
+
+
+def test_job_lists_of_new_codes_allocate_nothing(rt):
+    b = List(rt)
+    assert b.set_jobs(1, [384] * 152) == 0  # the check-node state of a full round
+    before = rt.fake_mallocs(), rt.fake_frees()
+    for z in ([2], [40] * 20, [64, 128, 208, 352], [7, 13, 36, 72, 144, 288, 384] * 3):
+        for bg in (1, 2):
+            assert b.set_jobs(bg, z) == 0
+            b.decode(None)
+    assert (rt.fake_mallocs(), rt.fake_frees()) == before
+    b.close()
+
+
+@pytest.mark.parametrize("bg,z", [(1, 384), (2, 208), (1, 96), (2, 40)])
+def test_handles_hold_the_cluster_sizes_that_they_can_pick(rt, bg, z):
+    def upload(n):
+        before = rt.fake_uploaded()
+        h = Handle(rt, bg, z, n)
+        return h, rt.fake_uploaded() - before
+    big, most = upload(400)
+    small, least = upload(1)
+    assert least < most
+    small.close()
+    for n in (1, 2, 7, 8, 20, 36, 60, 100, 152, 300):  # the same choice whatever the largest batch
+        picked = big.decode(n, None), rt.fake_last_cluster()
+        h, _ = upload(n)
+        assert (h.decode(n, None), rt.fake_last_cluster()) == picked
+        h.close()
+    big.close()
