@@ -1004,8 +1004,17 @@ int nrldpc_cb_desegment(const uint8_t* d_blocks, int block_stride, const nrldpc_
         info->k_prime <= info->L || block_stride * 8 < info->k_prime || (info->L > 0 && !d_crc_rem))
         return NRLDPC_ERR_INVALID_ARG;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    return map_cuda(launch_cb_desegment(d_blocks, block_stride, info->C, info->k_prime - info->L, info->k_prime, d_tb,
-                                        0x800063u, info->L > 0 ? 24 : 0, d_crc_rem, st));
+    const int data_bits = info->k_prime - info->L;
+    int len = info->L > 0 ? 24 : 0;
+    // in place (one block): its remainder is taken before the data are written
+    const size_t tb_bytes = (static_cast<size_t>(info->C) * data_bits + 7) / 8;
+    if (len && d_tb < d_blocks + static_cast<size_t>(info->C) * block_stride && d_blocks < d_tb + tb_bytes) {
+        if (launch_crc(d_blocks, info->C, block_stride, info->k_prime, 0x800063u, len, d_crc_rem, st) != cudaSuccess)
+            return NRLDPC_ERR_CUDA;
+        len = 0;
+    }
+    return map_cuda(launch_cb_desegment(d_blocks, block_stride, info->C, data_bits, info->k_prime, d_tb, 0x800063u, len,
+                                        d_crc_rem, st));
 }
 
 int nrldpc_device_error(nrldpc_handle* handle) {

@@ -240,3 +240,12 @@ def test_handles_hold_the_cluster_sizes_that_they_can_pick(rt, bg, z):
         assert (h.decode(n, None), rt.fake_last_cluster()) == picked
         h.close()
     big.close()
+
+
+@pytest.mark.parametrize("offset,launches", [(0, 2), (1 << 16, 1)])  # in place; apart
+def test_block_taken_apart_in_place_is_checked_first(rt, offset, launches):
+    info = _lib.SegmentInfoC(C=1, L=24, k_prime=1029)
+    buf, rem = np.zeros(1 << 17, np.uint8), np.zeros(1, np.uint32)
+    at = buf.ctypes.data
+    assert rt.nrldpc_cb_desegment(at, 256, C.byref(info), at + offset, rem.ctypes.data, None) == 0
+    assert rt.fake_launches() == launches
