@@ -84,15 +84,20 @@ int in_flight_others(const InFlight* me, cudaStream_t stream, long sms, int sm_c
 }
 
 void in_flight_note(InFlight* me, cudaStream_t stream) {
-    std::lock_guard<std::mutex> lock(g_flights_mu);
-    Flights& d = g_flights[me->device];
-    if (d.live.size() < 2) return;
-    d.last = me;
+    {
+        std::lock_guard<std::mutex> lock(g_flights_mu);
+        Flights& d = g_flights[me->device];
+        if (d.live.size() < 2) return;
+        d.last = me;
+    }
     const bool pending = cudaPeekAtLastError() != cudaSuccess;
     if (is_captured(stream, pending)) return;
-    me->recorded = cudaEventRecord(me->done, stream) == cudaSuccess;
+    // without the lock: on a stream that is full of work the record waits
+    const bool recorded = cudaEventRecord(me->done, stream) == cudaSuccess;
+    if (!recorded && !pending) cudaGetLastError();
+    std::lock_guard<std::mutex> lock(g_flights_mu);
+    me->recorded = recorded;
     me->stream = stream;
-    if (!me->recorded && !pending) cudaGetLastError();
 }
 }  // namespace nrldpc
 

@@ -3,17 +3,22 @@
 // what the test says they are.  Linked with the library's own object files.
 #include <cuda_runtime_api.h>
 
+#include <atomic>
+#include <chrono>
 #include <cstdlib>
 #include <cstring>
 #include <map>
 #include <set>
 #include <string>
+#include <thread>
 
 namespace {
 std::map<const void*, std::string> g_names;             // host stub -> mangled kernel name
 std::map<cudaEvent_t, cudaStream_t> g_recorded;
 std::map<cudaEvent_t, int> g_event_device;
 std::set<cudaStream_t> g_busy, g_capturing;
+std::atomic<void*> g_full{nullptr};                      // a stream that takes no more work
+std::atomic<int> g_blocked{0};                           // records that wait for it
 std::string g_launch;                                    // last kernel launched
 int g_cluster = 0, g_launches = 0, g_frees = 0, g_mallocs = 0, g_records = 0, g_occupancy = 0;
 int g_device = 0, g_fail_malloc = -1;
@@ -58,6 +63,8 @@ void fake_stream_capturing(void* s, int on) {
     if (on) g_capturing.insert(st);
     else g_capturing.erase(st);
 }
+void fake_stream_full(void* s) { g_full = s; }
+int fake_blocked() { return g_blocked; }
 void fake_fail_malloc(int after) { g_fail_malloc = after; }
 void fake_set_error(int e) { g_last = static_cast<cudaError_t>(e); }
 int fake_peek_error() { return g_last; }
@@ -189,6 +196,11 @@ cudaError_t cudaEventDestroy(cudaEvent_t e) {
     return cudaSuccess;
 }
 cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
+    if (s && g_full == s) {
+        g_blocked++;
+        for (int i = 0; i < 3000 && g_full == s; i++) std::this_thread::sleep_for(std::chrono::milliseconds(1));
+        g_blocked--;
+    }
     g_recorded[e] = s;
     g_records++;
     return cudaSuccess;

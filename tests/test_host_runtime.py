@@ -4,6 +4,8 @@ import ctypes as C
 import os
 import shutil
 import subprocess
+import threading
+import time
 
 import numpy as np
 import pytest
@@ -30,6 +32,7 @@ def fake(tmp_path_factory):
         fn.restype, fn.argtypes = res, args
     lib.fake_last_launch.restype = C.c_char_p
     lib.fake_unfinished.restype = lib.fake_uploaded.restype = C.c_long
+    lib.fake_stream_full.argtypes = [C.c_void_p]
     for f in ("fake_stream_busy", "fake_stream_capturing"):
         getattr(lib, f).argtypes = [C.c_void_p, C.c_int]
     return lib
@@ -249,3 +252,18 @@ def test_block_taken_apart_in_place_is_checked_first(rt, offset, launches):
     at = buf.ctypes.data
     assert rt.nrldpc_cb_desegment(at, 256, C.byref(info), at + offset, rem.ctypes.data, None) == 0
     assert rt.fake_launches() == launches
+
+
+def test_decoder_that_waits_for_its_stream_does_not_hold_up_others(rt):
+    a, b = Handle(rt), Handle(rt)
+    rt.fake_stream_full(STREAM[0])
+    t = threading.Thread(target=a.decode, args=(40, STREAM[0]))
+    t.start()
+    while not rt.fake_blocked():
+        time.sleep(0.001)
+    b.decode(40, STREAM[1])
+    assert rt.fake_blocked() == 1  # the first call still waits
+    rt.fake_stream_full(None)
+    t.join()
+    a.close()
+    b.close()
