@@ -24,7 +24,9 @@ struct Flights {
     const InFlight* last = nullptr;  // whose call was the last
 };
 std::mutex g_flights_mu;
-std::map<int, Flights> g_flights;  // a device's entry goes with its last decoder
+// A device's entry goes with its last decoder.  The map itself is never
+// destroyed: a program's static objects may destroy handles after that.
+std::map<int, Flights>& g_flights = *new std::map<int, Flights>;
 
 // true also where that cannot be told
 bool is_captured(cudaStream_t stream, bool pending) {

@@ -13,10 +13,11 @@
 #include <thread>
 
 namespace {
-std::map<const void*, std::string> g_names;             // host stub -> mangled kernel name
-std::map<cudaEvent_t, cudaStream_t> g_recorded;
-std::map<cudaEvent_t, int> g_event_device;
-std::set<cudaStream_t> g_busy, g_capturing;
+// never destroyed: the library may be called while the program exits
+auto& g_names = *new std::map<const void*, std::string>;  // host stub -> mangled kernel name
+auto& g_recorded = *new std::map<cudaEvent_t, cudaStream_t>;
+auto& g_busy = *new std::set<cudaStream_t>;
+auto& g_capturing = *new std::set<cudaStream_t>;
 std::atomic<void*> g_full{nullptr};                      // a stream that takes no more work
 std::atomic<int> g_blocked{0};                           // records that wait for it
 std::string g_launch;                                    // last kernel launched
@@ -186,12 +187,10 @@ cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode* m) {
 }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
     *e = reinterpret_cast<cudaEvent_t>(std::malloc(1));
-    g_event_device[*e] = g_device;
     return cudaSuccess;
 }
 cudaError_t cudaEventDestroy(cudaEvent_t e) {
     g_recorded.erase(e);
-    g_event_device.erase(e);
     std::free(e);
     return cudaSuccess;
 }

@@ -267,3 +267,27 @@ def test_decoder_that_waits_for_its_stream_does_not_hold_up_others(rt):
     t.join()
     a.close()
     b.close()
+
+
+def test_handle_destroyed_while_the_program_exits(rt, tmp_path):
+    # by a static object older than the library, so after the library's own
+    src = tmp_path / "late.cpp"
+    src.write_text("""
+#include <dlfcn.h>
+#include "nr_gpu_ldpc_gb300.h"
+static int (*destroy)(nrldpc_handle*);
+struct Late { nrldpc_handle* h[3] = {}; ~Late() { for (auto* x : h) destroy(x); } } late;
+int main(int, char** argv) {
+    void* so = dlopen(argv[1], RTLD_NOW);
+    auto init = reinterpret_cast<int (*)(const nrldpc_config*, nrldpc_handle**)>(dlsym(so, "nrldpc_init"));
+    destroy = reinterpret_cast<int (*)(nrldpc_handle*)>(dlsym(so, "nrldpc_destroy"));
+    nrldpc_config c{1, 64, 4, 0.75f, 0, 0};
+    for (auto& x : late.h) if (init(&c, &x)) return 2;
+    return 0;
+}
+""")
+    exe = str(tmp_path / "late")
+    subprocess.run(["g++", "-std=c++17", str(src), "-I", os.path.join(HERE, "..", "include"), "-ldl", "-o", exe],
+                   check=True, capture_output=True, text=True)
+    junk = {"MALLOC_PERTURB_": "165", "GLIBC_TUNABLES": "glibc.malloc.tcache_count=0"}  # in freed memory
+    assert subprocess.run([exe, rt._name], env={**os.environ, **junk}, timeout=60).returncode == 0
