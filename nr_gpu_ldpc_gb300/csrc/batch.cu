@@ -796,6 +796,13 @@ int nrldpc_batch_decode(nrldpc_batch* batch, const float* d_llr, uint8_t* d_pack
     k.early_stop = early_stop;
     k.alpha = b->alpha;
     void* params[1] = {&k};
+    if (cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+        is_captured(st, cudaPeekAtLastError() != cudaSuccess)) {
+        // a graph launch cannot be captured, what it does can
+        if (cudaMemsetAsync(b->d_scratch, 0, sizeof(int), st) != cudaSuccess) return NRLDPC_ERR_CUDA;
+        return map_cuda(cudaLaunchKernel(batch_decode_kernel_ptr(b->classes), dim3(b->grid), dim3(b->threads), params,
+                                         b->smem, st));
+    }
     cudaKernelNodeParams kp{};
     kp.func = const_cast<void*>(batch_decode_kernel_ptr(b->classes));
     kp.gridDim = dim3(b->grid);

@@ -27,15 +27,14 @@ std::mutex g_flights_mu;
 // A device's entry goes with its last decoder.  The map itself is never
 // destroyed: a program's static objects may destroy handles after that.
 std::map<int, Flights>& g_flights = *new std::map<int, Flights>;
+}  // namespace
 
-// true also where that cannot be told
 bool is_captured(cudaStream_t stream, bool pending) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
     if (!pending) cudaGetLastError();
     return true;
 }
-}  // namespace
 
 bool in_flight_join(InFlight* me, int device) {
     if (cudaEventCreateWithFlags(&me->done, cudaEventDisableTiming) != cudaSuccess) return false;

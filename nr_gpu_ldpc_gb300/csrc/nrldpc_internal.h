@@ -262,6 +262,9 @@ struct InFlight {
     bool recorded = false;
     int neighbours = -1;  // what the caller says instead of the count
 };
+// Whether work on the stream is being captured; true also where that cannot be
+// told.  pending: an error of the caller's that it has not read yet, left alone.
+bool is_captured(cudaStream_t stream, bool pending);
 bool in_flight_join(InFlight* me, int device);
 void in_flight_leave(InFlight* me);
 // Busy ones beside `me`; 0 where as many calls of `sms` SMs as there are

@@ -233,6 +233,7 @@ cudaError_t cudaGraphExecKernelNodeSetParams(cudaGraphExec_t, cudaGraphNode_t, c
     return cudaSuccess;
 }
 cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t s) {
+    if (g_capturing.count(s)) return note(cudaErrorStreamCaptureUnsupported);
     launched(g_node, 0, s);
     return cudaSuccess;
 }
