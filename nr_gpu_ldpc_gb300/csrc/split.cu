@@ -50,8 +50,8 @@ constexpr int kSplitThreads = kSplitMaxWarps * 32;
 // which early stop needs for its failures (sent and counted beside the dt they
 // made BG2 Z=40 16 codewords 7% slower, 20.7 -> 22.2 us).  A cluster barrier
 // takes 400-650 clocks of which 300-500 are the fence, more with stores on the
-// way; counting instead, 10 iterations: BG1 Z=384 49.4 -> 42.8 us on 16 CTAs,
-// 57.6 -> 52.0 on 10, 100.6 -> 94.6 on 4, BG2 Z=208 60 codewords 74.1 -> 65.7.
+// way; counting instead, 10 iterations: BG1 Z=384 49.4 -> 42.4 us on 16 CTAs,
+// 57.6 -> 52.3 on 10, 100.6 -> 95.7 on 4, BG2 Z=208 60 codewords 74.1 -> 65.6.
 // No count can run into the next phase's: a CTA sends a column's dt only after
 // it has that column's posteriors, which the owner sends after its dt are
 // complete, and those include dt that their readers sent after the posteriors
